@@ -72,9 +72,9 @@ constexpr i64 kPad = 32;
 constexpr int kThreads = 256;
 constexpr int kTileRows = 248;  // rows per tile (their offsets are staged in shared memory)
 constexpr int kLaneWork = 32;   // products one lane may sum for one row in a tile
-// Rows one thread of the work-item packer walks in order (a tile never spans
-// two such chunks): short enough that the packers' sequential walks take a
-// fraction of a millisecond, long enough to fill kTileRows-row tiles.  The
+// Rows one warp of the work-item packer takes (a tile never spans two such
+// chunks): short enough that the packers' tile after tile walks take a few
+// microseconds, long enough to fill kTileRows-row tiles.  The
 // panel and head layouts' rows are shorter (their items hold more rows), so
 // they are packed in longer chunks.
 constexpr i64 kPackRows = 256;

@@ -146,78 +146,99 @@ __global__ void k_cold_fill(const i32* __restrict__ toff, const i64* __restrict_
   }
 }
 
-// Work items of a CRS, one thread per chunk of rows (chunk p: piece p % sub
+// Work items of a CRS, one warp per chunk of rows (chunk p: piece p % sub
 // of the stretch of nhot rows p / sub), with the CRS schedule's packing rules
 // (tiles of short rows within `tile` entries, kTileRows rows and kLaneWork
 // products per lane; longer rows in pieces cut at 8-element boundaries).  The
-// greedy packing is sequential within a chunk; a thread walks its chunk's
-// offsets in order, loading them 8 at a time.  Pass 0 counts each chunk's items, long rows and pieces;
-// pass 1 writes them at the scanned offsets `base` (chunk-major: a chunk's
-// items, long rows and pieces are contiguous and numbered globally).
-__global__ void k_panel_pack(const i32* __restrict__ off, i64 nrows, i64 nhot, i64 sub, i64 np, int tile, int write,
-                             i32* __restrict__ cnt, const i32* __restrict__ base, Item* __restrict__ items,
-                             i32* __restrict__ lrows, i32* __restrict__ lpiece0, i32* __restrict__ lfirst) {
+// greedy packing is sequential from tile to tile, but the rows of one tile
+// are found together: lane L tests whether the tile may reach to row
+// t0 + L (every limit, once passed, stays passed), and the first lane that
+// fails ends it, 32 rows a step.  Pass 0 counts each chunk's items, long rows
+// and pieces; pass 1 writes them at the scanned offsets `base` (chunk-major: a
+// chunk's items, long rows and pieces are contiguous and numbered globally).
+// Bound by the latency of the longest chunk's tile to tile chain (rows of
+// 200-500 entries: 100 tiles and more in 256 rows), so the chunk's offsets are
+// read from shared memory: 44 us a pass over the transposed 25,600 x 20,000
+// minibatches of a Zipf matrix (a thread walking each chunk row by row: 97 us).
+constexpr int kPackThreads = 128;
+__global__ void __launch_bounds__(kPackThreads) k_panel_pack(const i32* __restrict__ off, i64 nrows, i64 nhot, i64 sub, i64 np,
+                                                    int tile, int write, i32* __restrict__ cnt,
+                                                    const i32* __restrict__ base, Item* __restrict__ items,
+                                                    i32* __restrict__ lrows, i32* __restrict__ lpiece0,
+                                                    i32* __restrict__ lfirst) {
+  __shared__ i32 soff[kPackThreads / 32][kPanelPackRows + 1];
   const i64 step = (nhot + sub - 1) / sub;
-  for (i64 p = (i64)blockIdx.x * blockDim.x + threadIdx.x; p < np; p += (i64)gridDim.x * blockDim.x) {
-    const i64 s0 = (p / sub) * nhot, s1 = min(s0 + nhot, nrows), j = p % sub;
-    const i64 r0 = min(s0 + j * step, s1), r1 = min(r0 + step, s1);
+  const int lane = threadIdx.x & 31;
+  i32* so = soff[threadIdx.x >> 5];
+  PWARP_STRIDE(p, np) {
+    const i64 s0 = (p / sub) * nhot, s1 = min(s0 + nhot, nrows), jc = p % sub;
+    const i64 r0 = min(s0 + jc * step, s1), r1 = min(r0 + step, s1);
+    __syncwarp();
+#pragma unroll 8
+    for (int q = lane; q <= (int)(r1 - r0); q += 32) so[q] = __ldg(off + r0 + q);  // step <= kPanelPackRows
+    __syncwarp();
     const i32 bi = write ? base[p] : 0, bl = write ? base[(np + 1) + p] : 0, bp = write ? base[2 * (np + 1) + p] : 0;
     i32 ni = 0, nl = 0, npc = 0;
-    i64 t0 = r0, tnnz = 0, tmax = 0;
-    i32 o_cur = off[r0], o_t0 = o_cur;  // off[r], off[t0]
-    auto row = [&](i64 r, i32 o_next) {
-      const i64 len = (i64)o_next - o_cur;
-      if (len > tile) {
-        if (r > t0) {
-          if (write) items[bi + ni] = Item{(int32_t)t0, (int32_t)r, o_t0, o_cur};
-          ni++;
+    i64 t0 = r0;
+    while (t0 < r1) {
+      const i32 o0 = so[t0 - r0];
+      int n = 0;       // rows of the tile starting at t0
+      int mx = 0;      // longest of its rows so far
+      i32 o_end = o0;  // the offset where the tile ends
+      i32 ob, oe;      // offsets of this lane's row t0 + n + lane
+      bool lng;        // that row is longer than a tile
+      for (;;) {
+        const i64 r = t0 + n + lane;
+        const bool valid = r < r1;
+        ob = valid ? so[r - r0] : 0;
+        oe = valid ? so[r - r0 + 1] : 0;
+        const int len = oe - ob;
+        lng = len > tile;
+        int m = max(mx, len);  // longest row up to this one
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int u = __shfl_up_sync(0xffffffffu, m, o);
+          if (lane >= o) m = max(m, u);
         }
-        const i64 st = o_cur, en = o_next, b8 = st & ~7ll;
-        const i64 npr = (en - b8 + tile - 1) / tile;  // pieces: b8 + k*tile < en
-        if (write) {  // its pieces' items: k_long_pieces
-          lrows[bl + nl] = (i32)r;
-          lpiece0[bl + nl] = bp + npc;
-          lfirst[bl + nl] = bi + ni;
-        }
-        nl++;
-        ni += (i32)npr;
-        npc += (i32)npr;
-        t0 = r + 1;
-        o_t0 = o_next;
-        tnnz = 0;
-        tmax = 0;
-      } else {
-        if (r > t0) {
-          const i64 R = r - t0 + 1, mx = max(tmax, len);
-          if (tnnz + len > tile || R > kTileRows || mx > (i64)kLaneWork * lanes_per_row((int)R)) {
-            if (write) items[bi + ni] = Item{(int32_t)t0, (int32_t)r, o_t0, o_cur};
-            ni++;
-            t0 = r;
-            o_t0 = o_cur;
-            tnnz = 0;
-            tmax = 0;
-          }
-        }
-        tnnz += len;
-        tmax = max(tmax, len);
+        const int R = n + lane + 1;
+        const bool ok = valid && !lng && oe - o0 <= tile && R <= kTileRows && m <= kLaneWork * lanes_per_row(R);
+        const unsigned bad = ~__ballot_sync(0xffffffffu, ok);
+        const int k = bad ? __ffs(bad) - 1 : 32;
+        if (k > 0) o_end = __shfl_sync(0xffffffffu, oe, k - 1);
+        n += k;
+        if (bad) break;
+        mx = __shfl_sync(0xffffffffu, m, 31);
       }
-      o_cur = o_next;
-    };
-    // the offsets of 8 rows are loaded together, then the rows walked in order
-    i64 r = r0;
-    for (; r + 8 <= r1; r += 8) {
-      i32 o[8];
+      if (n > 0) {
+        if (write && lane == 0) items[bi + ni] = Item{(int32_t)t0, (int32_t)(t0 + n), o0, o_end};
+        ni++;
+        t0 += n;
+        continue;
+      }
+      // t0 and the rows after it that are longer than a tile, a lane each
+      // (lane L holds row t0 + L): their pieces' items follow (k_long_pieces)
+      const unsigned sh = ~__ballot_sync(0xffffffffu, lng);
+      const int run = sh ? __ffs(sh) - 1 : 32;
+      const i64 b8 = (i64)ob & ~7ll;
+      const i32 npr = lane < run ? (i32)(((i64)oe - b8 + tile - 1) / tile) : 0;  // pieces: b8 + k*tile < oe
+      i32 incl = npr;
 #pragma unroll
-      for (int q = 0; q < 8; q++) o[q] = off[r + 1 + q];
-#pragma unroll
-      for (int q = 0; q < 8; q++) row(r + q, o[q]);
+      for (int o = 1; o < 32; o <<= 1) {
+        const i32 u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+      }
+      if (write && lane < run) {
+        lrows[bl + nl + lane] = (i32)(t0 + lane);
+        lpiece0[bl + nl + lane] = bp + npc + incl - npr;
+        lfirst[bl + nl + lane] = bi + ni + incl - npr;
+      }
+      const i32 all = __shfl_sync(0xffffffffu, incl, 31);
+      nl += run;
+      ni += all;
+      npc += all;
+      t0 += run;
     }
-    for (; r < r1; r++) row(r, off[r + 1]);
-    if (r1 > t0) {
-      if (write) items[bi + ni] = Item{(int32_t)t0, (int32_t)r1, o_t0, o_cur};
-      ni++;
-    }
-    if (!write) {
+    if (!write && lane == 0) {
       cnt[p] = ni;
       cnt[np + p] = nl;
       cnt[2 * np + p] = npc;
@@ -955,9 +976,10 @@ void device_pack(fvg_ctx* c, const i32* off, i64 nrows, i64 chunk, i64 nchunks, 
   const i64 np = std::max<i64>(nchunks, 1) * sub;
   DBuf cnt, basev;
   cnt.alloc(sizeof(i32) * 3 * np, c->stream);
-  // a thread per chunk
-  const unsigned pg = (unsigned)std::min<i64>((np + 255) / 256, 1 << 20);
-  k_panel_pack<<<pg, 256, 0, c->stream>>>(off, nrows, chunk, sub, np, tile, 0, cnt.as<i32>(), nullptr, nullptr,
+  if ((chunk + sub - 1) / sub > kPanelPackRows) fail(FVG_ERR_INTERNAL, "packing chunk too long");
+  constexpr int kPw = kPackThreads / 32;  // a warp per chunk
+  const unsigned pg = (unsigned)std::min<i64>((np + kPw - 1) / kPw, 1 << 20);
+  k_panel_pack<<<pg, kPackThreads, 0, c->stream>>>(off, nrows, chunk, sub, np, tile, 0, cnt.as<i32>(), nullptr, nullptr,
                                           nullptr, nullptr, nullptr);
   check_launch("pack");
   count_launch(c);
@@ -984,7 +1006,7 @@ void device_pack(fvg_ctx* c, const i32* off, i64 nrows, i64 chunk, i64 nchunks, 
   o.long_piece0.alloc(sizeof(i32) * (o.nlong + 1), c->stream);
   DBuf lfirst;
   lfirst.alloc(sizeof(i32) * std::max<i64>(o.nlong, 1), c->stream);
-  k_panel_pack<<<pg, 256, 0, c->stream>>>(off, nrows, chunk, sub, np, tile, 1, nullptr, basev.as<i32>(),
+  k_panel_pack<<<pg, kPackThreads, 0, c->stream>>>(off, nrows, chunk, sub, np, tile, 1, nullptr, basev.as<i32>(),
                                           o.items.as<Item>(), o.long_rows.as<i32>(), o.long_piece0.as<i32>(),
                                           lfirst.as<i32>());
   check_launch("pack");
@@ -1033,7 +1055,7 @@ void pack_split_items(fvg_ctx* c, DevPanels& pn) {
 
 void pack_panels(fvg_ctx* c, DevPanels& pn, i64 nhot, i64 np) {
   PackOut o;
-  // each panel's rows in pieces of ~kPanelPackRows rows, a packing thread each
+  // each panel's rows in pieces of ~kPanelPackRows rows, a packing warp each
   const i64 sub = std::max<i64>(1, (nhot + kPanelPackRows - 1) / kPanelPackRows);
   device_pack(c, pn.poff.as<i32>(), np * nhot, nhot, np, kWarpTile, o, sub);
   pn.nitems = o.nitems;
