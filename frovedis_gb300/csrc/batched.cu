@@ -755,8 +755,8 @@ struct BatchEval {
     // pieces listed by slabs of R that fit in L2 (48 MiB)
     slab = std::max<i64>(4096, (i64)((48ull << 20) / ((size_t)ld * (f64 ? 8 : 4))));
     for (int st : planes) {
-      crs_sched(c, *A, tile_for_storage(st));  // built before any capture
-      crs_sched_slabs(c, *AT, tile_for_storage(st), slab);
+      pass_sched(c, *A, st);  // built before any capture
+      crs_sched_slabs(c, *AT, st, slab);
       s1b = std::max(s1b, spmm_scratch_bytes(c, *A, st));
       s2b = std::max(s2b, spmm_scratch_bytes(c, *AT, st, slab));
     }

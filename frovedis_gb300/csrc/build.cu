@@ -202,10 +202,7 @@ void crs_build_transpose(fvg_ctx* c, const DevCRS& a, DevCRS& t, int master) {
 // thread each (a tile never spans two chunks).
 constexpr i64 kSchedChunk = kPackRows;
 
-const Sched& crs_sched(fvg_ctx* c, DevCRS& a, int tile) {
-  // slot 0: the CRS kernel's items (kWarpTile); slot 1: another item size
-  // (the split kernel's), built on its first use
-  const int slot = tile == kWarpTile ? 0 : 1;
+static const Sched& build_sched(fvg_ctx* c, DevCRS& a, int slot, int tile, int lane_work) {
   if (a.sched[slot]) {
     if (a.sched[slot]->tile != tile) fail(FVG_ERR_INTERNAL, "a second work-item size for one matrix");
     return *a.sched[slot];
@@ -216,7 +213,7 @@ const Sched& crs_sched(fvg_ctx* c, DevCRS& a, int tile) {
   const i64 m = a.m;
   const i64 nchunks = std::max<i64>(1, (m + kSchedChunk - 1) / kSchedChunk);
   PackOut o;
-  device_pack(c, a.off.as<i32>(), m, kSchedChunk, nchunks, tile, o);
+  device_pack(c, a.off.as<i32>(), m, kSchedChunk, nchunks, tile, o, 1, lane_work);
   s->nitems = o.nitems;
   s->nlong = o.nlong;
   s->npieces = o.npieces;
@@ -226,6 +223,18 @@ const Sched& crs_sched(fvg_ctx* c, DevCRS& a, int tile) {
   a.sched[slot] = std::move(s);
   return *a.sched[slot];
 }
+
+const Sched& crs_sched(fvg_ctx* c, DevCRS& a, int tile) {
+  // slot 0: the CRS kernel's items (kWarpTile); slot 1: another item size
+  // (the split kernel's), built on its first use
+  return build_sched(c, a, tile == kWarpTile ? 0 : 1, tile, kLaneWork);
+}
+
+// The FP64 kernel cuts an item among its lanes by entries, so only the
+// entries and rows limit its tiles: on power-law rows (2M x 2M, 40 entries a
+// row on average) the kLaneWork limit leaves 0.44 of an item's entries used,
+// without it 0.70.
+const Sched& crs_sched64(fvg_ctx* c, DevCRS& a) { return build_sched(c, a, 2, kWarpTile, kNoLaneWork); }
 
 // ------------------------------------------------------ slab-ordered pieces
 // Work items of a transposed product whose gathered vector rows are larger
@@ -278,9 +287,10 @@ __global__ void k_gather_items(const Item* __restrict__ src, const uint32_t* __r
   GRID_STRIDE(i, n) dst[i] = src[order[i]];
 }
 
-const Sched& crs_sched_slabs(fvg_ctx* c, DevCRS& a, int tile, i64 slab) {
-  if (a.slab_sched && a.slab_rows == slab && a.slab_sched->tile == tile) return *a.slab_sched;
-  const Sched& s0 = crs_sched(c, a, tile);
+const Sched& crs_sched_slabs(fvg_ctx* c, DevCRS& a, int storage, i64 slab) {
+  if (a.slab_sched && a.slab_rows == slab) return *a.slab_sched;
+  const Sched& s0 = pass_sched(c, a, storage);
+  const int tile = s0.tile;
   ProfScope ps(c, P_SCHED);
   auto s = std::make_unique<Sched>();
   s->tile = tile;

@@ -275,13 +275,17 @@ static void ensure_transpose(fvg_ctx* c, fvg_matrix* M) {
   }
 }
 
+// The CRS kernels' work schedules for the value planes the matrix has.
+static void crs_scheds(fvg_ctx* c, fvg_matrix* M, DevCRS& a) {
+  for (int dt : {FVG_F64, FVG_F32, FVG_BF16})
+    if (M->A.val[dt].p) pass_sched(c, a, dt);
+}
+
 static void prepare(fvg_ctx* c, fvg_matrix* M, int fmt, bool trans) {
   if (fmt == FVG_CRS) {
-    crs_sched(c, M->A, kWarpTile);  // the CRS kernel's work schedule
-    if (trans) {
-      ensure_transpose(c, M);
-      crs_sched(c, *M->AT, kWarpTile);
-    }
+    if (trans) ensure_transpose(c, M);
+    crs_scheds(c, M, M->A);
+    if (trans) crs_scheds(c, M, *M->AT);
   } else if (fmt == FVG_ELL) {
     if (!M->ell) {
       M->ell.reset(new DevELL());
@@ -403,6 +407,9 @@ static void ensure_plane_all(fvg_ctx* c, fvg_matrix* M, int dt) {
   }
   crs_ensure_plane(c, M->A, dt, M->master);
   if (M->AT) crs_ensure_plane(c, *M->AT, dt, M->master);
+  // a matrix prepared before it had this plane: its schedule too
+  for (DevCRS* a : {&M->A, M->AT.get()})
+    if (a && (a->sched[0] || a->sched[2])) pass_sched(c, *a, dt);
   if (M->ell) ensure_plane_generic(c, M->ell->val, M->ell->m * M->ell->width, dt, M->master);
   for (DevJDS* j : {M->jds.get(), M->tjds.get()})
     if (j) ensure_plane_generic(c, j->val, j->nnz, dt, M->master);

@@ -68,23 +68,38 @@ __device__ __forceinline__ void block_csum2(double a, double b, double* out_a, d
 }
 
 // ------------------------------------------------------- logistic math
-// logistic_gradient<T>::compute_dloss for one row (gradient.hpp:24-50).
+// logistic_gradient<T>::compute_dloss for one row (gradient.hpp:24-50) in
+// FP64 with one exponential, e = exp(-|z|): between the reference's
+// thresholds log(1 + exp(-z)) = log(1 + e) (+ |z| when z < 0) and
+// 1 / (1 + exp(z)) = e / (1 + e) (z > 0) or 1 / (1 + e).  GB300's FP64 unit
+// makes every FP64 instruction count (two exponentials and FP64 range tests:
+// 1.6x the time of this form), so the rarely met ranges are recognised from
+// the high word and tested exactly only there (NaN included).
+__device__ __forceinline__ bool dbl_at_least(double v, int hi) {  // |v|'s high word >= hi
+  return (__double2hiint(v) & 0x7fffffff) >= hi;
+}
 __device__ __forceinline__ void logistic_row(double wtx, double lab, double& loss, double& d) {
-  double z = lab * wtx;
-  double neg = lab * -1.0;
-  if (z > 18.0) {
-    double e = exp(-z);
+  const double z = lab * wtx;
+  const double neg = -lab;
+  const double az = __hiloint2double(__double2hiint(z) & 0x7fffffff, __double2loint(z));
+  const double e = exp(-az);
+  const bool up = __double2hiint(z) >= 0;  // z >= 0
+  if (dbl_at_least(z, 0x40320000) && z > 18.0) {
     loss = e;
     d = e * neg;
-  } else if (z < -18.0) {
-    loss = -z;
+  } else if (dbl_at_least(z, 0x40320000) && z < -18.0) {
+    loss = az;
     d = neg;
   } else {
-    loss = log(1.0 + exp(-z));
-    d = neg * (1.0 / (1.0 + exp(z)));
+    const double u = 1.0 + e;
+    loss = log(u);
+    if (!up) loss += az;
+    d = neg * ((up ? e : 1.0) / u);
   }
-  if (d > 1e12) d = 1e12;
-  else if (d < -1e12) d = -1e12;
+  if (dbl_at_least(d, 0x426d1a94)) {  // 1e12 and above
+    if (d > 1e12) d = 1e12;
+    else if (d < -1e12) d = -1e12;
+  }
 }
 // FP32 variant for the BF16/FP32-storage path (log1p form keeps small
 // losses that log(1+e) would round away in single precision).

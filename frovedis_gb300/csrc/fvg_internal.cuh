@@ -114,7 +114,6 @@ struct Sched {
 #define FVG_CRS_ROUNDS 8
 #endif
 constexpr int kWarpTile = FVG_WARP_TILE;  // nonzeros per warp item
-inline int tile_for_storage(int) { return kWarpTile; }
 
 // Device CRS matrix with up to three value planes.
 struct DevCRS {
@@ -122,7 +121,9 @@ struct DevCRS {
   DBuf off, idx;  // int32
   DBuf val[3];    // indexed by fvg_dtype
   DBuf lo;        // bf16 [nnz+kPad]: value - FP32 value (split storage; with val[FVG_F32])
-  std::unique_ptr<Sched> sched[2];  // work items: slot 0 kWarpTile, slot 1 the split kernel's size
+  // work items: slot 0 kWarpTile, slot 1 the split kernel's size, slot 2
+  // kWarpTile without the kLaneWork limit (FP64 values)
+  std::unique_ptr<Sched> sched[3];
   std::unique_ptr<Sched> slab_sched;  // long rows in slab-ordered pieces (crs_sched_slabs)
   i64 slab_rows = 0;
   i64 max_row = 0;
@@ -219,7 +220,11 @@ struct PackOut {
 };
 // Each chunk may itself be packed in `sub` pieces (a warp each; items never
 // span two pieces); base then has nchunks*sub+1 entries per kind.
-void device_pack(fvg_ctx* c, const i32* off, i64 nrows, i64 chunk, i64 nchunks, int tile, PackOut& o, i64 sub = 1);
+// lane_work: products one lane may sum for one row of a tile (kLaneWork, or
+// kNoLaneWork for kernels that cut the rows among the lanes by entries).
+constexpr int kNoLaneWork = 1 << 20;
+void device_pack(fvg_ctx* c, const i32* off, i64 nrows, i64 chunk, i64 nchunks, int tile, PackOut& o, i64 sub = 1,
+                 int lane_work = kLaneWork);
 
 struct Profiler;
 
@@ -327,9 +332,15 @@ void crs_upload(fvg_ctx* c, DevCRS& a, i64 m, i64 n, const i32* off, const i32* 
 void crs_ensure_plane(fvg_ctx* c, DevCRS& a, int dt, int master);
 void crs_build_transpose(fvg_ctx* c, const DevCRS& a, DevCRS& t, int master);
 const Sched& crs_sched(fvg_ctx* c, DevCRS& a, int tile);
+const Sched& crs_sched64(fvg_ctx* c, DevCRS& a);  // the FP64 kernel's items (slot 2)
+// The kWarpTile items a value storage's products walk: FP64 slot 2, FP32 and
+// BF16 slot 0 (the multi-vector kernels take either).
+inline const Sched& pass_sched(fvg_ctx* c, DevCRS& a, int storage) {
+  return storage == FVG_F64 ? crs_sched64(c, a) : crs_sched(c, a, kWarpTile);
+}
 // The rows longer than a tile cut into pieces also at every slab of `slab`
 // column ids, the pieces listed slab by slab before the tiles (cached).
-const Sched& crs_sched_slabs(fvg_ctx* c, DevCRS& a, int tile, i64 slab);
+const Sched& crs_sched_slabs(fvg_ctx* c, DevCRS& a, int storage, i64 slab);
 void ell_build(fvg_ctx* c, const DevCRS& a, DevELL& e, int master);
 void jds_build(fvg_ctx* c, const DevCRS& a, DevJDS& j, int master);
 void hyb_build(fvg_ctx* c, const DevCRS& a, DevHYB& h, int master, i64 threshold);

@@ -148,7 +148,7 @@ __global__ void k_cold_fill(const i32* __restrict__ toff, const i64* __restrict_
 
 // Work items of a CRS, one warp per chunk of rows (chunk p: piece p % sub
 // of the stretch of nhot rows p / sub), with the CRS schedule's packing rules
-// (tiles of short rows within `tile` entries, kTileRows rows and kLaneWork
+// (tiles of short rows within `tile` entries, kTileRows rows and lane_work
 // products per lane; longer rows in pieces cut at 8-element boundaries).  The
 // greedy packing is sequential from tile to tile, but the rows of one tile
 // are found together: lane L tests whether the tile may reach to row
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kPackThreads) k_panel_pack(const i32* __restri
                                                     int tile, int write, i32* __restrict__ cnt,
                                                     const i32* __restrict__ base, Item* __restrict__ items,
                                                     i32* __restrict__ lrows, i32* __restrict__ lpiece0,
-                                                    i32* __restrict__ lfirst) {
+                                                    i32* __restrict__ lfirst, int lane_work) {
   __shared__ i32 soff[kPackThreads / 32][kPanelPackRows + 1];
   const i64 step = (nhot + sub - 1) / sub;
   const int lane = threadIdx.x & 31;
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kPackThreads) k_panel_pack(const i32* __restri
           if (lane >= o) m = max(m, u);
         }
         const int R = n + lane + 1;
-        const bool ok = valid && !lng && oe - o0 <= tile && R <= kTileRows && m <= kLaneWork * lanes_per_row(R);
+        const bool ok = valid && !lng && oe - o0 <= tile && R <= kTileRows && m <= lane_work * lanes_per_row(R);
         const unsigned bad = ~__ballot_sync(0xffffffffu, ok);
         const int k = bad ? __ffs(bad) - 1 : 32;
         if (k > 0) o_end = __shfl_sync(0xffffffffu, oe, k - 1);
@@ -972,7 +972,8 @@ void fill_planes(fvg_ctx* c, const DevCRS& at, DevPanels& pn, const i32* B, cons
 // rows and pieces are contiguous, numbered globally), packed on the device:
 // counts, their exclusive scans (a few thousand numbers, on the host), then
 // the items.
-void device_pack(fvg_ctx* c, const i32* off, i64 nrows, i64 chunk, i64 nchunks, int tile, PackOut& o, i64 sub) {
+void device_pack(fvg_ctx* c, const i32* off, i64 nrows, i64 chunk, i64 nchunks, int tile, PackOut& o, i64 sub,
+                 int lane_work) {
   const i64 np = std::max<i64>(nchunks, 1) * sub;
   DBuf cnt, basev;
   cnt.alloc(sizeof(i32) * 3 * np, c->stream);
@@ -980,7 +981,7 @@ void device_pack(fvg_ctx* c, const i32* off, i64 nrows, i64 chunk, i64 nchunks, 
   constexpr int kPw = kPackThreads / 32;  // a warp per chunk
   const unsigned pg = (unsigned)std::min<i64>((np + kPw - 1) / kPw, 1 << 20);
   k_panel_pack<<<pg, kPackThreads, 0, c->stream>>>(off, nrows, chunk, sub, np, tile, 0, cnt.as<i32>(), nullptr, nullptr,
-                                          nullptr, nullptr, nullptr);
+                                          nullptr, nullptr, nullptr, lane_work);
   check_launch("pack");
   count_launch(c);
   std::vector<i32> hc((size_t)(3 * np));
@@ -1008,7 +1009,7 @@ void device_pack(fvg_ctx* c, const i32* off, i64 nrows, i64 chunk, i64 nchunks, 
   lfirst.alloc(sizeof(i32) * std::max<i64>(o.nlong, 1), c->stream);
   k_panel_pack<<<pg, kPackThreads, 0, c->stream>>>(off, nrows, chunk, sub, np, tile, 1, nullptr, basev.as<i32>(),
                                           o.items.as<Item>(), o.long_rows.as<i32>(), o.long_piece0.as<i32>(),
-                                          lfirst.as<i32>());
+                                          lfirst.as<i32>(), lane_work);
   check_launch("pack");
   count_launch(c);
   if (o.nlong > 0) {

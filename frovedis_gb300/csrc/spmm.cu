@@ -863,8 +863,7 @@ static int spmm_fin_grid(fvg_ctx* c, i64 nlong) {
 // Scratch of one block pass (sized for 128 columns): ticket, per-CTA
 // partials of the main and finalize kernels, long-row piece partials.
 i64 spmm_scratch_bytes(fvg_ctx* c, DevCRS& a, int storage, i64 slab) {
-  const Sched& s = slab > 0 ? crs_sched_slabs(c, a, tile_for_storage(storage), slab)
-                            : crs_sched(c, a, tile_for_storage(storage));
+  const Sched& s = slab > 0 ? crs_sched_slabs(c, a, storage, slab) : pass_sched(c, a, storage);
   const size_t at = storage == FVG_F64 ? 8 : 4;
   const i64 grid = 8 * (i64)c->num_sms;  // occupancy upper bound (8 CTAs of 256 threads per SM)
   return (i64)(al256(256) + al256(sizeof(double) * 2 * kSpmmMaxCols * grid) +
@@ -1050,8 +1049,7 @@ void crs_spmm_block(fvg_ctx* c, DevCRS& a, int storage, const void* X, i64 ldx, 
                     void* scratch, const int* gate, i64 slab) {
   if (kb < 1 || kb > kSpmmMaxCols) fail(FVG_ERR_INTERNAL, "spmm block width out of range");
   if (!a.val[storage].p) fail(FVG_ERR_INTERNAL, "missing value plane for the requested storage");
-  const Sched& s = slab > 0 ? crs_sched_slabs(c, a, tile_for_storage(storage), slab)
-                            : crs_sched(c, a, tile_for_storage(storage));
+  const Sched& s = slab > 0 ? crs_sched_slabs(c, a, storage, slab) : pass_sched(c, a, storage);
   SpmmK p = {};
   p.X = X;
   p.ldx = ldx;
@@ -1089,8 +1087,7 @@ void crs_spmm_store_seg(fvg_ctx* c, DevCRS& a, int storage, const void* X, i64 l
                         void* scratch, SpmmSeg& sg, i64 slab) {
   if (kb < 1 || kb > 64 || sg.nseg < 1) fail(FVG_ERR_INTERNAL, "stacked store: block width or datasets out of range");
   if (!a.val[storage].p) fail(FVG_ERR_INTERNAL, "missing value plane for the requested storage");
-  const Sched& s = slab > 0 ? crs_sched_slabs(c, a, tile_for_storage(storage), slab)
-                            : crs_sched(c, a, tile_for_storage(storage));
+  const Sched& s = slab > 0 ? crs_sched_slabs(c, a, storage, slab) : pass_sched(c, a, storage);
   SpmmK p = {};
   p.X = X;
   p.ldx = ldx;
@@ -1117,7 +1114,7 @@ void crs_spmm_logreg_block(fvg_ctx* c, DevCRS& a, int storage, const void* W, i6
                            const double* sw, const float* label_f, const float* sw_f, int icpt, const double* bias,
                            void* R, i64 ldr, double* out, double* gbias, void* scratch, int loss, double eps) {
   if (kb < 1 || kb > 64) fail(FVG_ERR_INTERNAL, "spmm block width out of range");
-  const Sched& s = crs_sched(c, a, tile_for_storage(storage));
+  const Sched& s = pass_sched(c, a, storage);
   SpmmK p = {};
   p.X = W;
   p.ldx = ldw;
@@ -1158,7 +1155,7 @@ void crs_spmm_logreg_seg(fvg_ctx* c, DevCRS& a, int storage, const void* W, i64 
                          const double* sw, const float* label_f, const float* sw_f, int icpt, const double* bias,
                          void* R, i64 ldr, void* scratch, SpmmSeg& sg, int loss, double eps) {
   if (kb < 1 || kb > 64 || sg.nseg < 1) fail(FVG_ERR_INTERNAL, "stacked pass: block width or datasets out of range");
-  const Sched& s = crs_sched(c, a, tile_for_storage(storage));
+  const Sched& s = pass_sched(c, a, storage);
   SpmmK p = {};
   p.X = W;
   p.ldx = ldw;
@@ -1213,7 +1210,7 @@ void crs_spmm_softmax(fvg_ctx* c, DevCRS& a, int storage, const void* W, i64 ldw
                       const double* sw, const float* label_f, const float* sw_f, int icpt, const double* icpt_v,
                       void* P, i64 ldp, void* scratch, double* loss_out) {
   if (K < 1 || K > kSpmmMaxCols) fail(FVG_ERR_INTERNAL, "softmax block width out of range");
-  const Sched& s = crs_sched(c, a, tile_for_storage(storage));
+  const Sched& s = pass_sched(c, a, storage);
   SpmmK p = {};
   p.X = W;
   p.ldx = ldw;

@@ -18,6 +18,10 @@
 // sums on the FP32-arithmetic path, which keep GB300's narrow FP64 unit out of
 // the per-row work; FP64 Neumaier sums on the FP64 path), which the finalize
 // kernel reduces in FP64 in a fixed order.
+#include <algorithm>
+#include <mutex>
+#include <vector>
+
 #include "device_common.cuh"
 
 namespace fvg {
@@ -66,30 +70,26 @@ __device__ __forceinline__ void epilogue(const CrsK& p, i32 row, AT acc, AT b, S
     }
     ((YT*)p.r)[row] = (YT)d;
     ls.add(loss);
-    bs.add(d);
+    if (p.icpt) bs.add(d);  // without an intercept the bias sum is reported as 0
   }
 }
 
 // ------------------------------------------------------------ warp tiles
 
-// Persistent CRS kernel.  Warp g of the grid handles items g, g+W, g+2W, ...
-// (W = warps in the grid).  Phase 1: the warp streams the item's nonzeros
-// with coalesced loads (lane L: nonzeros L, L+32, ...; a group of rounds
-// issued before any use), gathers x and writes the products to its own
-// shared-memory slice.  Phase 2: rows of a tile are
+// Persistent CRS kernel of the FP32-arithmetic paths.  Warp g of the grid
+// handles items g, g+W, g+2W, ... (W = warps in the grid).  Phase 1: the warp
+// streams the item's nonzeros with coalesced loads (lane L: nonzeros L, L+32,
+// ...; a group of rounds issued before any use), gathers x and writes the
+// products to its own shared-memory slice.  Phase 2: rows of a tile are
 // summed from shared memory by 1..32 lanes each (32 / rows, rounded to a
 // power of two), the lanes of a row combined by shuffles; a piece is summed
 // by the whole warp.  No CTA-wide barrier inside the loop.
 template <class VT, class XT, class AT, class YT, int EPI>
 __global__ void __launch_bounds__(kThreads, FVG_CRS_MIN_BLOCKS) k_crs(const CrsK p) {
+  static_assert(sizeof(AT) == 4, "FP64 sums: k_crs64");
   constexpr int SPAN = kWarpTile;        // products slice per warp
   constexpr int NR = SPAN / 32;          // element rounds per lane
-  constexpr int RG = sizeof(VT) == 8 ? (FVG_CRS_ROUNDS + 1) / 2 : FVG_CRS_ROUNDS;  // rounds in flight together
-  // FP64: GB300 issues FP64 at a small fraction of the FP32 rate, so phase 1
-  // only gathers x and phase 2 does one fused multiply-add per nonzero
-  // (instead of a multiply here and an add there) with the value re-read
-  // (the warp streamed it just before: L1/L2)
-  constexpr bool kFmaRows = sizeof(AT) == 8;
+  constexpr int RG = FVG_CRS_ROUNDS;     // rounds in flight together
   __shared__ AT sprod[kThreads / 32][SPAN];
   __shared__ int soffs[kThreads / 32][kTileRows + 1];
   using Sum = typename SumOf<AT>::type;
@@ -124,16 +124,13 @@ __global__ void __launch_bounds__(kThreads, FVG_CRS_MIN_BLOCKS) k_crs(const CrsK
         const int k = (g + q) * 32 + lane;
         if (g + q < NR && k < span) {
           c[q] = __ldcs(p.idx + a0 + k);
-          if constexpr (!kFmaRows) v[q] = ld_val<VT, AT>(val + a0 + k);
+          v[q] = ld_val<VT, AT>(val + a0 + k);
         }
       }
 #pragma unroll
       for (int q = 0; q < RG; q++) {
         const int k = (g + q) * 32 + lane;
-        if (g + q < NR && k < span) {
-          if constexpr (kFmaRows) prod[k] = (AT)__ldg(x + c[q]);  // the value joins in phase 2
-          else prod[k] = v[q] * (AT)__ldg(x + c[q]);
-        }
+        if (g + q < NR && k < span) prod[k] = v[q] * (AT)__ldg(x + c[q]);
       }
     }
     __syncwarp();
@@ -150,43 +147,22 @@ __global__ void __launch_bounds__(kThreads, FVG_CRS_MIN_BLOCKS) k_crs(const CrsK
         if (j < R) {
           const int s = soff[j] - a0, e = soff[j + 1] - a0;
           int k = s + sub;
-          if constexpr (kFmaRows) {
-            const VT* vr = val + a0;
-            if (e - s > 4 * Gl) {
-              AT a1 = 0, a2 = 0, a3 = 0;
-              for (; k + 3 * Gl < e; k += 4 * Gl) {
-                acc = fma((AT)vr[k], prod[k], acc);
-                a1 = fma((AT)vr[k + Gl], prod[k + Gl], a1);
-                a2 = fma((AT)vr[k + 2 * Gl], prod[k + 2 * Gl], a2);
-                a3 = fma((AT)vr[k + 3 * Gl], prod[k + 3 * Gl], a3);
-              }
-              for (; k < e; k += Gl) acc = fma((AT)vr[k], prod[k], acc);
-              acc = (acc + a1) + (a2 + a3);
-            } else {
-              for (; k < e; k += Gl) acc = fma((AT)vr[k], prod[k], acc);
-            }
-          } else {
-            AT a1 = 0, a2 = 0, a3 = 0;
-            for (; k + 3 * Gl < e; k += 4 * Gl) {
-              acc += prod[k];
-              a1 += prod[k + Gl];
-              a2 += prod[k + 2 * Gl];
-              a3 += prod[k + 3 * Gl];
-            }
-            for (; k < e; k += Gl) acc += prod[k];
-            acc = (acc + a1) + (a2 + a3);
+          AT a1 = 0, a2 = 0, a3 = 0;
+          for (; k + 3 * Gl < e; k += 4 * Gl) {
+            acc += prod[k];
+            a1 += prod[k + Gl];
+            a2 += prod[k + 2 * Gl];
+            a3 += prod[k + 3 * Gl];
           }
+          for (; k < e; k += Gl) acc += prod[k];
+          acc = (acc + a1) + (a2 + a3);
         }
         for (int o = Gl >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if (j < R && sub == 0) epilogue<AT, YT, EPI>(p, it.r0 + j, acc, bias, ls, bs);
       }
     } else {
       AT acc = 0;
-      if constexpr (kFmaRows) {
-        for (int k = it.e0 - a0 + lane; k < span; k += 32) acc = fma((AT)val[a0 + k], prod[k], acc);
-      } else {
-        for (int k = it.e0 - a0 + lane; k < span; k += 32) acc += prod[k];
-      }
+      for (int k = it.e0 - a0 + lane; k < span; k += 32) acc += prod[k];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
       if (lane == 0) ((AT*)p.partials)[-1 - it.r1] = acc;
@@ -194,6 +170,192 @@ __global__ void __launch_bounds__(kThreads, FVG_CRS_MIN_BLOCKS) k_crs(const CrsK
     __syncwarp();
   }
   if (EPI == EPI_LOGREG) block_csum2(ls.total(), bs.total(), &p.cta_part[2 * blockIdx.x], &p.cta_part[2 * blockIdx.x + 1]);
+}
+
+// ---------------------------------------------------------- FP64 products
+// The FP64 product.  GB300 runs about two FP64 operations a clock per SM, so
+// a warp-wide FP64 instruction costs 16 clocks whether 2 or 32 of its lanes
+// are used, while some 60 other instructions issue beside it: the row sums
+// must keep every lane's FP64 slot busy and may spend integer work freely.
+// Phase 1 (as k_crs): lane L streams nonzeros L, L+32, ... with coalesced
+// loads (one gather instruction covers 32 consecutive nonzeros) and puts the
+// gathered x and the value into the warp's shared slices.  Phase 2: lane L
+// owns ch = ceil(nonzeros / 32) consecutive nonzeros (16 of a full item) and
+// adds them with one fused multiply-add each, starting anew at the rows'
+// first entries, which sit as bits in a 512-bit map; the sum up to each row
+// start is parked in the slot of that start.  The segments open at the
+// chunks' ends are joined in lane order by a segmented scan that stops once
+// every lane has met a row start (rows of 60 entries: 3 of its 5 steps), and
+// added to the sum parked at the next chunk's first mark.  Phase 3, a lane
+// per row: the row's sum is the one parked at its end.  An item costs 16 +
+// about 4 FP64 instructions for 512 nonzeros; lanes_per_row() lanes a row
+// cost 30 to 60 on rows of uneven length and re-read the values lane by lane
+// from L1.  A long row's piece is added in registers by the whole warp.  The
+// next item's ids are loaded before this item's sums.
+// The gathers miss L1 one by one (an SM takes about one such sector a clock:
+// 2M x 2M with uniform columns cannot go below 0.27 ms), and each needs an L1
+// line while it is under way, so shared memory is kept to 3 CTAs of 4 warps:
+// 24 warps (222 KB of slices) took 1.21 ms where 12 (111 KB) take 0.44.
+// Measured (before: k_crs's rows by lanes, and its loss rows): 2M x 2M
+// power-law 558 -> 442 us; 1M x 100,000, 6.0e7 nonzeros, A w with hinge loss
+// 372 -> 221 + 60, A^T r 238 -> 221; 100,000 x 20,000, 4.0e6 nonzeros, A w
+// with logistic loss 81 -> 18 + 26, A^T r 22.6 -> 18.3.  At 6.0e7 nonzeros L1's
+// data pipe is 74% and the FP64 pipe 59% busy.
+static_assert(kWarpTile == 512, "k_crs64: 16 entries a lane, a 16-word row map");
+constexpr int kC64 = 16;                               // entries per lane
+constexpr int kC64Pad = kWarpTile + kWarpTile / kC64;  // doubles per slice
+constexpr int kC64SoffB = ((kTileRows + 1) * 2 + 15) / 16 * 16;
+constexpr int kC64Map = kWarpTile / 32 + 4;  // words of the row map (and padding)
+constexpr int kC64WarpB = 2 * kC64Pad * 8 + 4 * kC64Map + kC64SoffB;  // x, values, row map, row offsets
+static_assert(kC64WarpB % 16 == 0, "slices stay 16-byte aligned");
+#ifndef FVG_CRS64_WARPS
+#define FVG_CRS64_WARPS 4
+#endif
+#ifndef FVG_CRS64_BLOCKS
+#define FVG_CRS64_BLOCKS 3
+#endif
+#ifndef FVG_CRS64_RG
+#define FVG_CRS64_RG 16
+#endif
+constexpr int kC64Threads = 32 * FVG_CRS64_WARPS;
+constexpr int kC64Blocks = FVG_CRS64_BLOCKS;  // resident CTAs per SM
+constexpr int kC64Smem = kC64WarpB * FVG_CRS64_WARPS;
+
+struct Crs64K {
+  const i32* off;
+  const i32* idx;
+  const double* val;
+  const double* x;
+  const Item* items;
+  i64 nitems;
+  double* y;
+  double* partials;
+};
+
+__global__ void __launch_bounds__(kC64Threads, kC64Blocks) k_crs64(const Crs64K p) {
+  constexpr int NR = kWarpTile / 32, RG = FVG_CRS64_RG;
+  constexpr unsigned kFull = 0xffffffffu;
+  extern __shared__ __align__(16) unsigned char smem64[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double* xs = reinterpret_cast<double*>(smem64 + w * kC64WarpB);
+  double* vs = xs + kC64Pad;
+  unsigned* map = reinterpret_cast<unsigned*>(vs + kC64Pad);
+  unsigned short* soff = reinterpret_cast<unsigned short*>(map + kC64Map);
+  const i64 W = (i64)gridDim.x * (FVG_CRS64_WARPS), n = p.nitems;
+  const double* __restrict__ x = p.x;
+  const double* __restrict__ val = p.val;
+  // consecutive items go to different CTAs: small matrices spread over the SMs
+  i64 t = (i64)w * gridDim.x + blockIdx.x;
+  if (t >= n) return;
+  Item it = p.items[t], nx = (t + W < n) ? p.items[t + W] : Item{0, 0, 0, 0};
+  int c[NR];  // this item's column ids
+  auto fetch = [&](const Item& q) {
+    const int span = q.e1 - q.e0;
+#pragma unroll
+    for (int r = 0; r < NR; r++) {
+      const int k = r * 32 + lane;
+      c[r] = (k < span) ? __ldcs(p.idx + q.e0 + k) : 0;
+    }
+  };
+  fetch(it);
+  for (; t < n; t += W) {
+    const int a0 = it.e0, span = it.e1 - a0;
+    const Item cur = it;
+    it = nx;
+    if (t + 2 * W < n) nx = p.items[t + 2 * W];
+    if (cur.r1 < 0) {  // piece of a long row
+      double s = 0.0;  // (one warp a scheduler keeps its FP64 unit busy: no second chain)
+#pragma unroll
+      for (int g = 0; g < NR; g += RG) {
+        double xv[RG], vv[RG];
+#pragma unroll
+        for (int q = 0; q < RG; q++) {
+          const int k = (g + q) * 32 + lane;
+          xv[q] = (k < span) ? __ldg(x + c[g + q]) : 0.0;
+          vv[q] = (k < span) ? __ldcs(val + a0 + k) : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < RG; q++) s = fma(vv[q], xv[q], s);
+      }
+      if (t + W < n) fetch(it);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+      if (lane == 0) p.partials[-1 - cur.r1] = s;
+      continue;
+    }
+    const int R = cur.r1 - cur.r0;
+    // ch entries a lane; chunks start at odd multiples of 8 bytes, so that 32
+    // lanes reading their chunks' k-th entries meet no bank conflict
+    const int ch = max((span + 31) >> 5, 1), cap = 32 * ch;
+    const unsigned rcp = (ch & 1) ? 0u : (65536u + ch - 1) / ch;  // k / ch = k * rcp >> 16 for k < 1024
+    auto pos = [&](int k) { return k + (int)((unsigned)k * rcp >> 16); };
+#pragma unroll
+    for (int g = 0; g < NR; g += RG) {
+      double xv[RG], vv[RG];
+#pragma unroll
+      for (int q = 0; q < RG; q++) {
+        const int k = (g + q) * 32 + lane;
+        xv[q] = (k < span) ? __ldg(x + c[g + q]) : 0.0;
+        vv[q] = (k < span) ? __ldcs(val + a0 + k) : 0.0;
+      }
+      if (g == 0) {
+        if (lane < kC64Map) map[lane] = 0u;
+        for (int k = lane; k <= R; k += 32) soff[k] = (unsigned short)(__ldg(p.off + cur.r0 + k) - a0);
+        __syncwarp();
+        for (int j = lane; j < R; j += 32) {
+          const int s = soff[j];
+          if (soff[j + 1] > s) atomicOr(map + (s >> 5), 1u << (s & 31));
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < RG; q++) {
+        const int k = (g + q) * 32 + lane;
+        if (k < cap) {
+          xs[pos(k)] = xv[q];
+          vs[pos(k)] = vv[q];
+        }
+      }
+    }
+    if (t + W < n) fetch(it);
+    __syncwarp();
+    const int first = lane * ch;  // the lane's first entry; a 17th word pads the map
+    const unsigned marks = __funnelshift_r(map[first >> 5], map[(first >> 5) + 1], first & 31) & ((1u << ch) - 1u);
+    double* xc = xs + pos(first);
+    double S = 0.0;
+    {
+      const double* vc = vs + pos(first);
+#pragma unroll
+      for (int k = 0; k < kC64; k++) {
+        if (k >= ch) break;
+        const bool mk = (marks >> k) & 1u;
+        const double xk = xc[k], vk = vc[k];
+        if (mk) xc[k] = S;
+        S = mk ? 0.0 : S;
+        S = fma(vk, xk, S);
+      }
+    }
+    bool f = marks != 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      if (!__any_sync(kFull, !f)) break;
+      const double u = __shfl_up_sync(kFull, S, o);
+      const bool fu = __shfl_up_sync(kFull, (int)f, o) != 0;
+      if (lane >= o) {
+        S = f ? S : u + S;
+        f = f || fu;
+      }
+    }
+    // the row open at this lane's start ends at its first mark
+    const double carry = __shfl_up_sync(kFull, S, 1), last = __shfl_sync(kFull, S, 31);
+    if (lane > 0 && marks) xc[__ffs(marks) - 1] += carry;
+    __syncwarp();
+    for (int j = lane; j < R; j += 32) {
+      const int s = soff[j], e = soff[j + 1];
+      // the last row ends with the item: the scan's last value
+      p.y[cur.r0 + j] = e == s ? 0.0 : (e == span ? last : xs[pos(e)]);
+    }
+    __syncwarp();
+  }
 }
 
 // ------------------------------------------------------------- finalize
@@ -204,8 +366,6 @@ struct FinK {
   const void* partials;
   void* y;
   // logistic
-  const double* label;
-  const double* sw;
   const float* label_f;
   const float* sw_f;
   const double* intercept;
@@ -222,11 +382,42 @@ struct FinK {
   const float* ybase;
 };
 
+// The last CTA's reduction of every loss / bias partial, in a fixed order,
+// by the whole CTA: out[0] = loss, out[1] = bias (0 without an intercept).
+__device__ __forceinline__ void reduce_loss(const double* cta_part, i64 ncta, const double* long_part, i64 nlong,
+                                            int icpt, double* out, double* grad_bias, unsigned* ticket) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = (atomicAdd(ticket, 1u) == gridDim.x - 1);
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  CSum ls, bs;
+  for (i64 i = threadIdx.x; i < ncta; i += kThreads) {
+    ls.add(__ldcg(&cta_part[2 * i]));
+    bs.add(__ldcg(&cta_part[2 * i + 1]));
+  }
+  for (i64 i = threadIdx.x; i < nlong; i += kThreads) {
+    ls.add(__ldcg(&long_part[2 * i]));
+    bs.add(__ldcg(&long_part[2 * i + 1]));
+  }
+  double tl = 0, tb = 0;
+  block_csum2(ls.total(), bs.total(), &tl, &tb);
+  if (threadIdx.x == 0) {
+    out[0] = tl;
+    out[1] = icpt ? tb : 0.0;
+    if (grad_bias) *grad_bias = icpt ? tb : 0.0;
+    *ticket = 0u;
+  }
+}
+
 // Long rows: sum the pieces' partials in piece order and apply the
-// epilogue; then (logistic) the last CTA reduces every partial loss / bias
-// in a fixed order.
+// epilogue; then (logistic, FP32 sums) the last CTA reduces every partial
+// loss / bias in a fixed order.
 template <class AT, class YT, int EPI>
 __global__ void __launch_bounds__(kThreads) k_finalize(const FinK f) {
+  static_assert(EPI == EPI_STORE || sizeof(AT) == 4, "the FP64 loss rows run in k_logreg_rows");
   const AT b = (EPI == EPI_LOGREG && f.icpt) ? (AT)*f.intercept : (AT)0;
   const int lane = threadIdx.x & 31;
   // a warp per long row: lane L adds pieces L, L+32, ..., then the warp's tree
@@ -239,50 +430,39 @@ __global__ void __launch_bounds__(kThreads) k_finalize(const FinK f) {
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (lane == 0) {
       i32 row = f.long_rows[i];
-      if (EPI == EPI_STORE) {
+      if constexpr (EPI == EPI_STORE) {
         ((YT*)f.y)[row] = (YT)acc;
       } else {
         AT loss, d, wtx = acc + b;
-        if constexpr (sizeof(AT) == 4)
-          if (f.ybase) wtx += f.ybase[row];
-        if constexpr (sizeof(AT) == 8) {
-          glm_row<AT>(f.loss, (AT)f.eps, wtx, f.label[row], loss, d);
-          if (f.sw) d = d * f.sw[row];
-        } else {
-          glm_row<AT>(f.loss, (AT)f.eps, wtx, f.label_f[row], loss, d);
-          if (f.sw_f) d = d * f.sw_f[row];
-        }
+        if (f.ybase) wtx += f.ybase[row];
+        glm_row<AT>(f.loss, (AT)f.eps, wtx, f.label_f[row], loss, d);
+        if (f.sw_f) d = d * f.sw_f[row];
         ((YT*)f.r)[row] = (YT)d;
         f.long_part[2 * i] = (double)loss;
         f.long_part[2 * i + 1] = (double)d;
       }
     }
   }
-  if (EPI != EPI_LOGREG) return;
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = (atomicAdd(f.ticket, 1u) == gridDim.x - 1);
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  CSum ls, bs;
-  for (i64 i = threadIdx.x; i < f.ncta; i += kThreads) {
-    ls.add(__ldcg(&f.cta_part[2 * i]));
-    bs.add(__ldcg(&f.cta_part[2 * i + 1]));
-  }
-  for (i64 i = threadIdx.x; i < f.nlong; i += kThreads) {
-    ls.add(__ldcg(&f.long_part[2 * i]));
-    bs.add(__ldcg(&f.long_part[2 * i + 1]));
-  }
-  double tl = 0, tb = 0;
-  block_csum2(ls.total(), bs.total(), &tl, &tb);
-  if (threadIdx.x == 0) {
-    f.out[0] = tl;
-    f.out[1] = f.icpt ? tb : 0.0;
-    if (f.grad_bias) *f.grad_bias = f.icpt ? tb : 0.0;
-    *f.ticket = 0u;
-  }
+  if (EPI == EPI_LOGREG)
+    reduce_loss(f.cta_part, f.ncta, f.long_part, f.nlong, f.icpt, f.out, f.grad_bias, f.ticket);
+}
+
+// ------------------------------------------------- per-row logistic pass
+// The loss rows over a finished product z = A w (in place when wtx == r):
+// layouts whose product is computed first (ELL / JDS / hybrid) and the FP64
+// CRS pass.  A thread per row, so that all 32 lanes share each FP64
+// instruction of the loss: inside the product kernel only the lanes that
+// held a row total (12 of 32 at 40 entries a row) would.  The last CTA
+// reduces the CTAs' loss / bias partials in a fixed order.
+template <class AT>
+__global__ void __launch_bounds__(kThreads) k_logreg_rows(const AT* wtx, i64 m, const CrsK p, double* out,
+                                                          double* grad_bias, unsigned* ticket) {
+  typename SumOf<AT>::type ls, bs;
+  const AT b = p.icpt ? (AT)*p.intercept : (AT)0;
+  for (i64 r = (i64)blockIdx.x * blockDim.x + threadIdx.x; r < m; r += (i64)gridDim.x * blockDim.x)
+    epilogue<AT, AT, EPI_LOGREG>(p, (i32)r, wtx[r], b, ls, bs);
+  block_csum2(ls.total(), bs.total(), &p.cta_part[2 * blockIdx.x], &p.cta_part[2 * blockIdx.x + 1]);
+  reduce_loss(p.cta_part, gridDim.x, nullptr, 0, p.icpt, out, grad_bias, ticket);
 }
 
 // ------------------------------------------------------------- host side
@@ -315,8 +495,7 @@ static size_t carve(char* base, const Sched& s, int grid, size_t at_size, PassSc
 }
 
 i64 crs_pass_scratch_bytes(fvg_ctx* c, DevCRS& a, int storage) {
-  // pieces depend only on the item size, which FP32 and BF16 share
-  const Sched& s = crs_sched(c, a, tile_for_storage(storage));
+  const Sched& s = pass_sched(c, a, storage);
   return (i64)carve(nullptr, s, c->grid_spmv, 8, nullptr);
 }
 
@@ -365,8 +544,6 @@ static void launch_crs(fvg_ctx* c, DevCRS& a, const Sched& s, int storage, const
     f.nlong = s.nlong;
     f.partials = ps.partials;
     f.y = y;
-    f.label = p.label;
-    f.sw = p.sw;
     f.label_f = p.label_f;
     f.sw_f = p.sw_f;
     f.intercept = p.intercept;
@@ -389,9 +566,86 @@ static void launch_crs(fvg_ctx* c, DevCRS& a, const Sched& s, int storage, const
   }
 }
 
+// Raises the FP64 kernel's shared memory limit and sets its share of the
+// SM's memory, once per device.
+static void crs64_setup(fvg_ctx* c) {
+  static std::mutex mu;  // contexts of different host threads launch concurrently
+  static std::vector<int> done;
+  std::lock_guard<std::mutex> lock(mu);
+  if (std::find(done.begin(), done.end(), c->device) != done.end()) return;
+  int per_sm = 0, reserved = 0;
+  FVG_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, c->device));
+  FVG_CUDA(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, c->device));
+  FVG_CUDA(cudaFuncSetAttribute(k_crs64, cudaFuncAttributeMaxDynamicSharedMemorySize, kC64Smem));
+  const i64 need = 100ll * kC64Blocks * (kC64Smem + reserved);
+  FVG_CUDA(cudaFuncSetAttribute(k_crs64, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                (int)std::min<i64>(100, (need + per_sm - 1) / per_sm)));
+  done.push_back(c->device);
+}
+
+// y = A x, FP64 values and vectors.
+static void launch_crs64(fvg_ctx* c, DevCRS& a, const Sched& s, const void* x, void* y, void* partials,
+                         bool timed = true) {
+  if (s.nitems > 0) {
+    Crs64K p;
+    p.off = a.off.as<i32>();
+    p.idx = a.idx.as<i32>();
+    p.val = a.val[FVG_F64].as<double>();
+    p.x = (const double*)x;
+    p.items = s.items.as<Item>();
+    p.nitems = s.nitems;
+    p.y = (double*)y;
+    p.partials = (double*)partials;
+    crs64_setup(c);
+    const int grid = (int)std::min<i64>((i64)kC64Blocks * c->num_sms, s.nitems);
+    k_crs64<<<grid, kC64Threads, kC64Smem, c->stream>>>(p);
+    check_launch("k_crs64");
+    count_launch(c);
+  }
+  if (s.nlong > 0) {
+    FinK f = {};
+    f.long_rows = s.long_rows.as<i32>();
+    f.long_piece0 = s.long_piece0.as<i32>();
+    f.nlong = s.nlong;
+    f.partials = partials;
+    f.y = y;
+    const int fg = (int)std::min<i64>((s.nlong + 7) / 8, 4 * c->num_sms);  // a warp per long row
+    ProfScope pf(c, timed ? P_FINALIZE : P_NKEYS);
+    k_finalize<double, double, EPI_STORE><<<fg, kThreads, 0, c->stream>>>(f);
+    check_launch("k_finalize");
+    count_launch(c);
+  }
+}
+
+// The per-row loss pass over z (see k_logreg_rows); ticket zero on entry.
+static int logreg_rows_grid(fvg_ctx* c, i64 m) {
+  return (int)std::max<i64>(1, std::min<i64>(c->grid_spmv, (m + kThreads - 1) / kThreads));
+}
+static void launch_logreg_rows(fvg_ctx* c, const void* z, int z_dt, i64 m, const LogregEpi& lr, unsigned* ticket,
+                               double* cta_part, double* out) {
+  CrsK p = {};
+  p.label = lr.label;
+  p.sw = lr.sw;
+  p.label_f = lr.label_f;
+  p.sw_f = lr.sw_f;
+  p.intercept = lr.intercept;
+  p.icpt = lr.icpt;
+  p.r = lr.r;
+  p.cta_part = cta_part;
+  p.loss = lr.loss;
+  p.eps = lr.eps;
+  const int grid = logreg_rows_grid(c, m);
+  if (z_dt == FVG_F64)
+    k_logreg_rows<double><<<grid, kThreads, 0, c->stream>>>((const double*)z, m, p, out, lr.grad_bias, ticket);
+  else
+    k_logreg_rows<float><<<grid, kThreads, 0, c->stream>>>((const float*)z, m, p, out, lr.grad_bias, ticket);
+  check_launch("k_logreg_rows");
+  count_launch(c);
+}
+
 void crs_pass(fvg_ctx* c, DevCRS& a, int storage, int x_dt, const void* x, int y_dt, void* y, int epi,
               const LogregEpi* lr, void* scratch, int prof_key) {
-  const Sched& s = crs_sched(c, a, tile_for_storage(storage));
+  const Sched& s = pass_sched(c, a, storage);
   if (!a.val[storage].p) fail(FVG_ERR_INTERNAL, "missing value plane for the requested storage");
   const size_t at_size = (storage == FVG_F64) ? 8 : 4;
   DBuf tmp;
@@ -409,8 +663,12 @@ void crs_pass(fvg_ctx* c, DevCRS& a, int storage, int x_dt, const void* x, int y
   const int out_dt = (epi == EPI_LOGREG) ? (lr ? lr->r_dt : y_dt) : y_dt;
   if (storage == FVG_F64) {
     if (x_dt != FVG_F64 || out_dt != FVG_F64) fail(FVG_ERR_INVALID_ARG, "FP64 values need FP64 vectors");
-    if (epi == EPI_STORE) launch_crs<double, double, double, double, EPI_STORE>(c, a, s, storage, x, y, lr, ps);
-    else launch_crs<double, double, double, double, EPI_LOGREG>(c, a, s, storage, x, y, lr, ps);
+    if (epi == EPI_STORE) {
+      launch_crs64(c, a, s, x, y, ps.partials);
+    } else {  // z into r, then the loss rows in place
+      launch_crs64(c, a, s, x, lr->r, ps.partials);
+      launch_logreg_rows(c, lr->r, FVG_F64, a.m, *lr, ps.ticket, ps.cta_part, lr->out ? lr->out : ps.out);
+    }
   } else if (storage == FVG_F32) {
     if (x_dt != FVG_F32) fail(FVG_ERR_INVALID_ARG, "FP32 values need FP32 input vectors");
     if (epi == EPI_STORE && out_dt == FVG_F64)
@@ -435,7 +693,7 @@ void crs_pass(fvg_ctx* c, DevCRS& a, int storage, int x_dt, const void* x, int y
 // Returns the scratch bytes the pass needs when scratch is null.
 size_t crs_spmv_no_alloc(fvg_ctx* c, DevCRS& a, int storage, const void* x, void* y, void* scratch,
                          size_t scratch_bytes) {
-  const Sched* s = a.sched[0].get();
+  const Sched* s = a.sched[storage == FVG_F64 ? 2 : 0].get();
   if (!s) fail(FVG_ERR_INVALID_ARG, "matrix not prepared: call fvg_matrix_prepare(ctx, mat, FVG_CRS, ...) first");
   if (!a.val[storage].p) fail(FVG_ERR_INVALID_ARG, "value plane missing: call fvg_matrix_add_storage first");
   const size_t at_size = (storage == FVG_F64) ? 8 : 4;
@@ -445,7 +703,7 @@ size_t crs_spmv_no_alloc(fvg_ctx* c, DevCRS& a, int storage, const void* x, void
   PassScratch ps = {};
   ps.partials = scratch;
   if (storage == FVG_F64)
-    launch_crs<double, double, double, double, EPI_STORE>(c, a, *s, storage, x, y, nullptr, ps, false);
+    launch_crs64(c, a, *s, x, y, ps.partials, false);
   else if (storage == FVG_F32)
     launch_crs<float, float, float, float, EPI_STORE>(c, a, *s, storage, x, y, nullptr, ps, false);
   else
@@ -664,62 +922,12 @@ void sigmoid_probability(fvg_ctx* c, double* v, i64 m, double b) {
   count_launch(c);
 }
 
-// ------------------------------------------------- per-row logistic pass
-// For layouts whose product is computed first (ELL/JDS/hybrid): applies the
-// logistic epilogue to z = A w already in memory.
-template <class AT>
-__global__ void __launch_bounds__(256) k_logreg_rows(const AT* __restrict__ wtx, i64 m, const CrsK p) {
-  typename SumOf<AT>::type ls, bs;
-  const AT b = p.icpt ? (AT)*p.intercept : (AT)0;
-  for (i64 r = (i64)blockIdx.x * blockDim.x + threadIdx.x; r < m; r += (i64)gridDim.x * blockDim.x)
-    epilogue<AT, AT, EPI_LOGREG>(p, (i32)r, wtx[r], b, ls, bs);
-  block_csum2(ls.total(), bs.total(), &p.cta_part[2 * blockIdx.x], &p.cta_part[2 * blockIdx.x + 1]);
-}
-
 void logreg_rows(fvg_ctx* c, const void* wtx, int wtx_dt, i64 m, const LogregEpi& lr) {
-  int grid = (int)std::max<i64>(1, std::min<i64>(c->grid_spmv, (m + 255) / 256));
   DBuf tmp;
-  size_t need = 256 * 3 + sizeof(double) * 2 * (size_t)grid;
-  tmp.alloc(need, c->stream);
+  tmp.alloc(512 + sizeof(double) * 2 * (size_t)logreg_rows_grid(c, m), c->stream);
   FVG_CUDA(cudaMemsetAsync(tmp.p, 0, 256, c->stream));
-  unsigned* ticket = (unsigned*)tmp.p;
-  double* out = (double*)((char*)tmp.p + 256);
-  double* cta = (double*)((char*)tmp.p + 512);
-  CrsK p = {};
-  p.label = lr.label;
-  p.sw = lr.sw;
-  p.label_f = lr.label_f;
-  p.sw_f = lr.sw_f;
-  p.intercept = lr.intercept;
-  p.icpt = lr.icpt;
-  p.r = lr.r;
-  p.cta_part = cta;
-  p.loss = lr.loss;
-  p.eps = lr.eps;
-  if (wtx_dt == FVG_F64) k_logreg_rows<double><<<grid, 256, 0, c->stream>>>((const double*)wtx, m, p);
-  else k_logreg_rows<float><<<grid, 256, 0, c->stream>>>((const float*)wtx, m, p);
-  check_launch("k_logreg_rows");
-  count_launch(c);
-  FinK f = {};
-  f.nlong = 0;
-  f.label = lr.label;
-  f.sw = lr.sw;
-  f.label_f = lr.label_f;
-  f.sw_f = lr.sw_f;
-  f.intercept = lr.intercept;
-  f.icpt = lr.icpt;
-  f.r = lr.r;
-  f.cta_part = cta;
-  f.ncta = grid;
-  f.out = lr.out ? lr.out : out;
-  f.grad_bias = lr.grad_bias;
-  f.ticket = ticket;
-  f.loss = lr.loss;
-  f.eps = lr.eps;
-  if (wtx_dt == FVG_F64) k_finalize<double, double, EPI_LOGREG><<<1, kThreads, 0, c->stream>>>(f);
-  else k_finalize<float, float, EPI_LOGREG><<<1, kThreads, 0, c->stream>>>(f);
-  check_launch("k_finalize_rows");
-  count_launch(c);
+  launch_logreg_rows(c, wtx, wtx_dt, m, lr, (unsigned*)tmp.p, (double*)((char*)tmp.p + 512),
+                     lr.out ? lr.out : (double*)((char*)tmp.p + 256));
 }
 
 }  // namespace fvg
