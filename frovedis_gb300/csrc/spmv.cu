@@ -363,6 +363,7 @@ struct FinK {
   const i32* long_rows;
   const i32* long_piece0;
   i64 nlong;
+  int per_warp;  // rows a warp takes at a time: 4 or 1
   const void* partials;
   void* y;
   // logistic
@@ -412,24 +413,49 @@ __device__ __forceinline__ void reduce_loss(const double* cta_part, i64 ncta, co
   }
 }
 
-// Long rows: sum the pieces' partials in piece order and apply the
+// Long rows: sum the pieces' partials in a fixed order and apply the
 // epilogue; then (logistic, FP32 sums) the last CTA reduces every partial
-// loss / bias in a fixed order.
+// loss / bias in a fixed order.  A warp takes f.per_warp rows: 4 of 8 lanes
+// each (lane s adds pieces s, s+8, ..., then a tree), or 1.  The kernel is
+// bound by the latency of one row's chain of loads and adds, so where there
+// are more rows than warps four share it (2M x 2M power-law rows, mostly
+// under 40 pieces: 32 -> 6 us); a row of more than kFinShort pieces then takes
+// the whole warp in turn.
+constexpr i64 kFinShort = 32;
 template <class AT, class YT, int EPI>
 __global__ void __launch_bounds__(kThreads) k_finalize(const FinK f) {
   static_assert(EPI == EPI_STORE || sizeof(AT) == 4, "the FP64 loss rows run in k_logreg_rows");
   const AT b = (EPI == EPI_LOGREG && f.icpt) ? (AT)*f.intercept : (AT)0;
   const int lane = threadIdx.x & 31;
-  // a warp per long row: lane L adds pieces L, L+32, ..., then the warp's tree
-  for (i64 i = (i64)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5); i < f.nlong;
-       i += (i64)gridDim.x * (kThreads / 32)) {
-    i64 c0 = f.long_piece0[i], c1 = f.long_piece0[i + 1];
+  const int G = 32 / f.per_warp, sub = lane & (G - 1);
+  const AT* part = (const AT*)f.partials;
+  // a warp's rows lie `rows` apart: the longest rows of a matrix with sorted
+  // columns are neighbours, and land in different warps
+  const i64 rows = (f.nlong + f.per_warp - 1) / f.per_warp;
+  for (i64 b0 = (i64)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5); b0 < rows;
+       b0 += (i64)gridDim.x * (kThreads / 32)) {
+    const i64 i = b0 + (lane / G) * rows;
+    const bool valid = i < f.nlong;
+    const i32 c0 = valid ? f.long_piece0[i] : 0, c1 = valid ? f.long_piece0[i + 1] : 0;
+    const i32 row = valid ? f.long_rows[i] : 0;
+    const bool big = G < 32 && c1 - c0 > kFinShort;
     AT acc = 0;
-    for (i64 j = c0 + lane; j < c1; j += 32) acc += ((const AT*)f.partials)[j];
+    if (!big) {
+#pragma unroll 4
+      for (i32 j = c0 + sub; j < c1; j += G) acc += part[j];
+    }
+    for (int o = G / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    for (unsigned todo = __ballot_sync(0xffffffffu, big && sub == 0); todo; todo &= todo - 1) {
+      const int src = __ffs(todo) - 1;
+      const i32 d0 = __shfl_sync(0xffffffffu, c0, src), d1 = __shfl_sync(0xffffffffu, c1, src);
+      AT s = 0;
+#pragma unroll 4
+      for (i32 j = d0 + lane; j < d1; j += 32) s += part[j];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) {
-      i32 row = f.long_rows[i];
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == src) acc = s;
+    }
+    if (valid && sub == 0) {
       if constexpr (EPI == EPI_STORE) {
         ((YT*)f.y)[row] = (YT)acc;
       } else {
@@ -499,6 +525,14 @@ i64 crs_pass_scratch_bytes(fvg_ctx* c, DevCRS& a, int storage) {
   return (i64)carve(nullptr, s, c->grid_spmv, 8, nullptr);
 }
 
+// Long rows a warp of k_finalize takes at a time: one while every row can
+// have a warp of its own, four above that (4,864 rows on 152 SMs).
+static int fin_rows(fvg_ctx* c, const Sched& s) { return s.nlong > 4ll * c->num_sms * (kThreads / 32) ? 4 : 1; }
+static int fin_grid(fvg_ctx* c, const Sched& s) {
+  const i64 per_cta = (i64)fin_rows(c, s) * (kThreads / 32);
+  return (int)std::max<i64>(1, std::min<i64>((s.nlong + per_cta - 1) / per_cta, 4 * c->num_sms));
+}
+
 template <class VT, class XT, class AT, class YT, int EPI>
 static int crs_grid(fvg_ctx* c, int tile) {
   (void)tile;
@@ -558,7 +592,8 @@ static void launch_crs(fvg_ctx* c, DevCRS& a, const Sched& s, int storage, const
     f.ticket = ps.ticket;
     f.loss = p.loss;
     f.eps = p.eps;
-    int fg = (int)std::max<i64>(1, std::min<i64>((s.nlong + 7) / 8, 4 * c->num_sms));  // a warp per long row
+    f.per_warp = fin_rows(c, s);
+    const int fg = fin_grid(c, s);
     ProfScope pf(c, timed ? P_FINALIZE : P_NKEYS);
     k_finalize<AT, YT, EPI><<<fg, kThreads, 0, c->stream>>>(f);
     check_launch("k_finalize");
@@ -609,7 +644,8 @@ static void launch_crs64(fvg_ctx* c, DevCRS& a, const Sched& s, const void* x, v
     f.nlong = s.nlong;
     f.partials = partials;
     f.y = y;
-    const int fg = (int)std::min<i64>((s.nlong + 7) / 8, 4 * c->num_sms);  // a warp per long row
+    f.per_warp = fin_rows(c, s);
+    const int fg = fin_grid(c, s);
     ProfScope pf(c, timed ? P_FINALIZE : P_NKEYS);
     k_finalize<double, double, EPI_STORE><<<fg, kThreads, 0, c->stream>>>(f);
     check_launch("k_finalize");
