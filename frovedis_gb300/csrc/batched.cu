@@ -764,6 +764,7 @@ struct BatchEval {
     s1.alloc((size_t)s1b, s);
     s2.alloc((size_t)s2b, s);
     slots.alloc((size_t)spmm_seg_slot_bytes(c, nd, std::min(ld, 64)), s);
+    spmm_seg_init(c, slots.p, nd);
     std::vector<i32> sr((size_t)nd + 1);
     std::vector<i64> gr((size_t)nd);
     for (int d = 0; d <= nd; d++) sr[d] = (i32)roff[d];

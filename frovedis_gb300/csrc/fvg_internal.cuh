@@ -417,6 +417,7 @@ struct SpmmSeg {
   int nc = 0, icpt = 0;
 };
 i64 spmm_seg_slot_bytes(fvg_ctx* c, int nseg, int kb);
+void spmm_seg_init(fvg_ctx* c, void* slots, int nseg);  // once, before the first pass
 void crs_spmm_logreg_seg(fvg_ctx* c, DevCRS& a, int storage, const void* W, i64 ldw, int kb, const double* label,
                          const double* sw, const float* label_f, const float* sw_f, int icpt, const double* bias,
                          void* R, i64 ldr, void* scratch, SpmmSeg& sg, int loss = 0, double eps = 0.0);

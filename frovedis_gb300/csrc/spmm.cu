@@ -15,6 +15,8 @@
 // finalize kernel adds them in piece order.  Loss and bias sums of the
 // logistic epilogue are compensated per lane, then combined per CTA and
 // across CTAs in a fixed order (deterministic).
+#include <type_traits>
+
 #include "device_common.cuh"
 
 namespace fvg {
@@ -474,7 +476,7 @@ __global__ void __launch_bounds__(kThreads) k_spmm_fin(const SpmmFin f) {
     spmm_epi<AT, YT, EPI, CPL, VEC>(p, row, a, b, lane, ls, bs, mw);
   }
   if (track && !seg) return;
-  if (seg) {
+  if (seg && p.nseg > 1) {
     sw.finish(p, cols, ls, bs);
     return;
   }
@@ -493,8 +495,9 @@ __global__ void __launch_bounds__(kThreads) k_spmm_fin(const SpmmFin f) {
       double t = 0;
 #pragma unroll
       for (int w = 0; w < kThreads / 32; w++) t += red[w][col][qq];
-      f.fin_part[((i64)blockIdx.x * NC + col) * 2 + qq] = t;
+      (seg ? f.seg_fpart : f.fin_part)[((i64)blockIdx.x * NC + col) * 2 + qq] = t;
     }
+    if (seg) return;  // one stacked dataset: a slot per CTA
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last = (atomicAdd(f.ticket, 1u) == gridDim.x - 1);
@@ -803,10 +806,11 @@ __global__ void __launch_bounds__(kThreads, 4) k_spmm_g(const SpmmK p) {
   if (track && !seg) return;
   if constexpr (EPI == EPI_LOGREG || EPI == EPI_SOFTMAX) {
     if (EPI == EPI_SOFTMAX && !p.cta_part) return;
-    if (seg) {
+    if (seg && p.nseg > 1) {
       walk.finish(p, cols, ls, bs);
       return;
     }
+    // one dataset (stacked or not): the CTA's warps added in order
     __shared__ double red[kThreads / 32][NC][2];
 #pragma unroll
     for (int q = 0; q < QG; q++) {
@@ -819,41 +823,60 @@ __global__ void __launch_bounds__(kThreads, 4) k_spmm_g(const SpmmK p) {
       double t = 0;
 #pragma unroll
       for (int w8 = 0; w8 < kThreads / 32; w8++) t += red[w8][col][qq];
-      p.cta_part[((i64)blockIdx.x * NC + col) * 2 + qq] = t;
+      (seg ? p.seg_part : p.cta_part)[((i64)blockIdx.x * NC + col) * 2 + qq] = t;
     }
   }
 }
 
-// Stacked datasets: loss / bias sums of dataset blockIdx.x from the warp
-// slots of the main kernel (nw1 warps) and the finalize kernel (nw2), each
-// in warp order.  A CTA of 1024 threads takes 32 (column, quantity) pairs
-// (blockIdx.y: which 32) x 32 stripes; stripe s adds warps s, s + 32, ...;
-// the stripes are added in order.  out[2 * (d * ldo + col) + q]; the bias
-// sums also go to gb[grow[d] * ldg + col].
+// Stacked datasets: loss / bias sums of dataset blockIdx.x from the slots of
+// the main kernel (nw1 slots: its warps, or its CTAs when one dataset is
+// stacked) and of the finalize kernel (nw2), in a fixed order.  A compensated
+// FP64 add costs five FP64 instructions, so the slots are spread over
+// gridDim.z CTAs: CTA (d, y, z) takes the 32 (column, quantity) pairs of y in
+// 8 stripes, stripe s the slots z*8 + s, + 8 * gridDim.z, ...; the last CTA of
+// (d, y) adds the CTAs' sums in order.  out[2 * (d * ldo + col) + q]; the bias
+// sums also go to gb[grow[d] * ldg + col].  One dataset of 200,000 rows, 64
+// models, averaged over the launches of a training (half of them gated off):
+// 1.8 us; one CTA per 32 pairs over a slot per warp took 27.8 us.
+constexpr int kSegZ = 16;  // most CTAs per (dataset, 32 pairs)
 template <int NC>
-__global__ void __launch_bounds__(1024) k_spmm_seg_reduce(const double* __restrict__ s1, i64 nw1,
-                                                          const double* __restrict__ s2, i64 nw2, int kout, int icpt,
-                                                          double* __restrict__ out, i64 ldo, double* __restrict__ gb,
-                                                          const i64* __restrict__ grow, i64 ldg, const int* gate,
-                                                          const unsigned long long* mask, i64 mstride, int mword) {
-  constexpr int P = 2 * NC, S = 32;
+__global__ void __launch_bounds__(256) k_spmm_seg_reduce(const double* __restrict__ s1, i64 nw1,
+                                                         const double* __restrict__ s2, i64 nw2, int kout, int icpt,
+                                                         double* __restrict__ out, i64 ldo, double* __restrict__ gb,
+                                                         const i64* __restrict__ grow, i64 ldg, const int* gate,
+                                                         const unsigned long long* mask, i64 mstride, int mword,
+                                                         double* __restrict__ rpart, unsigned* __restrict__ tickets) {
+  constexpr int P = 2 * NC, S = 8;
   static_assert(P % 32 == 0, "pairs per CTA");
   __shared__ double part[S][33];
+  __shared__ bool last;
   if (gated_off(gate)) return;
-  const int d = blockIdx.x;
+  const int d = blockIdx.x, dy = d * gridDim.y + blockIdx.y, Z = gridDim.z;
   const int pl = threadIdx.x & 31, st = threadIdx.x >> 5;
   const int pr = blockIdx.y * 32 + pl;
   CSum t;
-  const double* b1 = s1 + (i64)d * nw1 * P;
-  for (i64 w = st; w < nw1; w += S) t.add(__ldcg(b1 + w * P + pr));
-  const double* b2 = s2 + (i64)d * nw2 * P;
-  for (i64 w = st; w < nw2; w += S) t.add(__ldcg(b2 + w * P + pr));
+  const double* b1 = s1 + (i64)d * nw1 * P + pr;
+  const double* b2 = s2 + (i64)d * nw2 * P + pr;
+  for (i64 w = blockIdx.z * S + st; w < nw1 + nw2; w += S * Z) t.add(w < nw1 ? __ldcg(b1 + w * P) : __ldcg(b2 + (w - nw1) * P));
   part[st][pl] = t.total();
   __syncthreads();
   if (st != 0) return;
   double tot = 0.0;
 #pragma unroll
   for (int q = 0; q < S; q++) tot += part[q][pl];
+  if (Z > 1) {
+    double* rp = rpart + (i64)dy * kSegZ * 32;
+    rp[blockIdx.z * 32 + pl] = tot;
+    __threadfence();
+    __syncwarp();
+    if (pl == 0) last = atomicAdd(tickets + dy, 1u) == (unsigned)Z - 1;
+    __syncwarp();
+    if (!last) return;
+    __threadfence();
+    tot = 0.0;
+    for (int z = 0; z < Z; z++) tot += __ldcg(rp + z * 32 + pl);
+    if (pl == 0) tickets[dy] = 0u;
+  }
   const int col = pr >> 1, qq = pr & 1;
   if (col >= kout) return;
   if (mask && !col_on(__ldcg(mask + (i64)d * mstride + mword), col)) return;  // not evaluated: keep
@@ -930,6 +953,16 @@ static void launch_spmm_l(fvg_ctx* c, DevCRS& a, const Sched& s, int storage, Sp
 
 static bool aligned_to(const void* ptr, size_t b) { return ((uintptr_t)ptr % b) == 0; }
 
+// Scratch of a stacked-dataset pass (SpmmSeg::slots): the reduction's tickets
+// (zeroed once by spmm_seg_init) and its CTAs' sums, then the slots.
+constexpr int kSegY = 2 * kSpmmMaxCols / 32;  // 32-pair groups of the widest block
+static i64 seg_ticket_bytes(int nseg) { return (i64)al256(sizeof(unsigned) * kSegY * (size_t)nseg); }
+static i64 seg_part_bytes(int nseg) { return (i64)sizeof(double) * kSegY * kSegZ * 32 * nseg; }
+static double* seg_parts(const SpmmSeg& sg) { return (double*)((char*)sg.slots + seg_ticket_bytes(sg.nseg)); }
+static double* seg_slots(const SpmmSeg& sg) {
+  return (double*)((char*)sg.slots + seg_ticket_bytes(sg.nseg) + seg_part_bytes(sg.nseg));
+}
+
 // Grouped layout launch: k_spmm_g and its finalize kernel (NC / 32
 // columns a lane); for stacked datasets the slot reduction is left to
 // crs_spmm_seg_finish.
@@ -956,7 +989,10 @@ static void launch_grouped_l(fvg_ctx* c, DevCRS& a, const Sched& s, int storage,
   p.cta_part = reduce ? cta : nullptr;
   const bool track = sg && sg->nseg > 0;
   const bool seg = EPI == EPI_LOGREG && track;
-  const i64 nw1 = (i64)grid * (kThreads / 32), nw2 = (i64)fg * (kThreads / 32);
+  // slots of a stacked dataset: a warp each, or with one dataset a CTA each
+  const i64 per = track && sg->nseg == 1 ? 1 : kThreads / 32;
+  const i64 nw1 = grid * per, nw2 = fg * per;
+  double* const slots = seg ? seg_slots(*sg) : nullptr;
   if (track) {
     if (!sg->seg_row || (seg && !sg->slots) || sg->nseg > 65535)
       fail(FVG_ERR_INTERNAL, "stacked-dataset pass without its row bounds or slots");
@@ -964,7 +1000,7 @@ static void launch_grouped_l(fvg_ctx* c, DevCRS& a, const Sched& s, int storage,
     p.nseg = sg->nseg;
     p.seg_row = sg->seg_row;
     p.ldb = sg->ldb;
-    p.seg_part = seg ? sg->slots : nullptr;
+    p.seg_part = slots;
     p.gate = sg->gate;
     p.mask = sg->mask;
     p.mstride = sg->mstride;
@@ -986,7 +1022,7 @@ static void launch_grouped_l(fvg_ctx* c, DevCRS& a, const Sched& s, int storage,
     f.out = out;
     f.gbias = gbias;
     f.ticket = ticket;
-    f.seg_fpart = seg ? sg->slots + (i64)sg->nseg * nw1 * NC * 2 : nullptr;
+    f.seg_fpart = seg ? slots + (i64)sg->nseg * nw1 * NC * 2 : nullptr;
     k_spmm_fin<AT, YT, EPI, CF, true><<<fg, kThreads, 0, c->stream>>>(f);
     check_launch("k_spmm_fin");
     count_launch(c);
@@ -1165,7 +1201,12 @@ void crs_spmm_logreg_block(fvg_ctx* c, DevCRS& a, int storage, const void* W, i6
 i64 spmm_seg_slot_bytes(fvg_ctx* c, int nseg, int kb) {
   const i64 nc = kb <= 32 ? 32 : (kb <= 64 ? 64 : 128);
   const i64 warps = (8 * (i64)c->num_sms + 2 * (i64)c->num_sms) * (kThreads / 32);
-  return (i64)std::max(nseg, 1) * warps * nc * 2 * (i64)sizeof(double);
+  const int ns = std::max(nseg, 1);
+  return seg_ticket_bytes(ns) + seg_part_bytes(ns) + ns * warps * nc * 2 * (i64)sizeof(double);
+}
+
+void spmm_seg_init(fvg_ctx* c, void* slots, int nseg) {
+  FVG_CUDA(cudaMemsetAsync(slots, 0, (size_t)seg_ticket_bytes(std::max(nseg, 1)), c->stream));
 }
 
 void crs_spmm_logreg_seg(fvg_ctx* c, DevCRS& a, int storage, const void* W, i64 ldw, int kb, const double* label,
@@ -1203,19 +1244,19 @@ void crs_spmm_logreg_seg(fvg_ctx* c, DevCRS& a, int storage, const void* W, i64 
 // the backward product, which writes the bias rows of the gradient as 0).
 void crs_spmm_seg_finish(fvg_ctx* c, const SpmmSeg& sg) {
   if (sg.nw1 <= 0) fail(FVG_ERR_INTERNAL, "stacked-dataset reduction without its pass");
-  const double* s2 = sg.slots + (i64)sg.nseg * sg.nw1 * sg.nc * 2;
-  if (sg.nc == 32)
-    k_spmm_seg_reduce<32><<<dim3(sg.nseg, 2), 1024, 0, c->stream>>>(sg.slots, sg.nw1, s2, sg.nw2, sg.kout, sg.icpt, sg.out,
-                                                           sg.ldo, sg.gb, sg.grow, sg.ldg, sg.gate, sg.mask,
-                                                           sg.mstride, sg.mword);
-  else if (sg.nc == 64)
-    k_spmm_seg_reduce<64><<<dim3(sg.nseg, 4), 1024, 0, c->stream>>>(sg.slots, sg.nw1, s2, sg.nw2, sg.kout, sg.icpt, sg.out,
-                                                           sg.ldo, sg.gb, sg.grow, sg.ldg, sg.gate, sg.mask,
-                                                           sg.mstride, sg.mword);
-  else
-    k_spmm_seg_reduce<128><<<dim3(sg.nseg, 8), 1024, 0, c->stream>>>(sg.slots, sg.nw1, s2, sg.nw2, sg.kout, sg.icpt, sg.out,
-                                                            sg.ldo, sg.gb, sg.grow, sg.ldg, sg.gate, sg.mask,
-                                                           sg.mstride, sg.mword);
+  const double* s1 = seg_slots(sg);
+  const double* s2 = s1 + (i64)sg.nseg * sg.nw1 * sg.nc * 2;
+  // at least 64 slots a CTA: 8 a thread
+  const unsigned z = (unsigned)std::max<i64>(1, std::min<i64>(kSegZ, (sg.nw1 + sg.nw2) / 64));
+  auto launch = [&](auto nc) {
+    constexpr int NC = decltype(nc)::value;
+    k_spmm_seg_reduce<NC><<<dim3(sg.nseg, 2 * NC / 32, z), 256, 0, c->stream>>>(
+        s1, sg.nw1, s2, sg.nw2, sg.kout, sg.icpt, sg.out, sg.ldo, sg.gb, sg.grow, sg.ldg, sg.gate, sg.mask,
+        sg.mstride, sg.mword, seg_parts(sg), (unsigned*)sg.slots);
+  };
+  if (sg.nc == 32) launch(std::integral_constant<int, 32>{});
+  else if (sg.nc == 64) launch(std::integral_constant<int, 64>{});
+  else launch(std::integral_constant<int, 128>{});
   check_launch("k_spmm_seg_reduce");
   count_launch(c);
 }
