@@ -213,7 +213,7 @@ static const Sched& build_sched(fvg_ctx* c, DevCRS& a, int slot, int tile, int l
   const i64 m = a.m;
   const i64 nchunks = std::max<i64>(1, (m + kSchedChunk - 1) / kSchedChunk);
   PackOut o;
-  device_pack(c, a.off.as<i32>(), m, kSchedChunk, nchunks, tile, o, 1, lane_work);
+  device_pack(c, a.off.as<i32>(), m, kSchedChunk, nchunks, tile, o, lane_work);
   s->nitems = o.nitems;
   s->nlong = o.nlong;
   s->npieces = o.npieces;

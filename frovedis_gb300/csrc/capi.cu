@@ -328,11 +328,13 @@ FVG_API fvg_status fvg_matrix_prepare(fvg_ctx* c, fvg_matrix* M, fvg_format fmt,
   if (with_transpose && (fmt == FVG_CRS || fmt == FVG_ELL) && (M->A.val[FVG_F32].p || M->A.val[FVG_BF16].p)) {
     DevPanels* pt = panels_for(c, M);
     DevPanels* hd = fmt == FVG_CRS ? head_for(c, M) : nullptr;
-    for (int dt : {FVG_F32, FVG_BF16})
-      if (M->A.val[dt].p) {
-        if (pt) panel_ensure_plane(c, *pt, dt);
-        if (hd) head_ensure_plane(c, *hd, dt);
-      }
+    const bool split = M->A.lo.p != nullptr;  // its FP32 plane belongs to the split values
+    for (DevPanels* p : {pt, hd}) {
+      if (!p) continue;
+      if (split) panel_ensure_split(c, *p);
+      for (int dt : {FVG_F32, FVG_BF16})
+        if (M->A.val[dt].p && !(split && dt == FVG_F32)) panel_ensure_plane(c, *p, dt);
+    }
   }
   FVG_CUDA(cudaStreamSynchronize(c->stream));
   API_END(c)
@@ -459,9 +461,11 @@ FVG_API int64_t fvg_matrix_device_bytes(const fvg_matrix* M) {
   for (const DevPanels* p : {M->pan.get(), M->head.get()}) {
     if (!p) continue;
     b += crs_bytes(p->cold);
-    for (const DBuf* d : {&p->hot_cols, &p->poff, &p->prow, &p->items, &p->pitem0, &p->long_rows, &p->plong0,
-                          &p->long_piece0, &p->ypan, &p->partials})
+    for (const DBuf* d : {&p->hot_cols, &p->poff, &p->prow, &p->lo, &p->coff, &p->vout, &p->vsrc, &p->vlen, &p->wstart,
+                          &p->ulong0, &p->long_rows, &p->long_piece0, &p->ypan, &p->partials, &p->ypan2,
+                          &p->partials2})
       b += (int64_t)d->bytes;
+    for (auto& r : p->rec) b += (int64_t)r.bytes;
     for (auto& v : p->val) b += (int64_t)v.bytes;
   }
   return b;

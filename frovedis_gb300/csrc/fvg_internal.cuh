@@ -74,11 +74,8 @@ constexpr int kTileRows = 248;  // rows per tile (their offsets are staged in sh
 constexpr int kLaneWork = 32;   // products one lane may sum for one row in a tile
 // Rows one warp of the work-item packer takes (a tile never spans two such
 // chunks): short enough that the packers' tile after tile walks take a few
-// microseconds, long enough to fill kTileRows-row tiles.  The
-// panel and head layouts' rows are shorter (their items hold more rows), so
-// they are packed in longer chunks.
+// microseconds, long enough to fill kTileRows-row tiles.
 constexpr i64 kPackRows = 256;
-constexpr i64 kPanelPackRows = 1024;
 // Lanes per row when a warp sums a tile of R rows: 32 / R rounded to a power
 // of two; tiles of 32 or more rows take rounds of 32 rows, one lane each.
 __host__ __device__ __forceinline__ int lanes_per_row(int R) {
@@ -167,14 +164,6 @@ struct DevHYB {  // jds_crs_hybrid_local (jds_crs_hybrid.hpp:8-153)
   bool all_crs = false;  // m <= threshold: the whole matrix is the CRS part
 };
 
-// Work items over a panel layout's rows, panel by panel (Item as in Sched):
-// a panel's items start at pitem0[panel], its long rows at plong0[panel].
-struct PanelItems {
-  int tile = 0;
-  i64 nitems = 0, nlong = 0, npieces = 0;
-  DBuf items, pitem0, long_rows, plong0, long_piece0;
-};
-
 // Row-panel layout of the backward product g = A^T r (FP32 arithmetic).
 // A's rows are cut into panels of `rows` consecutive rows; a CTA stages one
 // panel's slice of r in shared memory and sums, for every hot column h, the
@@ -195,15 +184,16 @@ struct DevPanels {
   DBuf val[3];                      // [E + kPad] per dtype
   DBuf lo;                          // bf16 [E + kPad]: residual of the FP32 values (split storage)
   DevCRS cold;                      // n rows, hot rows empty
-  // work items over the panel rows, panel by panel (Item as in Sched)
-  i64 nitems = 0, nlong = 0, npieces = 0;
-  DBuf items, pitem0, long_rows, plong0, long_piece0;
-  DBuf ypan;                        // float [npanels*nhot]
-  DBuf partials;                    // float [npieces]
-  // split storage: its own work items (smaller staging buffers) and df-pair
-  // partial sums (float2)
-  std::unique_ptr<PanelItems> split_items;
-  DBuf ypan2, partials2;
+  // streamed layout of the panel rows (panel.cu): segments of at most 64
+  // entries, sorted by length within a panel, in slices of 32 lanes
+  i64 group = 1, nunits = 0;        // panels a CTA takes at a time, such units
+  i64 nslices = 0, nchunks = 0;
+  DBuf coff, vout, vsrc, vlen, wstart;
+  i64 nlong = 0, npieces = 0;       // panel rows of several segments
+  DBuf ulong0, long_rows, long_piece0;
+  DBuf rec[4];                      // records by value storage (FVG_F32, FVG_BF16, FVG_SPLIT)
+  DBuf ypan, partials;              // float [npanels*nhot], [npieces]
+  DBuf ypan2, partials2;            // df pairs (float2), split storage
   // forward head (shared = true): every CTA stages w at the columns
   // hot_cols[0..rows) once; panels are stretches of nhot rows of A; `cold`
   // holds the rest of each row (m rows, int32 column ids)
@@ -218,12 +208,10 @@ struct PackOut {
   DBuf items, long_rows, long_piece0;
   std::vector<i32> base;
 };
-// Each chunk may itself be packed in `sub` pieces (a warp each; items never
-// span two pieces); base then has nchunks*sub+1 entries per kind.
 // lane_work: products one lane may sum for one row of a tile (kLaneWork, or
 // kNoLaneWork for kernels that cut the rows among the lanes by entries).
 constexpr int kNoLaneWork = 1 << 20;
-void device_pack(fvg_ctx* c, const i32* off, i64 nrows, i64 chunk, i64 nchunks, int tile, PackOut& o, i64 sub = 1,
+void device_pack(fvg_ctx* c, const i32* off, i64 nrows, i64 chunk, i64 nchunks, int tile, PackOut& o,
                  int lane_work = kLaneWork);
 
 struct Profiler;

@@ -9,10 +9,9 @@
 // bytes, so that pass is bound by L2-to-SM traffic, far below HBM speed.
 // The row-panel layout regroups the columns that occur in most stretches of
 // rows.  A's rows are cut into panels of `rows` consecutive rows.  A CTA
-// copies one panel's slice of r into shared memory and walks the panel's
-// entries of the hot columns in (column, row) order, gathering from shared
-// memory; each (panel, hot column) pair gives one FP32 partial sum ("panel
-// row" q = panel * nhot + h).  g[hot column] is the compensated sum of its
+// copies one panel's slice of r into shared memory and streams the panel's
+// entries of the hot columns, gathering from shared memory; each (panel, hot
+// column) pair gives one partial sum ("panel row" q = panel * nhot + h).  g[hot column] is the compensated sum of its
 // partials in a fixed order.  Columns with fewer entries keep their rows in
 // a transposed CRS of their own (the hot rows emptied), multiplied by the
 // plain CRS kernel first.
@@ -44,13 +43,25 @@ unsigned grid_n(i64 n, int threads = 256) {
   if (g > 152 * 32) g = 152 * 32;
   return (unsigned)(g < 1 ? 1 : g);
 }
+// Warps of the streamed product, bulk copies in flight per warp, chunks a copy
+// (build-time knobs; the defaults are the measured best).
+#ifndef FVG_STREAM_WARPS
+#define FVG_STREAM_WARPS 20
+#endif
+#ifndef FVG_STREAM_STAGES
+#define FVG_STREAM_STAGES 2
+#endif
+#ifndef FVG_STREAM_CHUNKS
+#define FVG_STREAM_CHUNKS 2
+#endif
 #define PGRID_STRIDE(i, n) for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += (i64)gridDim.x * blockDim.x)
 #define PWARP_STRIDE(q, n)                                                              \
   for (i64 q = ((i64)blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < (n);             \
        q += ((i64)gridDim.x * blockDim.x) >> 5)
 
-constexpr int kPanelWarps = 32;          // one CTA of 32 warps per SM
-constexpr i64 kPanelRowsAuto = 1 << 30;  // auto: the tallest panels shared memory holds
+constexpr i64 kPanelMinRows = 4096;      // auto: shortest panels
+constexpr i64 kPanelMinMatrix = 76800;   // auto: rows of a matrix that gets panels
+constexpr i64 kHeadMinMatrix = 311296;   // auto: rows of a matrix that gets a head
 constexpr double kPanelMinAuto = 2.0;    // hot: >= this many entries per panel on average
 
 // ------------------------------------------------------------------ build
@@ -146,8 +157,8 @@ __global__ void k_cold_fill(const i32* __restrict__ toff, const i64* __restrict_
   }
 }
 
-// Work items of a CRS, one warp per chunk of rows (chunk p: piece p % sub
-// of the stretch of nhot rows p / sub), with the CRS schedule's packing rules
+// Work items of a CRS, one warp per chunk of `step` rows (at most kPackRows),
+// with the CRS schedule's packing rules
 // (tiles of short rows within `tile` entries, kTileRows rows and lane_work
 // products per lane; longer rows in pieces cut at 8-element boundaries).  The
 // greedy packing is sequential from tile to tile, but the rows of one tile
@@ -161,21 +172,19 @@ __global__ void k_cold_fill(const i32* __restrict__ toff, const i64* __restrict_
 // read from shared memory: 44 us a pass over the transposed 25,600 x 20,000
 // minibatches of a Zipf matrix (a thread walking each chunk row by row: 97 us).
 constexpr int kPackThreads = 128;
-__global__ void __launch_bounds__(kPackThreads) k_panel_pack(const i32* __restrict__ off, i64 nrows, i64 nhot, i64 sub, i64 np,
-                                                    int tile, int write, i32* __restrict__ cnt,
+__global__ void __launch_bounds__(kPackThreads) k_pack(const i32* __restrict__ off, i64 nrows, i64 step, i64 np, int tile,
+                                                    int write, i32* __restrict__ cnt,
                                                     const i32* __restrict__ base, Item* __restrict__ items,
                                                     i32* __restrict__ lrows, i32* __restrict__ lpiece0,
                                                     i32* __restrict__ lfirst, int lane_work) {
-  __shared__ i32 soff[kPackThreads / 32][kPanelPackRows + 1];
-  const i64 step = (nhot + sub - 1) / sub;
+  __shared__ i32 soff[kPackThreads / 32][kPackRows + 1];
   const int lane = threadIdx.x & 31;
   i32* so = soff[threadIdx.x >> 5];
   PWARP_STRIDE(p, np) {
-    const i64 s0 = (p / sub) * nhot, s1 = min(s0 + nhot, nrows), jc = p % sub;
-    const i64 r0 = min(s0 + jc * step, s1), r1 = min(r0 + step, s1);
+    const i64 r0 = min(p * step, nrows), r1 = min(r0 + step, nrows);
     __syncwarp();
 #pragma unroll 8
-    for (int q = lane; q <= (int)(r1 - r0); q += 32) so[q] = __ldg(off + r0 + q);  // step <= kPanelPackRows
+    for (int q = lane; q <= (int)(r1 - r0); q += 32) so[q] = __ldg(off + r0 + q);
     __syncwarp();
     const i32 bi = write ? base[p] : 0, bl = write ? base[(np + 1) + p] : 0, bp = write ? base[2 * (np + 1) + p] : 0;
     i32 ni = 0, nl = 0, npc = 0;
@@ -349,200 +358,419 @@ __global__ void k_head_fill(const i32* __restrict__ off, const i32* __restrict__
 }
 
 // ---------------------------------------------------------------- product
-struct PanK {
-  const i32* poff;
-  const uint16_t* prow;
-  const void* val;
-  const float* r;
-  i64 m, rows, npanels;
-  const Item* items;
-  const i32* pitem0;
+// Streamed layout.  A panel row's entries are cut into segments of at most
+// kSegChunks chunks of 4 entries; a panel's segments are sorted by length
+// (stable, longest first) and dealt in slices of 32, a lane each.  Chunk c of
+// a slice is one record: for every lane the 4 values (and BF16 residuals) and
+// the 4 slots of its segment's entries 4c .. 4c+3, each kind contiguous over
+// the lanes.  Segments that end earlier are padded with value 0 and the slot
+// `rows`, whose staged vector entry is 0.  A warp's share of a panel is a run
+// of slices, so it reads one contiguous stretch of memory; a lane adds its own
+// segment from front to back and nothing is exchanged between lanes.
+// (Measured against staging 480 entries a warp in row order, cutting them
+// among the lanes by position and joining the rows with marks, selects and a
+// segmented scan: that took 69 warp instructions per 32 entries of split
+// values, this 30.  10M x 1M split values, 4.7e8 head and 4.9e8 panel entries:
+// 1.12 + 1.29 ms before with 11,000-entry slices, 0.81 + 0.82 ms now with
+// 16,400 to 18,800, 5.4 TB/s of records, rows and sums; 2M x 200,000 BF16
+// values: 135 -> 124 us.  More copies in flight, larger copies, and records
+// asked into L2 ahead of the copies change nothing or cost time, as does
+// leaving out the gathers or the sums: the split stream is bound by HBM.  The
+// BF16 one, half the bytes a chunk, is bound by the chain of a warp's copies:
+// 8 / 16 / 24 warps take 188 / 124 / 113 us, but the split rings of 24 warps
+// leave too small a slice, and one layout serves every storage.)
+constexpr int kStreamWarps = FVG_STREAM_WARPS;    // one CTA per SM
+constexpr int kStreamStages = FVG_STREAM_STAGES;  // copies in flight per warp
+constexpr int kStreamChunks = FVG_STREAM_CHUNKS;  // chunks of one copy
+constexpr int kSegChunks = 16;                    // longest segment: 64 entries
+constexpr int kAhead = 4;                         // slices whose row numbers are loaded early (a power of two)
+constexpr i32 kNoRow = (i32)0x80000000;           // lane without a segment
+
+// Record of a chunk by value storage: bytes of the values, residuals, slots.
+template <int ST> struct StreamRec {
+  using X = std::conditional_t<ST == FVG_SPLIT, float2, float>;  // vector entry
+  static constexpr int kValB = (ST == FVG_BF16 ? 2 : 4) * 128;
+  static constexpr int kLoB = ST == FVG_SPLIT ? 256 : 0;
+  static constexpr int kB = kValB + kLoB + 256;
+  static constexpr int kBarB = (8 * kStreamWarps * kStreamStages + 127) / 128 * 128;
+  static constexpr int kRingB = kStreamStages * kStreamChunks * kB;  // per warp
+  static constexpr int kStatic = kBarB + kStreamWarps * (kRingB + kAhead * 128);
+};
+
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+struct StreamK {
+  const unsigned char* rec;
+  const i32* coff;    // first chunk of each slice
+  const i32* vout;    // [slices][32]: panel row, ~piece, or kNoRow
+  const i32* wstart;  // [units][kStreamWarps + 1]: first slice of each warp
+  const i32* ulong0;  // [units + 1]: first long row of each unit
   const i32* long_rows;
-  const i32* plong0;
   const i32* long_piece0;
-  float* partials;
-  float* ypan;
+  const void* x;
+  const i32* xmap;  // forward head: the slice is x[xmap[0..rows)], staged once
+  i64 m, rows;
+  i64 nunits;
+  void* ypan;
+  void* partials;
   unsigned* err;
   unsigned wait_limit;  // poll budget of the copy waits
-  int aligned;  // r is 16-byte aligned: the slice is staged with 16-byte loads
-  // forward head: every CTA stages the same slice r[xmap[0..rows)] once
-  // (the frequent columns of w), panels are stretches of A's rows
-  const i32* xmap;
-  i64 group;  // consecutive panels a CTA takes at a time
+  int aligned;          // x is 16-byte aligned
 };
 
+__device__ __forceinline__ df shfl_xor_df(df a, int o) {
+  return {__shfl_xor_sync(0xffffffffu, a.h, o), __shfl_xor_sync(0xffffffffu, a.l, o)};
+}
 
-// Shared memory of one CTA: per warp one staging buffer for a work item's
-// entries (panel rows as uint16, then the values; the item's products are
-// later written over it) with its mbarrier and the tile's row offsets; then
-// the panel's slice of r.
-template <class VT> struct PanelSmem {
-  static constexpr int kCap = kWarpTile + 16;  // entries of one copy: 16-byte aligned ends
-  static constexpr int kIdxB = kCap * 2;
-  static constexpr int kStageB = kIdxB + kCap * (int)sizeof(VT);  // >= kCap * 4: room for the products
-  static constexpr int kSoffB = ((kTileRows + 1) * 2 + 15) / 16 * 16;
-  static constexpr int kWarpB = kStageB + kSoffB;
-  static constexpr int kStatic = 16 * kPanelWarps + kPanelWarps * kWarpB;  // mbarriers, then the warps' areas
+// One lane's 4 products of a chunk, and a segment's running sum.  FP32: one
+// sum per entry of a chunk, so chains stay at 16 adds; split: exact products
+// p + t, df sums (TwoSum).
+template <int ST> struct ChunkProd {
+  float p[4];
+  __device__ __forceinline__ void load(const unsigned char* rec, int lane, const float* xs) {
+    using R = StreamRec<ST>;
+    const uint2 q = reinterpret_cast<const uint2*>(rec + R::kValB)[lane];
+    float v[4];
+    if constexpr (ST == FVG_F32) {
+      const float4 h = reinterpret_cast<const float4*>(rec)[lane];
+      v[0] = h.x; v[1] = h.y; v[2] = h.z; v[3] = h.w;
+    } else {
+      const uint2 h = reinterpret_cast<const uint2*>(rec)[lane];
+      v[0] = __uint_as_float(h.x << 16); v[1] = __uint_as_float(h.x & 0xffff0000u);
+      v[2] = __uint_as_float(h.y << 16); v[3] = __uint_as_float(h.y & 0xffff0000u);
+    }
+    p[0] = v[0] * xs[q.x & 0xffffu];
+    p[1] = v[1] * xs[q.x >> 16];
+    p[2] = v[2] * xs[q.y & 0xffffu];
+    p[3] = v[3] * xs[q.y >> 16];
+  }
+};
+template <> struct ChunkProd<FVG_SPLIT> {
+  float p[4], t[4];
+  __device__ __forceinline__ void load(const unsigned char* rec, int lane, const float2* xs) {
+    using R = StreamRec<FVG_SPLIT>;
+    const uint2 q = reinterpret_cast<const uint2*>(rec + R::kValB + R::kLoB)[lane];
+    const float4 h = reinterpret_cast<const float4*>(rec)[lane];
+    const uint2 l = reinterpret_cast<const uint2*>(rec + R::kValB)[lane];
+    const float2 x0 = xs[q.x & 0xffffu], x1 = xs[q.x >> 16], x2 = xs[q.y & 0xffffu], x3 = xs[q.y >> 16];
+    df_prod(h.x, __uint_as_float(l.x << 16), x0, p[0], t[0]);
+    df_prod(h.y, __uint_as_float(l.x & 0xffff0000u), x1, p[1], t[1]);
+    df_prod(h.z, __uint_as_float(l.y << 16), x2, p[2], t[2]);
+    df_prod(h.w, __uint_as_float(l.y & 0xffff0000u), x3, p[3], t[3]);
+  }
+};
+template <int ST> struct SegSum {
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+  __device__ __forceinline__ void add(const ChunkProd<ST>& c) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) s[k] += c.p[k];
+  }
+  __device__ __forceinline__ float get() const { return (s[0] + s[1]) + (s[2] + s[3]); }
+};
+template <> struct SegSum<FVG_SPLIT> {
+  DfAcc a;
+  __device__ __forceinline__ void add(const ChunkProd<FVG_SPLIT>& c) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) a.add(c.p[k], c.t[k]);
+  }
+  __device__ __forceinline__ float2 get() const { return df_pack(a.get()); }
 };
 
-// One CTA of kPanelWarps warps per SM takes units of `group` consecutive
-// panels: b, b+G, ...  Per unit: the vector's slice into shared memory (row
-// panels: r's rows of the panel; forward head: w at the head columns, staged
-// once); then the warps walk the unit's work items (tiles of short rows,
-// pieces of long ones; warp w takes items w, w+W, ...).  Per item a bulk copy
-// stages the entries in the warp's buffer (the copies of the other 31 warps
-// cover its latency); the products with the vector gathered from shared
-// memory overwrite the staged entries, and each row is added by 1..32 lanes
-// in a fixed order.  After a barrier the pieces of long rows are added in
-// piece order.  (Measured on GB300 against a double-buffered variant with 16
-// warps and a separate product buffer: this one is 10% faster on the 10M x 1M
-// benchmark matrix.)
-template <class VT>
-__global__ void __launch_bounds__(kPanelWarps * 32, 1) k_panel(const PanK p) {
-  using SM = PanelSmem<VT>;
-  constexpr int NW = kPanelWarps;
-  constexpr int NR2 = (kWarpTile + 16 + 63) / 64;  // pair rounds of a staged copy (<= 520 entries)
+// One CTA of kStreamWarps warps per SM takes units (a row panel; for the
+// forward head a CTA's whole share of the rows): b, b+G, ...  Per unit the
+// vector's slice goes to shared memory (row panels: r's rows of the panel;
+// head: w at the head columns, once), then every warp streams its run of
+// slices through a ring of kStreamStages bulk copies (cp.async.bulk, an
+// mbarrier each, bounded waits) that passes by L1: a panel's slice leaves
+// little L1, and loads under way would need lines there.  After a barrier the
+// segments of long rows are added in order.  Every sum has a fixed order.
+template <int ST>
+__global__ void __launch_bounds__(kStreamWarps * 32, 1) k_panel_stream(const StreamK p) {
+  using R = StreamRec<ST>;
+  using X = typename R::X;
+  constexpr int NW = kStreamWarps, NS = kStreamStages, SC = kStreamChunks;
   extern __shared__ __align__(128) unsigned char smem[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem) + 2 * w;
-  unsigned char* area = smem + 16 * NW + w * SM::kWarpB;
-  unsigned short* soff = reinterpret_cast<unsigned short*>(area + SM::kStageB);
-  float* prod = reinterpret_cast<float*>(area);
-  float2* prod2 = reinterpret_cast<float2*>(area);
-  float* xs = reinterpret_cast<float*>(smem + SM::kStatic);
-  const VT* __restrict__ val = (const VT*)p.val;
-  if (lane == 0) mbar_init(bar, 1);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem) + w * NS;
+  unsigned char* ring = smem + R::kBarB + w * R::kRingB;
+  X* xs = reinterpret_cast<X*>(smem + R::kStatic);
+  const X* __restrict__ x = (const X*)p.x;
+  X* ypan = (X*)p.ypan;
+  X* partials = (X*)p.partials;
+  if (lane == 0)
+    for (int i = 0; i < NS; i++) mbar_init(bars + i, 1);
   fence_mbar_init();
+  if (threadIdx.x == 0) xs[p.rows] = X{};  // the padding's vector entry
   __syncthreads();
   const uint64_t pol = policy_evict_first();
-  unsigned parity = 0;
-  bool pend = false, dead = false;
-  const bool shared = p.xmap != nullptr;
-  // a CTA takes `group` consecutive panels at a time (their items and long
-  // rows are contiguous): one per step for row panels, a whole share of the
-  // rows at once for the forward head (one barrier per CTA)
-  const int nunits = (int)((p.npanels + p.group - 1) / p.group);
-  for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
-    const int pn = u * (int)p.group, pe = (int)min((i64)pn + p.group, p.npanels);
-    const i64 base = shared ? 0 : (i64)pn * p.rows;
-    const int nr = shared ? (int)p.rows : (int)min(p.rows, p.m - base);
-    __syncthreads();
-    if (shared) {
-      if (u == blockIdx.x)
-        for (int i = threadIdx.x; i < nr; i += NW * 32) xs[i] = __ldg(p.r + p.xmap[i]);
-    } else {
-      const int n4 = p.aligned ? nr >> 2 : 0;
-      const float4* src = reinterpret_cast<const float4*>(p.r + base);
-      float4* dst = reinterpret_cast<float4*>(xs);
-      int i = threadIdx.x;
-      for (; i + 3 * NW * 32 < n4; i += 4 * NW * 32) {
-        const float4 a0 = src[i], a1 = src[i + NW * 32], a2 = src[i + 2 * NW * 32], a3 = src[i + 3 * NW * 32];
-        dst[i] = a0;
-        dst[i + NW * 32] = a1;
-        dst[i + 2 * NW * 32] = a2;
-        dst[i + 3 * NW * 32] = a3;
+  int is = 0, us = 0;  // ring slots of the next copy and of the next wait
+  unsigned phase = 0;  // parity of the next wait's slot
+  int flying = 0;      // copies under way
+  bool dead = false;
+  // kAhead slices' row numbers, copied asynchronously: each lane reads only
+  // its own words
+  i32* oq = reinterpret_cast<i32*>(smem + R::kBarB + NW * R::kRingB) + w * (kAhead * 32) + lane;
+  for (int u = blockIdx.x; u < (int)p.nunits; u += gridDim.x) {
+    const int s0 = p.wstart[(i64)u * (NW + 1) + w], s1 = p.wstart[(i64)u * (NW + 1) + w + 1];
+    int g = p.coff[s0];  // next chunk to add
+    const int ge = p.coff[s1];
+    int gi = g;          // next chunk to copy
+    // a copy always takes SC records (the records are padded past the last)
+    auto issue = [&]() {
+      if (gi >= ge || dead) return;
+      if (lane == 0) {
+        mbar_arrive_expect_tx(bars + is, SC * R::kB);
+        bulk_g2s(ring + is * (SC * R::kB), p.rec + (i64)gi * R::kB, SC * R::kB, bars + is, pol);
       }
-      for (; i < n4; i += NW * 32) dst[i] = src[i];
-      for (i = (n4 << 2) + threadIdx.x; i < nr; i += NW * 32) xs[i] = p.r[base + i];
+      gi += SC;
+      flying++;
+      is = is + 1 == NS ? 0 : is + 1;
+    };
+#pragma unroll
+    for (int i = 0; i < NS; i++) issue();
+    const i32* vo = p.vout + lane;
+    auto fetch_out = [&](int s) {
+      if (s < s1) cp_async4(oq + (s & (kAhead - 1)) * 32, vo + (i64)s * 32);
+      cp_async_commit();
+    };
+#pragma unroll
+    for (int i = 0; i < kAhead; i++) fetch_out(s0 + i);
+    __syncthreads();  // the slice of the unit before is no longer read
+    if (p.xmap) {
+      if (u == (int)blockIdx.x)
+#pragma unroll 4
+        for (int i = threadIdx.x; i < (int)p.rows; i += NW * 32) xs[i] = __ldg(x + p.xmap[i]);
+    } else {
+      const i64 base = (i64)u * p.rows;
+      const int nr = (int)min(p.rows, p.m - base);
+      constexpr int V = 16 / (int)sizeof(X);
+      const int nv = p.aligned ? nr / V : 0;  // rows is a multiple of 4
+      const float4* src = reinterpret_cast<const float4*>(x + base);
+#pragma unroll 4
+      for (int i = threadIdx.x; i < nv; i += NW * 32) reinterpret_cast<float4*>(xs)[i] = __ldg(src + i);
+      for (int i = nv * V + threadIdx.x; i < nr; i += NW * 32) xs[i] = __ldg(x + base + i);
     }
     __syncthreads();
-    const int t1 = p.pitem0[pe];
-    int t = p.pitem0[pn] + w;
-    Item nx = (t < t1) ? p.items[t] : Item{0, 0, 0, 0};
-    for (; t < t1 && !dead; t += NW) {
-      const Item it = nx;
-      if (t + NW < t1) nx = p.items[t + NW];
-      const int q0 = it.e0 & ~7, q1 = (it.e1 + 7) & ~7;
-      const unsigned n = (unsigned)(q1 - q0);
-      if (lane == 0) {
-        fence_proxy_async();
-        mbar_arrive_expect_tx(bar, n * 2u + n * (unsigned)sizeof(VT));
-        if (n > 0) {
-          bulk_g2s(area, p.prow + q0, n * 2u, bar, pol);
-          bulk_g2s(area + SM::kIdxB, val + q0, n * (unsigned)sizeof(VT), bar, pol);
-        }
+    // lane L holds the end of slice win + L, then of win + 32 + L
+    int s = s0, win = s0;
+    i32 ends = s0 + lane < s1 ? p.coff[s0 + lane + 1] : 0;
+    i32 ends2 = s0 + 32 + lane < s1 ? p.coff[s0 + 32 + lane + 1] : 0;
+    int ce = __shfl_sync(0xffffffffu, ends, 0);  // end of slice s
+    SegSum<ST> sum;
+    // writes slice s's sums and moves to the next one
+    auto next_slice = [&]() {
+      cp_async_wait<kAhead - 1>();
+      const i32 o = oq[(s & (kAhead - 1)) * 32];
+      fetch_out(s + kAhead);
+      const auto r = sum.get();
+      sum = SegSum<ST>();
+      if (o >= 0) ypan[o] = r;
+      else if (o != kNoRow) partials[~o] = r;
+      s++;
+      if (s - win == 32) {
+        win = s;
+        ends = ends2;
+        ends2 = s + 32 + lane < s1 ? p.coff[s + 32 + lane + 1] : 0;
       }
-      pend = true;
-      if (it.r1 >= 0)
-        for (int k = lane; k <= it.r1 - it.r0; k += 32) soff[k] = (unsigned short)(__ldg(p.poff + it.r0 + k) - q0);
-      if (!mbar_wait_bounded(bar, parity, p.err, p.wait_limit)) {
+      ce = __shfl_sync(0xffffffffu, ends, s - win);
+    };
+    while (g < ge) {
+      if (!mbar_wait_bounded(bars + us, phase, p.err, p.wait_limit)) {
         dead = true;
         break;
       }
-      parity ^= 1u;
-      pend = false;
-      __syncwarp();
-      {
-        // every staged pair into registers first: the products overwrite them
-        const unsigned* sidx2 = reinterpret_cast<const unsigned*>(area);
-        const VT* sval = reinterpret_cast<const VT*>(area + SM::kIdxB);
-        const int n2 = (int)(n >> 1);
-        unsigned c[NR2];
-        float v0[NR2], v1[NR2];
+      // all the copy's products first (their shared loads overlap), so that
+      // the ring slot is free for the next copy before the sums
+      const unsigned char* cur = ring + us * (SC * R::kB);
+      ChunkProd<ST> c[SC];
 #pragma unroll
-        for (int q = 0; q < NR2; q++) {
-          const int k2 = q * 32 + lane;
-          if (k2 < n2) {
-            c[q] = sidx2[k2];
-            v0[q] = (float)sval[2 * k2];
-            v1[q] = (float)sval[2 * k2 + 1];
-          }
-        }
-        __syncwarp();
-#pragma unroll
-        for (int q = 0; q < NR2; q++) {
-          const int k2 = q * 32 + lane;
-          if (k2 < n2) prod2[k2] = make_float2(v0[q] * xs[c[q] & 0xffffu], v1[q] * xs[c[q] >> 16]);
-        }
+      for (int k = 0; k < SC; k++) c[k].load(cur + k * R::kB, lane, xs);
+      flying--;
+      us++;
+      if (us == NS) {
+        us = 0;
+        phase ^= 1u;
       }
-      __syncwarp();
-      if (it.r1 >= 0) {
-        const int R = it.r1 - it.r0;
-        const int Gl = lanes_per_row(R);
-        const int per_round = 32 / Gl;
-        for (int rb = 0; rb < R; rb += per_round) {
-          const int j = rb + lane / Gl, sub = lane % Gl;
-          float acc = 0.f;
-          if (j < R) {
-            const int s = soff[j], e = soff[j + 1];
-            float a1 = 0.f, a2 = 0.f, a3 = 0.f;
-            int k = s + sub;
-            for (; k + 3 * Gl < e; k += 4 * Gl) {
-              acc += prod[k];
-              a1 += prod[k + Gl];
-              a2 += prod[k + 2 * Gl];
-              a3 += prod[k + 3 * Gl];
-            }
-            for (; k < e; k += Gl) acc += prod[k];
-            acc = (acc + a1) + (a2 + a3);
-          }
-          for (int o = Gl >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-          if (j < R && sub == 0) p.ypan[it.r0 + j] = acc;
-        }
-      } else {
-        float acc = 0.f;
-        const int e = it.e1 - q0;
-        for (int k = it.e0 - q0 + lane; k < e; k += 32) acc += prod[k];
+      __syncwarp();  // every lane has read the copy
+      issue();
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) p.partials[-1 - it.r1] = acc;
+      for (int k = 0; k < SC; k++) {
+        if (g >= ge) break;
+        while (g == ce) next_slice();
+        sum.add(c[k]);
+        g++;
       }
-      __syncwarp();
     }
+    if (!dead)
+      while (s < s1) next_slice();
+    cp_async_wait<0>();
     __syncthreads();
-    const int l1 = p.plong0[pe];
-    for (int L = p.plong0[pn] + w; L < l1; L += NW) {
+    const int l1 = p.ulong0[u + 1];
+    for (int L = p.ulong0[u] + w; L < l1; L += NW) {
       const int c0 = p.long_piece0[L], c1 = p.long_piece0[L + 1];
-      float acc = 0.f;
-      for (int j = c0 + lane; j < c1; j += 32) acc += __ldcg(p.partials + j);
+      if constexpr (ST == FVG_SPLIT) {
+        df a = {0.f, 0.f};
+        for (int j = c0 + lane; j < c1; j += 32) a = df_add(a, df_unpack(__ldcg(partials + j)));
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (lane == 0) p.ypan[p.long_rows[L]] = acc;
+        for (int o = 16; o > 0; o >>= 1) a = df_add(a, shfl_xor_df(a, o));
+        if (lane == 0) ypan[p.long_rows[L]] = df_pack(a);
+      } else {
+        float a = 0.f;
+        for (int j = c0 + lane; j < c1; j += 32) a += __ldcg(partials + j);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (lane == 0) ypan[p.long_rows[L]] = a;
+      }
     }
   }
-  // a warp that gave up still drains its copy in flight (default budget)
-  // before the CTA's shared memory is released
-  if (pend) mbar_wait_bounded(bar, parity, nullptr, kCopyPolls);
+  // a warp that gave up still drains its copies in flight (default budget)
+  for (; flying > 0; flying--) {
+    mbar_wait_bounded(bars + us, phase, nullptr, kCopyPolls);
+    us++;
+    if (us == NS) {
+      us = 0;
+      phase ^= 1u;
+    }
+  }
+}
+
+// ------------------------------------------------- streamed layout's build
+// Segments per panel row, and the rows cut into several (long rows).
+__global__ void k_seg_counts(const i32* __restrict__ poff, i64 Q, i64* __restrict__ nv, i64* __restrict__ lng,
+                             i64* __restrict__ lpc) {
+  PGRID_STRIDE(q, Q) {
+    const i32 n = max(1, (((poff[q + 1] - poff[q]) + 3) / 4 + kSegChunks - 1) / kSegChunks);
+    nv[q] = n;
+    lng[q] = n > 1;
+    lpc[q] = n > 1 ? n : 0;
+  }
+}
+
+// chunks [c0, c1) of segment j of n of a row of `len` entries
+__device__ __forceinline__ void seg_chunks(i32 len, i32 j, i32 n, i32& c0, i32& c1) {
+  const i64 c = (len + 3) / 4;
+  c0 = (i32)(c * j / n);
+  c1 = (i32)(c * (j + 1) / n);
+}
+
+// sort keys: the panel, then the segments by decreasing chunks
+__global__ void k_seg_keys(const i32* __restrict__ poff, const i64* __restrict__ voff, i64 Q, i64 nhot,
+                           uint32_t* __restrict__ keys, uint32_t* __restrict__ ids, i32* __restrict__ vq) {
+  PGRID_STRIDE(q, Q) {
+    const i64 v0 = voff[q];
+    const i32 n = (i32)(voff[q + 1] - v0), len = poff[q + 1] - poff[q];
+    const uint32_t p = (uint32_t)(q / nhot) << 5;
+    for (i32 j = 0; j < n; j++) {
+      i32 c0, c1;
+      seg_chunks(len, j, n, c0, c1);
+      keys[v0 + j] = p | (uint32_t)(kSegChunks - (c1 - c0));
+      ids[v0 + j] = (uint32_t)(v0 + j);
+      vq[v0 + j] = (i32)q;
+    }
+  }
+}
+
+// out[i] = src[min(i * step, limit)]
+__global__ void k_take_every(const i64* __restrict__ src, i64 step, i64 limit, i64 n, i64* __restrict__ out) {
+  PGRID_STRIDE(i, n) out[i] = src[min(i * step, limit)];
+}
+
+// per (slice, lane): where the segment's sum goes, its first entry and its
+// entries; per slice its chunks (lane 0 holds the longest segment)
+__global__ void k_slices(const i32* __restrict__ poff, const i64* __restrict__ voff, const i64* __restrict__ lpc,
+                         const uint32_t* __restrict__ ids, const i32* __restrict__ vq, const i64* __restrict__ sbase,
+                         const i64* __restrict__ pstart, i64 np, i64 ns, i32* __restrict__ vout,
+                         i32* __restrict__ vsrc, unsigned char* __restrict__ vlen, i64* __restrict__ width) {
+  PGRID_STRIDE(t, ns * 32) {
+    const i64 s = t >> 5;
+    i64 a = 0, b = np;  // the panel holding slice s: sbase[a] <= s < sbase[a + 1]
+    while (b - a > 1) {
+      const i64 mid = (a + b) >> 1;
+      if (sbase[mid] <= s) a = mid;
+      else b = mid;
+    }
+    const i64 i = pstart[a] + (s - sbase[a]) * 32 + (t & 31);
+    i32 out = kNoRow, src = 0, cnt = 0, c0 = 0, c1 = 0;
+    if (i < pstart[a + 1]) {
+      const i64 v = ids[i];
+      const i32 q = vq[v];
+      const i32 n = (i32)(voff[q + 1] - voff[q]), j = (i32)(v - voff[q]), len = poff[q + 1] - poff[q];
+      seg_chunks(len, j, n, c0, c1);
+      out = n > 1 ? ~(i32)(lpc[q] + j) : q;
+      src = poff[q] + 4 * c0;
+      cnt = min(4 * c1, len) - 4 * c0;
+    }
+    vout[t] = out;
+    vsrc[t] = src;
+    vlen[t] = (unsigned char)cnt;
+    if ((t & 31) == 0) width[s] = c1 - c0;
+  }
+}
+
+__global__ void k_long_list(const i64* __restrict__ lng, const i64* __restrict__ lpos, const i64* __restrict__ lpc,
+                            i64 Q, i32* __restrict__ rows, i32* __restrict__ piece0) {
+  PGRID_STRIDE(q, Q)
+    if (lng[q]) {
+      rows[lpos[q]] = (i32)q;
+      piece0[lpos[q]] = (i32)lpc[q];
+    }
+}
+
+// first slice of each warp's share of a unit: equal chunks + slices
+__global__ void k_warp_starts(const i32* __restrict__ coff, const i64* __restrict__ sbase, i64 group, i64 np,
+                              i64 nunits, i32* __restrict__ wstart) {
+  PGRID_STRIDE(t, nunits * (kStreamWarps + 1)) {
+    const i64 u = t / (kStreamWarps + 1), w = t - u * (kStreamWarps + 1);
+    const i64 a = sbase[u * group], b = sbase[min((u + 1) * group, np)];
+    const i64 c0 = coff[a] + a, c1 = coff[b] + b;
+    const i64 target = c0 + (c1 - c0) * w / kStreamWarps;
+    i64 lo = a, hi = b;  // first slice whose start costs at least the target
+    while (lo < hi) {
+      const i64 mid = (lo + hi) >> 1;
+      if (coff[mid] + mid < target) lo = mid + 1;
+      else hi = mid;
+    }
+    wstart[t] = (i32)lo;
+  }
+}
+
+// a warp per slice: its records from the packed entries
+template <int ST>
+__global__ void k_fill_records(const i32* __restrict__ coff, const i32* __restrict__ vsrc,
+                               const unsigned char* __restrict__ vlen, i64 ns, const uint16_t* __restrict__ prow,
+                               const float* __restrict__ v32, const unsigned short* __restrict__ v16,
+                               const unsigned short* __restrict__ lo, unsigned pad, unsigned char* __restrict__ rec) {
+  using R = StreamRec<ST>;
+  const int lane = threadIdx.x & 31;
+  PWARP_STRIDE(s, ns) {
+    const i32 src = vsrc[s * 32 + lane];
+    const int n = vlen[s * 32 + lane], c0 = coff[s], w = coff[s + 1] - c0;
+    for (int c = 0; c < w; c++) {
+      unsigned char* r = rec + (i64)(c0 + c) * R::kB;
+      float v[4];
+      unsigned h[4], l[4], q[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const bool in = 4 * c + k < n;
+        const i64 e = (i64)src + 4 * c + k;
+        q[k] = in ? prow[e] : pad;
+        if (ST == FVG_BF16) h[k] = in ? v16[e] : 0u;
+        else v[k] = in ? v32[e] : 0.f;
+        if (ST == FVG_SPLIT) l[k] = in ? lo[e] : 0u;
+      }
+      if (ST == FVG_BF16) reinterpret_cast<uint2*>(r)[lane] = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
+      else reinterpret_cast<float4*>(r)[lane] = make_float4(v[0], v[1], v[2], v[3]);
+      if (ST == FVG_SPLIT)
+        reinterpret_cast<uint2*>(r + R::kValB)[lane] = make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
+      reinterpret_cast<uint2*>(r + R::kValB + R::kLoB)[lane] = make_uint2(q[0] | (q[1] << 16), q[2] | (q[3] << 16));
+    }
+  }
 }
 
 // g[hot[h]] = sum over panels of ypan[panel*nhot + h] in a fixed order:
@@ -577,308 +805,6 @@ __global__ void __launch_bounds__(1024) k_panel_colsum(const float* __restrict__
   }
 }
 
-// ------------------------------------------------------ split storage
-// The row-panel / forward-head kernel for split values (FP32 value + BF16
-// residual per entry, df64 products: df64.cuh).  Same layout as k_panel; the
-// staged entry is 8 bytes (uint16 slot, FP32 value, BF16 residual) and the
-// vector slice keeps both FP32 words of each df pair (8 bytes a row: rounding
-// the slice's low word would add noise that changes from one evaluation to
-// the next and, unlike the fixed rounding of the values, does not cancel in
-// the L-BFGS gradient differences).  To fit a panel beside the staging
-// buffers, one CTA of kSplitWarps warps per SM walks its own work items of at
-// most kSplitTile entries, so that one item is one pass of 32 lanes x
-// kSplitChunk entries: no products are staged and no second pass re-reads
-// them.
-#ifndef FVG_SPLIT_WARPS
-#define FVG_SPLIT_WARPS 28
-#endif
-constexpr int kSplitWarps = FVG_SPLIT_WARPS;  // one CTA per SM (its shared slice fills the SM)
-constexpr int kSplitTile = 480;  // an item's staged copy (8-aligned ends) fits 32 lanes x 16 entries
-constexpr int kSplitChunk = 16;  // entries per lane
-struct SplitSmem {
-  static constexpr int kCap = 32 * kSplitChunk;        // entries of one copy
-  static constexpr int kHiB = kCap * 2;                // offset of the FP32 values
-  static constexpr int kLoB = kHiB + kCap * 4;         // offset of the BF16 residuals
-  static constexpr int kStageB = kLoB + kCap * 2;      // = kCap * 8
-  static constexpr int kSoffB = ((kTileRows + 1) * 2 + 15) / 16 * 16;
-  static constexpr int kWarpB = kStageB + kSoffB;
-  static constexpr int kStatic = 16 * kSplitWarps + kSplitWarps * kWarpB;
-};
-
-struct PanSK {
-  const i32* poff;
-  const uint16_t* prow;
-  const float* vh;
-  const unsigned short* vl;
-  const float2* x;  // df pairs: r (row panels) or w (forward head)
-  i64 m, rows, npanels;
-  const Item* items;
-  const i32* pitem0;
-  const i32* long_rows;
-  const i32* plong0;
-  const i32* long_piece0;
-  float2* partials;
-  float2* ypan;
-  unsigned* err;
-  unsigned wait_limit;
-  const i32* xmap;  // forward head: the slice is x[xmap[0..rows)], staged once
-  i64 group;
-};
-
-__device__ __forceinline__ df shfl_xor_df(df a, int o) {
-  return {__shfl_xor_sync(0xffffffffu, a.h, o), __shfl_xor_sync(0xffffffffu, a.l, o)};
-}
-__device__ __forceinline__ df shfl_up_df(df a, int o) {
-  return {__shfl_up_sync(0xffffffffu, a.h, o), __shfl_up_sync(0xffffffffu, a.l, o)};
-}
-
-// Segmented inclusive scan over the warp's lanes, in lane order:
-// S_L = v_L + (reset_L ? 0 : S_{L-1}) (Hillis-Steele; a lane stops adding
-// once a reset lies between it and the lane it reads).
-__device__ __forceinline__ df seg_scan_df(df v, bool reset, int lane) {
-  bool f = reset;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const df u = shfl_up_df(v, o);
-    const bool fu = __shfl_up_sync(0xffffffffu, (int)f, o) != 0;
-    if (lane >= o) {
-      if (!f) v = df_add(u, v);
-      f = f || fu;
-    }
-  }
-  return v;
-}
-
-// One CTA of kSplitWarps warps per SM takes units of `group` consecutive
-// panels (as k_panel).  Per work item (at most kSplitTile entries) a bulk
-// copy stages the entries (uint16 slots, FP32 values, BF16 residuals); lane L
-// then takes the kSplitChunk staged entries from kSplitChunk*L on (16-byte
-// shared loads), makes each
-// product exact (p + t), and adds its row segments in registers with TwoSum:
-// a row that ends inside the chunk is written at once when it also started
-// there; the row that was open at the chunk's start and the one open at its
-// end join the neighbouring lanes' segments through a segmented scan in lane
-// order.  Pieces of long rows: a warp reduction, added after the CTA barrier
-// in piece order.  Every sum has a fixed order.
-// MID (the row panels, whose rows are often shorter than a lane's chunk): the
-// rows that start and end inside one lane's chunk are summed in the chunk's
-// single pass, parked in the warp's staging area (free once the entries are
-// in registers) and written after it; without MID (the forward head, rows
-// longer than a chunk) each such row is re-summed over the chunk.
-template <bool MID>
-__global__ void __launch_bounds__(kSplitWarps * 32, 1) k_panel_split(const PanSK p) {
-  using SM = SplitSmem;
-  constexpr int NW = kSplitWarps;
-  constexpr int CH = kSplitChunk;
-  extern __shared__ __align__(128) unsigned char smem[];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem) + 2 * w;
-  unsigned char* area = smem + 16 * NW + w * SM::kWarpB;
-  unsigned short* soff = reinterpret_cast<unsigned short*>(area + SM::kStageB);
-  float2* xs = reinterpret_cast<float2*>(smem + SM::kStatic);  // df pairs: one 8-byte load a gather
-  if (lane == 0) mbar_init(bar, 1);
-  fence_mbar_init();
-  __syncthreads();
-  const uint64_t pol = policy_evict_first();
-  unsigned parity = 0;
-  bool pend = false, dead = false;
-  const bool shared = p.xmap != nullptr;
-  const int nunits = (int)((p.npanels + p.group - 1) / p.group);
-  for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
-    const int pn = u * (int)p.group, pe = (int)min((i64)pn + p.group, p.npanels);
-    const i64 base = shared ? 0 : (i64)pn * p.rows;
-    const int nr = shared ? (int)p.rows : (int)min(p.rows, p.m - base);
-    __syncthreads();
-    if (!shared || u == blockIdx.x)
-      for (int i = threadIdx.x; i < nr; i += NW * 32) {
-        const float2 v = __ldg(p.x + (shared ? (i64)p.xmap[i] : base + i));
-        xs[i] = v;
-      }
-    __syncthreads();
-    const int t1 = p.pitem0[pe];
-    int t = p.pitem0[pn] + w;
-    Item nx = (t < t1) ? p.items[t] : Item{0, 0, 0, 0};
-    for (; t < t1 && !dead; t += NW) {
-      const Item it = nx;
-      if (t + NW < t1) nx = p.items[t + NW];
-      const int q0 = it.e0 & ~7, q1 = (it.e1 + 7) & ~7;
-      const unsigned n = (unsigned)(q1 - q0);
-      if (lane == 0) {
-        fence_proxy_async();
-        mbar_arrive_expect_tx(bar, n * 8u);
-        if (n > 0) {
-          bulk_g2s(area, p.prow + q0, n * 2u, bar, pol);
-          bulk_g2s(area + SM::kHiB, p.vh + q0, n * 4u, bar, pol);
-          bulk_g2s(area + SM::kLoB, p.vl + q0, n * 2u, bar, pol);
-        }
-      }
-      pend = true;
-      const bool tile = it.r1 >= 0;
-      const int R = tile ? it.r1 - it.r0 : 0;
-      if (tile)
-        for (int k = lane; k <= R; k += 32) soff[k] = (unsigned short)(__ldg(p.poff + it.r0 + k) - q0);
-      if (!mbar_wait_bounded(bar, parity, p.err, p.wait_limit)) {
-        dead = true;
-        break;
-      }
-      parity ^= 1u;
-      pend = false;
-      __syncwarp();
-      // The copy's padding entries (before e0, and from e1 to the end of the
-      // lane chunk holding it: at most 7 and 15) become slot 0, value 0, so
-      // that their products are exact zeros and no entry needs a range test.
-      {
-        const int lead = it.e0 - q0, tz = it.e1 - q0;
-        const int tend = min((tz + CH - 1) / CH * CH, SM::kCap);
-        unsigned short* ss = reinterpret_cast<unsigned short*>(area);
-        float* sh = reinterpret_cast<float*>(area + SM::kHiB);
-        unsigned short* sl = reinterpret_cast<unsigned short*>(area + SM::kLoB);
-        if (lane < lead) {
-          ss[lane] = 0;
-          sh[lane] = 0.f;
-          sl[lane] = 0;
-        }
-        if (lane < tend - tz) {
-          ss[tz + lane] = 0;
-          sh[tz + lane] = 0.f;
-          sl[tz + lane] = 0;
-        }
-        __syncwarp();
-      }
-      // this lane's CH staged entries (16-byte shared loads)
-      unsigned sw[CH / 2], lw[CH / 2];
-      float hv[CH];
-#pragma unroll
-      for (int q = 0; q < CH / 8; q++) {
-        const uint4 s4 = reinterpret_cast<const uint4*>(area)[lane * (CH / 8) + q];
-        const uint4 l4 = reinterpret_cast<const uint4*>(area + SM::kLoB)[lane * (CH / 8) + q];
-        sw[4 * q] = s4.x; sw[4 * q + 1] = s4.y; sw[4 * q + 2] = s4.z; sw[4 * q + 3] = s4.w;
-        lw[4 * q] = l4.x; lw[4 * q + 1] = l4.y; lw[4 * q + 2] = l4.z; lw[4 * q + 3] = l4.w;
-      }
-#pragma unroll
-      for (int q = 0; q < CH / 4; q++) {
-        const float4 h = reinterpret_cast<const float4*>(area + SM::kHiB)[lane * (CH / 4) + q];
-        hv[4 * q] = h.x; hv[4 * q + 1] = h.y; hv[4 * q + 2] = h.z; hv[4 * q + 3] = h.w;
-      }
-      const int lo_e = max(it.e0 - q0, lane * CH), hi_e = min(it.e1 - q0, lane * CH + CH);
-      const bool any = lo_e < hi_e;
-      // a lane past the item's end reads stale (or never written) slots: slot 0
-#pragma unroll
-      for (int q = 0; q < CH / 2; q++) sw[q] = any ? sw[q] : 0u;
-      if (!tile) {
-        DfAcc acc;
-#pragma unroll
-        for (int k = 0; k < CH; k++) {
-          const unsigned c = (sw[k >> 1] >> ((k & 1) * 16)) & 0xffffu;
-          const float vl = __uint_as_float((k & 1) ? (lw[k >> 1] & 0xffff0000u) : (lw[k >> 1] << 16));
-          float pp, tt;
-          df_prod(hv[k], vl, xs[c], pp, tt);
-          acc.add(pp, tt);
-        }
-        if (!any) acc = DfAcc{};
-        df a = acc.get();
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a = df_add(a, shfl_xor_df(a, o));
-        if (lane == 0) p.partials[-1 - it.r1] = df_pack(a);
-      } else {
-        __syncwarp();  // soff
-        for (int j = lane; j < R; j += 32)
-          if (soff[j] == soff[j + 1]) p.ypan[it.r0 + j] = make_float2(0.f, 0.f);  // empty rows
-        // the lane's CH products (padding entries give exact zeros; a lane
-        // past the item's end has any == false and its sums are dropped)
-        float pp[CH], tt[CH];
-#pragma unroll
-        for (int k = 0; k < CH; k++) {
-          const unsigned c = (sw[k >> 1] >> ((k & 1) * 16)) & 0xffffu;
-          const float vl = __uint_as_float((k & 1) ? (lw[k >> 1] & 0xffff0000u) : (lw[k >> 1] << 16));
-          df_prod(hv[k], vl, xs[c], pp[k], tt[k]);
-        }
-        // rows: j0 holds the first valid entry; B marks the rows starting after it
-        unsigned B = 0;
-        int j = 0, j0 = 0, nb = 0;
-        bool starts = false;
-        if (any) {
-          int a = 0, b = R;  // the last row starting at or before lo_e (the non-empty one holding it)
-          while (b - a > 1) {
-            const int mid = (a + b) >> 1;
-            if ((int)soff[mid] <= lo_e) a = mid;
-            else b = mid;
-          }
-          j = j0 = a;
-          starts = (int)soff[j] == lo_e;
-          nb = soff[j + 1];
-          while (nb < hi_e) {
-            B |= 1u << (nb - lane * CH);
-            do {
-              j++;
-              nb = soff[j + 1];
-            } while (nb == (int)soff[j]);
-          }
-        }
-        df H, T;
-        float2* mid = reinterpret_cast<float2*>(area);  // kCap pairs: the staging area's 8 bytes an entry
-        if constexpr (MID) {
-          chunk_segments_mid<CH>(pp, tt, B, H, T, mid, lane * CH);
-        } else {
-          chunk_segments<CH>(pp, tt, B, H, T);
-          if (__popc(B) >= 2) {  // rows between two marks: started and ended in this chunk
-            unsigned rest = B & (B - 1);
-            int a = __ffs(B) - 1, jj = j0;
-            do {
-              jj++;
-            } while (soff[jj + 1] == soff[jj]);
-            while (rest) {
-              const int b = __ffs(rest) - 1;
-              rest &= rest - 1;
-              p.ypan[it.r0 + jj] = df_pack(chunk_range<CH>(pp, tt, a, b));
-              a = b;
-              do {
-                jj++;
-              } while (soff[jj + 1] == soff[jj]);
-            }
-          }
-        }
-        // the tail segment starts inside this lane when a row starts here
-        const df S = seg_scan_df(any ? T : df{0.f, 0.f}, any && (B != 0 || starts), lane);
-        df carry = shfl_up_df(S, 1);
-        if (lane == 0) carry = {0.f, 0.f};
-        if (B) p.ypan[it.r0 + j0] = df_pack(starts ? H : df_add(carry, H));
-        if (any && nb == hi_e) p.ypan[it.r0 + j] = df_pack(S);  // the tail row ends with this lane's range
-        if constexpr (MID) {
-          // the middle rows: non-empty rows whose start and end are both marks
-          // of one lane (start after the lane's first entry, end before its
-          // range ends)
-          __syncwarp();
-          const int ie0 = it.e0 - q0, ie1 = it.e1 - q0;
-          for (int jr = lane; jr < R; jr += 32) {
-            const int s0 = soff[jr], s1 = soff[jr + 1];
-            if (s1 == s0) continue;
-            const int L = s0 / CH;
-            if (s0 > max(ie0, L * CH) && s1 < min(ie1, L * CH + CH)) {
-              const float2 v = mid[s0];
-              p.ypan[it.r0 + jr] = df_pack(fast_two_sum(v.x, v.y));
-            }
-          }
-        }
-      }
-      fence_proxy_async();  // the padding stores, before the next copy into the area
-      __syncwarp();
-    }
-    __syncthreads();
-    const int l1 = p.plong0[pe];
-    for (int L = p.plong0[pn] + w; L < l1; L += NW) {
-      const int c0 = p.long_piece0[L], c1 = p.long_piece0[L + 1];
-      df a = {0.f, 0.f};
-      for (int jj = c0 + lane; jj < c1; jj += 32) a = df_add(a, df_unpack(__ldcg(p.partials + jj)));
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) a = df_add(a, shfl_xor_df(a, o));
-      if (lane == 0) p.ypan[p.long_rows[L]] = df_pack(a);
-    }
-  }
-  // a warp that gave up still drains its copy in flight (default budget)
-  if (pend) mbar_wait_bounded(bar, parity, nullptr, kCopyPolls);
-}
-
 // g[hot[h]] = sum over panels of the df partials ypan[panel*nhot + h]:
 // 32 columns per CTA of 1024 threads, warp w adds panels w, w+32, ...; warp
 // 0 adds the 32 warp sums in order; FP64 result.
@@ -904,22 +830,21 @@ __global__ void __launch_bounds__(1024) k_panel_colsum_split(const float2* __res
   }
 }
 
-int panel_split_smem_bytes(i64 rows) { return SplitSmem::kStatic + (int)(rows * 8); }
+template <int ST> int stream_smem_bytes(i64 rows) {
+  using R = StreamRec<ST>;
+  return R::kStatic + (int)((rows + 1) * (i64)sizeof(typename R::X));  // + the padding's entry
+}
 
-template <class VT> int panel_smem_bytes(i64 rows) { return PanelSmem<VT>::kStatic + (int)(rows * 4); }
-
-// Tallest panel (or head) one CTA can stage beside the staging buffers, for
-// the FP32 / BF16 kernel and the split kernel alike.
+// Tallest panel (or head) one CTA can stage beside the copy rings, for every
+// value storage alike (split values need the most: 8 bytes an entry of the
+// slice and the largest records), so that one layout serves all.
 i64 panel_rows_cap(fvg_ctx* c) {
   int per_sm = 0, reserved = 0, optin = 0;
   FVG_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, c->device));
   FVG_CUDA(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, c->device));
   FVG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
   const i64 per_cta = std::min<i64>((i64)per_sm - (i64)reserved, (i64)optin);
-  // the FP32 kernel stages 4 bytes a row, the split kernel 8 (beside
-  // smaller staging buffers): a layout serves both
-  i64 cap = std::min<i64>((per_cta - PanelSmem<float>::kStatic) / 4, (per_cta - SplitSmem::kStatic) / 8);
-  cap = std::min<i64>(cap, 65536);  // panel-local rows are uint16
+  const i64 cap = std::min<i64>((per_cta - StreamRec<FVG_SPLIT>::kStatic) / 8 - 1, 65535);  // slots are uint16
   return cap & ~3ll;
 }
 
@@ -972,15 +897,15 @@ void fill_planes(fvg_ctx* c, const DevCRS& at, DevPanels& pn, const i32* B, cons
 // rows and pieces are contiguous, numbered globally), packed on the device:
 // counts, their exclusive scans (a few thousand numbers, on the host), then
 // the items.
-void device_pack(fvg_ctx* c, const i32* off, i64 nrows, i64 chunk, i64 nchunks, int tile, PackOut& o, i64 sub,
+void device_pack(fvg_ctx* c, const i32* off, i64 nrows, i64 chunk, i64 nchunks, int tile, PackOut& o,
                  int lane_work) {
-  const i64 np = std::max<i64>(nchunks, 1) * sub;
+  const i64 np = std::max<i64>(nchunks, 1);
   DBuf cnt, basev;
   cnt.alloc(sizeof(i32) * 3 * np, c->stream);
-  if ((chunk + sub - 1) / sub > kPanelPackRows) fail(FVG_ERR_INTERNAL, "packing chunk too long");
+  if (chunk > kPackRows) fail(FVG_ERR_INTERNAL, "packing chunk too long");
   constexpr int kPw = kPackThreads / 32;  // a warp per chunk
   const unsigned pg = (unsigned)std::min<i64>((np + kPw - 1) / kPw, 1 << 20);
-  k_panel_pack<<<pg, kPackThreads, 0, c->stream>>>(off, nrows, chunk, sub, np, tile, 0, cnt.as<i32>(), nullptr, nullptr,
+  k_pack<<<pg, kPackThreads, 0, c->stream>>>(off, nrows, chunk, np, tile, 0, cnt.as<i32>(), nullptr, nullptr,
                                           nullptr, nullptr, nullptr, lane_work);
   check_launch("pack");
   count_launch(c);
@@ -1007,7 +932,7 @@ void device_pack(fvg_ctx* c, const i32* off, i64 nrows, i64 chunk, i64 nchunks, 
   o.long_piece0.alloc(sizeof(i32) * (o.nlong + 1), c->stream);
   DBuf lfirst;
   lfirst.alloc(sizeof(i32) * std::max<i64>(o.nlong, 1), c->stream);
-  k_panel_pack<<<pg, kPackThreads, 0, c->stream>>>(off, nrows, chunk, sub, np, tile, 1, nullptr, basev.as<i32>(),
+  k_pack<<<pg, kPackThreads, 0, c->stream>>>(off, nrows, chunk, np, tile, 1, nullptr, basev.as<i32>(),
                                           o.items.as<Item>(), o.long_rows.as<i32>(), o.long_piece0.as<i32>(),
                                           lfirst.as<i32>(), lane_work);
   check_launch("pack");
@@ -1026,57 +951,137 @@ void device_pack(fvg_ctx* c, const i32* off, i64 nrows, i64 chunk, i64 nchunks, 
 
 namespace {
 
-// The split kernel's work items: the same packing with kSplitTile-entry items
-void pack_split_items(fvg_ctx* c, DevPanels& pn) {
-  const i64 nhot = pn.nhot, np = pn.npanels;
-  PackOut o;
-  const i64 sub = std::max<i64>(1, (nhot + kPanelPackRows - 1) / kPanelPackRows);
-  device_pack(c, pn.poff.as<i32>(), np * nhot, nhot, np, kSplitTile, o, sub);
-  auto it = std::make_unique<PanelItems>();
-  it->tile = kSplitTile;
-  it->nitems = o.nitems;
-  it->nlong = o.nlong;
-  it->npieces = o.npieces;
-  it->items = std::move(o.items);
-  it->long_rows = std::move(o.long_rows);
-  it->long_piece0 = std::move(o.long_piece0);
-  const i64 nc = np * sub;
-  std::vector<i32> pi((size_t)np + 1), pl((size_t)np + 1);
-  for (i64 q = 0; q <= np; q++) {
-    pi[(size_t)q] = o.base[(size_t)(q * sub)];
-    pl[(size_t)q] = o.base[(size_t)((nc + 1) + q * sub)];
-  }
-  it->pitem0.alloc(sizeof(i32) * (np + 1), c->stream);
-  it->plong0.alloc(sizeof(i32) * (np + 1), c->stream);
-  FVG_CUDA(cudaMemcpyAsync(it->pitem0.p, pi.data(), sizeof(i32) * (np + 1), cudaMemcpyHostToDevice, c->stream));
-  FVG_CUDA(cudaMemcpyAsync(it->plong0.p, pl.data(), sizeof(i32) * (np + 1), cudaMemcpyHostToDevice, c->stream));
-  FVG_CUDA(cudaStreamSynchronize(c->stream));  // host arrays go out of scope
-  pn.split_items = std::move(it);
+// The streamed layout of the packed panel rows (poff); false when it would
+// not fit its index types.
+bool stream_layout(fvg_ctx* c, DevPanels& pn) {
+  cudaStream_t st = c->stream;
+  const i64 np = pn.npanels, nhot = pn.nhot, Q = np * nhot;
+  const i32* poff = pn.poff.as<i32>();
+  DBuf nv, lng, lpcn, voff, lpos, lpc;
+  for (DBuf* b : {&nv, &lng, &lpcn}) b->alloc(sizeof(i64) * Q, st);
+  for (DBuf* b : {&voff, &lpos, &lpc}) b->alloc(sizeof(i64) * (Q + 1), st);
+  k_seg_counts<<<grid_n(Q), 256, 0, st>>>(poff, Q, nv.as<i64>(), lng.as<i64>(), lpcn.as<i64>());
+  check_launch("seg_counts");
+  scan_i64(c, nv.as<i64>(), voff.as<i64>(), Q);
+  scan_i64(c, lng.as<i64>(), lpos.as<i64>(), Q);
+  scan_i64(c, lpcn.as<i64>(), lpc.as<i64>(), Q);
+  // per panel: its first segment; per unit: its first long row
+  pn.nunits = (np + pn.group - 1) / pn.group;
+  DBuf pstart, ul;
+  pstart.alloc(sizeof(i64) * (np + 1), st);
+  ul.alloc(sizeof(i64) * (pn.nunits + 1), st);
+  k_take_every<<<grid_n(np + 1), 256, 0, st>>>(voff.as<i64>(), nhot, Q, np + 1, pstart.as<i64>());
+  k_take_every<<<grid_n(pn.nunits + 1), 256, 0, st>>>(lpos.as<i64>(), nhot * pn.group, Q, pn.nunits + 1,
+                                                       ul.as<i64>());
+  check_launch("take_every");
+  std::vector<i64> hp((size_t)np + 1), sb((size_t)np + 1, 0);
+  i64 tot[2];
+  FVG_CUDA(cudaMemcpyAsync(hp.data(), pstart.p, sizeof(i64) * (np + 1), cudaMemcpyDeviceToHost, st));
+  FVG_CUDA(cudaMemcpyAsync(&tot[0], lpos.as<i64>() + Q, sizeof(i64), cudaMemcpyDeviceToHost, st));
+  FVG_CUDA(cudaMemcpyAsync(&tot[1], lpc.as<i64>() + Q, sizeof(i64), cudaMemcpyDeviceToHost, st));
+  FVG_CUDA(cudaStreamSynchronize(st));
+  const i64 V = hp[(size_t)np];
+  for (i64 p = 0; p < np; p++) sb[(size_t)p + 1] = sb[(size_t)p] + (hp[(size_t)p + 1] - hp[(size_t)p] + 31) / 32;
+  const i64 ns = sb[(size_t)np];
+  if (V >= (1ll << 31) - 1 || ns * 32 >= (1ll << 31) - 1) return false;
+  pn.nslices = ns;
+  pn.nlong = tot[0];
+  pn.npieces = tot[1];
+  DBuf keys, ids, vq, sbase, width, coff;
+  keys.alloc(sizeof(uint32_t) * std::max<i64>(V, 1), st);
+  ids.alloc(sizeof(uint32_t) * std::max<i64>(V, 1), st);
+  vq.alloc(sizeof(i32) * std::max<i64>(V, 1), st);
+  k_seg_keys<<<grid_n(Q), 256, 0, st>>>(poff, voff.as<i64>(), Q, nhot, keys.as<uint32_t>(), ids.as<uint32_t>(),
+                                        vq.as<i32>());
+  check_launch("seg_keys");
+  int bits = 5;
+  while ((1ll << (bits - 5)) < np) bits++;
+  radix_sort_pairs(c, keys.as<uint32_t>(), ids.as<uint32_t>(), V, bits);
+  sbase.alloc(sizeof(i64) * (np + 1), st);
+  FVG_CUDA(cudaMemcpyAsync(sbase.p, sb.data(), sizeof(i64) * (np + 1), cudaMemcpyHostToDevice, st));
+  pn.vout.alloc(sizeof(i32) * std::max<i64>(ns * 32, 1), st);
+  pn.vsrc.alloc(sizeof(i32) * std::max<i64>(ns * 32, 1), st);
+  pn.vlen.alloc(std::max<i64>(ns * 32, 1), st);
+  width.alloc(sizeof(i64) * std::max<i64>(ns, 1), st);
+  coff.alloc(sizeof(i64) * (ns + 1), st);
+  k_slices<<<grid_n(ns * 32), 256, 0, st>>>(poff, voff.as<i64>(), lpc.as<i64>(), ids.as<uint32_t>(), vq.as<i32>(),
+                                            sbase.as<i64>(), pstart.as<i64>(), np, ns, pn.vout.as<i32>(),
+                                            pn.vsrc.as<i32>(), pn.vlen.as<unsigned char>(), width.as<i64>());
+  check_launch("slices");
+  scan_i64(c, width.as<i64>(), coff.as<i64>(), ns);
+  FVG_CUDA(cudaMemcpyAsync(&pn.nchunks, coff.as<i64>() + ns, sizeof(i64), cudaMemcpyDeviceToHost, st));
+  FVG_CUDA(cudaStreamSynchronize(st));
+  if (pn.nchunks + ns >= (1ll << 31) - 1) return false;
+  pn.coff.alloc(sizeof(i32) * (ns + 1), st);
+  k_i64_to_i32<<<grid_n(ns + 1), 256, 0, st>>>(coff.as<i64>(), pn.coff.as<i32>(), ns + 1);
+  pn.ulong0.alloc(sizeof(i32) * (pn.nunits + 1), st);
+  k_i64_to_i32<<<grid_n(pn.nunits + 1), 256, 0, st>>>(ul.as<i64>(), pn.ulong0.as<i32>(), pn.nunits + 1);
+  pn.long_rows.alloc(sizeof(i32) * std::max<i64>(pn.nlong, 1), st);
+  pn.long_piece0.alloc(sizeof(i32) * (pn.nlong + 1), st);
+  k_long_list<<<grid_n(Q), 256, 0, st>>>(lng.as<i64>(), lpos.as<i64>(), lpc.as<i64>(), Q, pn.long_rows.as<i32>(),
+                                         pn.long_piece0.as<i32>());
+  const i32 npc = (i32)pn.npieces;
+  FVG_CUDA(cudaMemcpyAsync(pn.long_piece0.as<i32>() + pn.nlong, &npc, sizeof(i32), cudaMemcpyHostToDevice, st));
+  pn.wstart.alloc(sizeof(i32) * pn.nunits * (kStreamWarps + 1), st);
+  k_warp_starts<<<grid_n(pn.nunits * (kStreamWarps + 1)), 256, 0, st>>>(pn.coff.as<i32>(), sbase.as<i64>(), pn.group,
+                                                                        np, pn.nunits, pn.wstart.as<i32>());
+  check_launch("stream_layout");
+  count_launch(c, 9);
+  FVG_CUDA(cudaStreamSynchronize(st));  // host values go out of scope
+  return true;
 }
 
-void pack_panels(fvg_ctx* c, DevPanels& pn, i64 nhot, i64 np) {
-  PackOut o;
-  // each panel's rows in pieces of ~kPanelPackRows rows, a packing warp each
-  const i64 sub = std::max<i64>(1, (nhot + kPanelPackRows - 1) / kPanelPackRows);
-  device_pack(c, pn.poff.as<i32>(), np * nhot, nhot, np, kWarpTile, o, sub);
-  pn.nitems = o.nitems;
-  pn.nlong = o.nlong;
-  pn.npieces = o.npieces;
-  pn.items = std::move(o.items);
-  pn.long_rows = std::move(o.long_rows);
-  pn.long_piece0 = std::move(o.long_piece0);
-  // a panel's items and long rows: from its first piece's on
-  const i64 nc = np * sub;
-  std::vector<i32> pi((size_t)np + 1), pl((size_t)np + 1);
-  for (i64 q = 0; q <= np; q++) {
-    pi[(size_t)q] = o.base[(size_t)(q * sub)];
-    pl[(size_t)q] = o.base[(size_t)((nc + 1) + q * sub)];
+// The records of a value storage, from the packed entries' planes.
+template <int ST> void fill_records(fvg_ctx* c, DevPanels& pn) {
+  DBuf rec;
+  rec.alloc((size_t)(pn.nchunks + kStreamChunks) * StreamRec<ST>::kB, c->stream);  // a copy may read past the last
+  FVG_CUDA(cudaMemsetAsync(rec.as<unsigned char>() + (size_t)pn.nchunks * StreamRec<ST>::kB, 0,
+                           (size_t)kStreamChunks * StreamRec<ST>::kB, c->stream));
+  k_fill_records<ST><<<grid_n(32 * std::max<i64>(pn.nslices, 1)), 256, 0, c->stream>>>(
+      pn.coff.as<i32>(), pn.vsrc.as<i32>(), pn.vlen.as<unsigned char>(), pn.nslices, pn.prow.as<uint16_t>(),
+      pn.val[FVG_F32].as<float>(), pn.val[FVG_BF16].as<unsigned short>(), pn.lo.as<unsigned short>(),
+      (unsigned)pn.rows, rec.as<unsigned char>());
+  check_launch("fill_records");
+  count_launch(c);
+  pn.rec[ST] = std::move(rec);
+}
+
+// ypan (and the long rows' partials) of the layout for a vector x.
+template <int ST> void launch_stream(fvg_ctx* c, DevPanels& pn, const void* x, void* ypan, void* partials) {
+  auto kfn = k_panel_stream<ST>;
+  static std::mutex mu;  // contexts of different host threads launch concurrently
+  static std::vector<int> attr_set;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (std::find(attr_set.begin(), attr_set.end(), c->device) == attr_set.end()) {
+      int optin = 0;
+      FVG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+      FVG_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+      attr_set.push_back(c->device);
+    }
   }
-  pn.pitem0.alloc(sizeof(i32) * (np + 1), c->stream);
-  pn.plong0.alloc(sizeof(i32) * (np + 1), c->stream);
-  FVG_CUDA(cudaMemcpyAsync(pn.pitem0.p, pi.data(), sizeof(i32) * (np + 1), cudaMemcpyHostToDevice, c->stream));
-  FVG_CUDA(cudaMemcpyAsync(pn.plong0.p, pl.data(), sizeof(i32) * (np + 1), cudaMemcpyHostToDevice, c->stream));
-  FVG_CUDA(cudaStreamSynchronize(c->stream));  // host arrays go out of scope
+  StreamK k;
+  k.rec = pn.rec[ST].as<unsigned char>();
+  k.coff = pn.coff.as<i32>();
+  k.vout = pn.vout.as<i32>();
+  k.wstart = pn.wstart.as<i32>();
+  k.ulong0 = pn.ulong0.as<i32>();
+  k.long_rows = pn.long_rows.as<i32>();
+  k.long_piece0 = pn.long_piece0.as<i32>();
+  k.x = x;
+  k.xmap = pn.shared ? pn.hot_cols.as<i32>() : nullptr;
+  k.m = pn.m;
+  k.rows = pn.rows;
+  k.nunits = pn.nunits;
+  k.ypan = ypan;
+  k.partials = partials;
+  k.err = c->dev_err;
+  k.wait_limit = copy_polls(c);
+  k.aligned = ((reinterpret_cast<uintptr_t>(x) & 15) == 0) ? 1 : 0;
+  const int grid = (int)std::max<i64>(1, std::min<i64>(pn.nunits, c->num_sms));
+  kfn<<<grid, kStreamWarps * 32, stream_smem_bytes<ST>(pn.rows), c->stream>>>(k);
+  check_launch("k_panel_stream");
+  count_launch(c);
 }
 
 // Builds the layout from the transposed CRS; null when it would not pay
@@ -1094,18 +1099,12 @@ std::unique_ptr<DevPanels> panel_build(fvg_ctx* c, const DevCRS& at, int master,
       fail(FVG_ERR_INVALID_ARG, "panel rows must be a multiple of 4 and at most " + std::to_string(cap));
     rows = force_rows;
   } else {
-    const i64 target = std::min<i64>(kPanelRowsAuto, cap);
-    const i64 grid = c->num_sms;  // one CTA per SM
-    const i64 np0 = (m + target - 1) / target;
-    if (np0 < 8) return nullptr;  // too few panels to pay for the split
-    if (np0 >= grid) {
-      // the fewest whole rounds over the persistent grid whose panels fit in
-      // shared memory (the tallest panels: the most columns count as hot)
-      const i64 rounds = (m + cap * grid - 1) / (cap * grid);
-      rows = ((m + rounds * grid - 1) / (rounds * grid) + 3) & ~3ll;
-    } else {
-      rows = target;
-    }
+    if (m < kPanelMinMatrix) return nullptr;  // too few panels to pay for the split
+    // the fewest whole rounds over the SMs whose panels fit in shared memory
+    // (the tallest panels: the most columns count as hot); one round of at
+    // least kPanelMinRows rows on smaller matrices
+    const i64 grid = c->num_sms, rounds = (m + cap * grid - 1) / (cap * grid);
+    rows = std::min<i64>(cap, std::max<i64>(kPanelMinRows, ((m + rounds * grid - 1) / (rounds * grid) + 3) & ~3ll));
   }
   const double mpp = min_pp > 0 ? min_pp : kPanelMinAuto;
   auto pn = std::make_unique<DevPanels>();
@@ -1128,7 +1127,7 @@ std::unique_ptr<DevPanels> panel_build(fvg_ctx* c, const DevCRS& at, int master,
   i64 nhot = 0;
   FVG_CUDA(cudaMemcpyAsync(&nhot, pos.as<i64>() + n, sizeof(i64), cudaMemcpyDeviceToHost, c->stream));
   FVG_CUDA(cudaStreamSynchronize(c->stream));
-  if (nhot == 0 || np * nhot >= (1ll << 31) - 1) return nullptr;
+  if (nhot == 0 || np * nhot >= (1ll << 31) - 1 || np >= (1ll << 26)) return nullptr;
   pn->nhot = nhot;
   pn->hot_cols.alloc(sizeof(i32) * nhot, c->stream);
   k_hot_list<<<grid_n(n), 256, 0, c->stream>>>(flag.as<i64>(), pos.as<i64>(), n, pn->hot_cols.as<i32>());
@@ -1181,51 +1180,10 @@ std::unique_ptr<DevPanels> panel_build(fvg_ctx* c, const DevCRS& at, int master,
   else if (master == FVG_F32) fill_planes<float>(c, at, *pn, B.as<i32>(), poff64.as<i64>(), flag.as<i64>(), coff64.as<i64>());
   else fill_planes<bf16>(c, at, *pn, B.as<i32>(), poff64.as<i64>(), flag.as<i64>(), coff64.as<i64>());
   cold.max_row = 0;  // not used by the product
-  pack_panels(c, *pn, nhot, np);
-  const i64 pieces = pn->npieces;
-  crs_sched(c, pn->cold, kWarpTile);  // the cold product's work items
-  pn->ypan.alloc(sizeof(float) * Q, c->stream);
-  pn->partials.alloc(sizeof(float) * std::max<i64>(pieces, 1), c->stream);
+  if (!stream_layout(c, *pn)) return nullptr;
   FVG_CUDA(cudaStreamSynchronize(c->stream));  // host vectors go out of scope
   return pn;
 }
-
-template <class VT>
-void launch_panel(fvg_ctx* c, const PanK& k, i64 rows) {
-  constexpr int threads = kPanelWarps * 32;
-  auto kfn = k_panel<VT>;
-  // the attribute once per device, at the device's limit (row panels and
-  // the forward head ask for different sizes call after call); resident
-  // CTAs per SM for the (device, size) pairs seen so far
-  static std::mutex mu;  // contexts of different host threads launch concurrently
-  static std::vector<int> attr_set;
-  static std::vector<std::pair<long long, int>> blocks_for;
-  const int smem = panel_smem_bytes<VT>(rows);
-  std::unique_lock<std::mutex> lock(mu);
-  if (std::find(attr_set.begin(), attr_set.end(), c->device) == attr_set.end()) {
-    int optin = 0;
-    FVG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-    FVG_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-    attr_set.push_back(c->device);
-  }
-  const long long key = ((long long)c->device << 32) | (unsigned)smem;
-  int blocks = 0;
-  for (auto& e : blocks_for)
-    if (e.first == key) blocks = e.second;
-  if (!blocks) {
-    int nb = 0;
-    FVG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kfn, threads, smem));
-    blocks = std::max(1, nb);
-    blocks_for.push_back({key, blocks});
-  }
-  lock.unlock();
-  const i64 nunits = (k.npanels + k.group - 1) / k.group;
-  const int grid = (int)std::max<i64>(1, std::min<i64>(nunits, (i64)blocks * c->num_sms));
-  kfn<<<grid, threads, smem, c->stream>>>(k);
-  check_launch("k_panel");
-  count_launch(c);
-}
-
 
 // The forward head of A: the H most frequent columns (ties: lower column
 // first), H at most what one CTA stages beside the staging buffers.  Null
@@ -1240,7 +1198,7 @@ std::unique_ptr<DevPanels> head_build(fvg_ctx* c, const DevCRS& a, const DevCRS&
   if (forced && force_cols > cap)
     fail(FVG_ERR_INVALID_ARG, "head columns must be at most " + std::to_string(cap));
   const i64 grid = c->num_sms;  // one CTA (one stretch of rows) per SM
-  if (!forced && m < 64 * grid * kPanelWarps) return nullptr;
+  if (!forced && m < kHeadMinMatrix) return nullptr;
   const i64 H = std::min<i64>(n, forced ? force_cols : cap);
   // the H largest column counts (from the transposed offsets), on the
   // device: a stable sort of the columns by decreasing count (ties keep
@@ -1263,8 +1221,9 @@ std::unique_ptr<DevPanels> head_build(fvg_ctx* c, const DevCRS& a, const DevCRS&
   hd->m = H;  // the staged slice: w at the head columns (slot order)
   hd->n = n;
   hd->rows = H;
-  // stretches of at most ~4096 rows, a whole number of them per CTA: the
-  // device packer takes one warp per stretch
+  // stretches of at most ~4096 rows, a whole number of them per CTA: their
+  // segments are sorted by length stretch by stretch, so that the sums of
+  // neighbouring rows are written close together
   const i64 per_cta = std::max<i64>(1, (m + grid * 4096 - 1) / (grid * 4096));
   hd->nhot = (m + grid * per_cta - 1) / (grid * per_cta);  // rows per stretch
   hd->npanels = (m + hd->nhot - 1) / hd->nhot;
@@ -1318,10 +1277,8 @@ std::unique_ptr<DevPanels> head_build(fvg_ctx* c, const DevCRS& a, const DevCRS&
   else if (master == FVG_F32) fill(float{});
   else fill(bf16{});
   tail.max_row = 0;
-  pack_panels(c, *hd, chunk, np);
-  crs_sched(c, tail, kWarpTile);
-  hd->ypan.alloc(sizeof(float) * Q, c->stream);
-  hd->partials.alloc(sizeof(float) * std::max<i64>(hd->npieces, 1), c->stream);
+  hd->group = (np + grid - 1) / grid;  // a CTA's whole share of the stretches
+  if (!stream_layout(c, *hd)) return nullptr;
   FVG_CUDA(cudaStreamSynchronize(c->stream));  // host vectors go out of scope
   return hd;
 }
@@ -1344,8 +1301,18 @@ DevPanels* panels_for(fvg_ctx* c, fvg_matrix* M) {
 }
 
 void panel_ensure_plane(fvg_ctx* c, DevPanels& pn, int dt) {
-  ensure_plane_generic(c, pn.val, pn.E, dt, pn.master);
+  if (!pn.rec[dt].p) {
+    ensure_plane_generic(c, pn.val, pn.E, dt, pn.master);
+    if (dt == FVG_F32) fill_records<FVG_F32>(c, pn);
+    else fill_records<FVG_BF16>(c, pn);
+    if (dt != pn.master) pn.val[dt].release();  // the records hold them
+  }
+  if (!pn.ypan.p) {
+    pn.ypan.alloc(sizeof(float) * std::max<i64>(pn.npanels * pn.nhot, 1), c->stream);
+    pn.partials.alloc(sizeof(float) * std::max<i64>(pn.npieces, 1), c->stream);
+  }
   crs_ensure_plane(c, pn.cold, dt, pn.master);
+  crs_sched(c, pn.cold, kWarpTile);  // the cold product's work items
 }
 
 i64 panel_scratch_bytes(fvg_ctx* c, DevPanels& pn, int storage) { return crs_pass_scratch_bytes(c, pn.cold, storage); }
@@ -1358,28 +1325,8 @@ void panel_trans_mv(fvg_ctx* c, DevPanels& pn, int storage, const float* r, int 
   ProfScope pr(c, prof_key);
   // cold columns (and zeros for the hot ones) by the transposed CRS kernel
   crs_pass(c, pn.cold, storage, FVG_F32, r, y_dt, y, EPI_STORE, nullptr, scratch, P_NKEYS);
-  PanK k;
-  k.poff = pn.poff.as<i32>();
-  k.prow = pn.prow.as<uint16_t>();
-  k.val = pn.val[storage].p;
-  k.r = r;
-  k.m = pn.m;
-  k.rows = pn.rows;
-  k.npanels = pn.npanels;
-  k.items = pn.items.as<Item>();
-  k.pitem0 = pn.pitem0.as<i32>();
-  k.long_rows = pn.long_rows.as<i32>();
-  k.plong0 = pn.plong0.as<i32>();
-  k.long_piece0 = pn.long_piece0.as<i32>();
-  k.partials = pn.partials.as<float>();
-  k.ypan = pn.ypan.as<float>();
-  k.err = c->dev_err;
-  k.wait_limit = copy_polls(c);
-  k.aligned = ((reinterpret_cast<uintptr_t>(r) & 15) == 0) ? 1 : 0;
-  k.xmap = nullptr;
-  k.group = 1;
-  if (storage == FVG_F32) launch_panel<float>(c, k, pn.rows);
-  else launch_panel<bf16>(c, k, pn.rows);
+  if (storage == FVG_F32) launch_stream<FVG_F32>(c, pn, r, pn.ypan.p, pn.partials.p);
+  else launch_stream<FVG_BF16>(c, pn, r, pn.ypan.p, pn.partials.p);
   const unsigned cg = (unsigned)std::max<i64>(1, std::min<i64>((pn.nhot + 31) / 32, 2 * c->num_sms));
   if (y_dt == FVG_F64)
     k_panel_colsum<double><<<cg, 1024, 0, c->stream>>>(pn.ypan.as<float>(), pn.hot_cols.as<i32>(), pn.nhot,
@@ -1409,10 +1356,7 @@ DevPanels* head_for(fvg_ctx* c, fvg_matrix* M) {
   return M->head.get();
 }
 
-void head_ensure_plane(fvg_ctx* c, DevPanels& hd, int dt) {
-  ensure_plane_generic(c, hd.val, hd.E, dt, hd.master);
-  crs_ensure_plane(c, hd.cold, dt, hd.master);
-}
+void head_ensure_plane(fvg_ctx* c, DevPanels& hd, int dt) { panel_ensure_plane(c, hd, dt); }
 
 i64 head_scratch_bytes(fvg_ctx* c, DevPanels& hd, int storage) { return crs_pass_scratch_bytes(c, hd.cold, storage); }
 
@@ -1421,28 +1365,8 @@ void head_logreg_pass(fvg_ctx* c, DevPanels& hd, int storage, const float* w, co
   if (storage == FVG_F64) fail(FVG_ERR_INTERNAL, "the head pass runs on FP32 or BF16 values");
   head_ensure_plane(c, hd, storage);
   ProfScope pr(c, prof_key);
-  PanK k;
-  k.poff = hd.poff.as<i32>();
-  k.prow = hd.prow.as<uint16_t>();
-  k.val = hd.val[storage].p;
-  k.r = w;
-  k.m = hd.m;
-  k.rows = hd.rows;
-  k.npanels = hd.npanels;
-  k.items = hd.items.as<Item>();
-  k.pitem0 = hd.pitem0.as<i32>();
-  k.long_rows = hd.long_rows.as<i32>();
-  k.plong0 = hd.plong0.as<i32>();
-  k.long_piece0 = hd.long_piece0.as<i32>();
-  k.partials = hd.partials.as<float>();
-  k.ypan = hd.ypan.as<float>();
-  k.err = c->dev_err;
-  k.wait_limit = copy_polls(c);
-  k.aligned = 0;
-  k.xmap = hd.hot_cols.as<i32>();
-  k.group = (hd.npanels + c->num_sms - 1) / c->num_sms;  // a CTA's whole share of the stretches
-  if (storage == FVG_F32) launch_panel<float>(c, k, hd.rows);
-  else launch_panel<bf16>(c, k, hd.rows);
+  if (storage == FVG_F32) launch_stream<FVG_F32>(c, hd, w, hd.ypan.p, hd.partials.p);
+  else launch_stream<FVG_BF16>(c, hd, w, hd.ypan.p, hd.partials.p);
   LogregEpi t = lr;
   t.ybase = hd.ypan.as<float>();
   crs_pass(c, hd.cold, storage, FVG_F32, w, FVG_F32, nullptr, EPI_LOGREG, &t, scratch, P_NKEYS);
@@ -1453,69 +1377,17 @@ void head_logreg_pass(fvg_ctx* c, DevPanels& hd, int storage, const float* w, co
 // ------------------------------------------------------------ split storage
 namespace fvg {
 
-namespace {
-void launch_panel_split(fvg_ctx* c, const PanSK& k, i64 rows) {
-  constexpr int threads = kSplitWarps * 32;
-  static std::mutex mu;  // contexts of different host threads launch concurrently
-  static std::vector<int> attr_set;
-  const int smem = panel_split_smem_bytes(rows);
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if (std::find(attr_set.begin(), attr_set.end(), c->device) == attr_set.end()) {
-      int optin = 0;
-      FVG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-      FVG_CUDA(cudaFuncSetAttribute(k_panel_split<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-      FVG_CUDA(cudaFuncSetAttribute(k_panel_split<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-      attr_set.push_back(c->device);
-    }
-  }
-  // the row panels (no shared slice map) take the middle-row pass
-  const bool panels = k.xmap == nullptr;
-  const void* kfn = panels ? (const void*)k_panel_split<true> : (const void*)k_panel_split<false>;
-  const int blocks = occupancy_blocks(kfn, threads, (size_t)smem);
-  const i64 nunits = (k.npanels + k.group - 1) / k.group;
-  const int grid = (int)std::max<i64>(1, std::min<i64>(nunits, (i64)blocks * c->num_sms));
-  if (panels) k_panel_split<true><<<grid, threads, smem, c->stream>>>(k);
-  else k_panel_split<false><<<grid, threads, smem, c->stream>>>(k);
-  check_launch("k_panel_split");
-  count_launch(c);
-}
-
-PanSK split_args(fvg_ctx* c, DevPanels& pn, const void* x) {
-  PanSK k;
-  k.poff = pn.poff.as<i32>();
-  k.prow = pn.prow.as<uint16_t>();
-  k.vh = pn.val[FVG_F32].as<float>();
-  k.vl = pn.lo.as<unsigned short>();
-  k.x = (const float2*)x;
-  k.m = pn.m;
-  k.rows = pn.rows;
-  k.npanels = pn.npanels;
-  const PanelItems& si = *pn.split_items;
-  k.items = si.items.as<Item>();
-  k.pitem0 = si.pitem0.as<i32>();
-  k.long_rows = si.long_rows.as<i32>();
-  k.plong0 = si.plong0.as<i32>();
-  k.long_piece0 = si.long_piece0.as<i32>();
-  k.partials = pn.partials2.as<float2>();
-  k.ypan = pn.ypan2.as<float2>();
-  k.err = c->dev_err;
-  k.wait_limit = copy_polls(c);
-  k.xmap = nullptr;
-  k.group = 1;
-  return k;
-}
-}  // namespace
-
 void panel_ensure_split(fvg_ctx* c, DevPanels& pn) {
-  if (pn.rows > panel_rows_cap(c))
-    fail(FVG_ERR_INTERNAL, "panel layout too tall for the split kernel");
-  ensure_split_planes(c, pn.val, pn.E, pn.master, pn.lo);
+  if (!pn.rec[FVG_SPLIT].p) {
+    ensure_split_planes(c, pn.val, pn.E, pn.master, pn.lo);
+    fill_records<FVG_SPLIT>(c, pn);
+    if (pn.master != FVG_F32) pn.val[FVG_F32].release();  // the records hold both
+    pn.lo.release();
+  }
   crs_ensure_split(c, pn.cold, pn.master);
-  if (!pn.split_items) pack_split_items(c, pn);
   if (!pn.ypan2.p) {
     pn.ypan2.alloc(sizeof(float2) * std::max<i64>(pn.npanels * pn.nhot, 1), c->stream);
-    pn.partials2.alloc(sizeof(float2) * std::max<i64>(pn.split_items->npieces, 1), c->stream);
+    pn.partials2.alloc(sizeof(float2) * std::max<i64>(pn.npieces, 1), c->stream);
   }
 }
 
@@ -1527,7 +1399,7 @@ void panel_trans_mv_split(fvg_ctx* c, DevPanels& pn, const void* r, double* y, v
   panel_ensure_split(c, pn);
   // cold columns (and zeros for the hot ones) by the transposed CRS kernel
   crs_pass_split(c, pn.cold, r, false, y, scratch, P_NKEYS);
-  launch_panel_split(c, split_args(c, pn, r), pn.rows);
+  launch_stream<FVG_SPLIT>(c, pn, r, pn.ypan2.p, pn.partials2.p);
   const unsigned cg = (unsigned)std::max<i64>(1, std::min<i64>((pn.nhot + 31) / 32, 2 * c->num_sms));
   k_panel_colsum_split<<<cg, 1024, 0, c->stream>>>(pn.ypan2.as<float2>(), pn.hot_cols.as<i32>(), pn.nhot,
                                                     pn.npanels, y);
@@ -1537,10 +1409,7 @@ void panel_trans_mv_split(fvg_ctx* c, DevPanels& pn, const void* r, double* y, v
 
 void head_pass_split(fvg_ctx* c, DevPanels& hd, const void* w, void* wtx, void* scratch) {
   panel_ensure_split(c, hd);
-  PanSK k = split_args(c, hd, w);
-  k.xmap = hd.hot_cols.as<i32>();
-  k.group = (hd.npanels + c->num_sms - 1) / c->num_sms;  // a CTA's whole share of the stretches
-  launch_panel_split(c, k, hd.rows);
+  launch_stream<FVG_SPLIT>(c, hd, w, hd.ypan2.p, hd.partials2.p);
   crs_pass_split(c, hd.cold, w, true, wtx, scratch, P_NKEYS);
 }
 
