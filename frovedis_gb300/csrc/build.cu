@@ -190,6 +190,7 @@ void crs_build_transpose(fvg_ctx* c, const DevCRS& a, DevCRS& t, int master) {
   count_launch(c);
   keys.release();
   t.max_row = max_row_len(c, t.off.as<i32>(), t.m);
+  FVG_CUDA(cudaStreamSynchronize(c->stream));
   check_device_error(c);  // the sort's bounded copy waits
 }
 

@@ -104,8 +104,13 @@ FVG_API fvg_status fvg_ctx_create(int device, fvg_ctx** out) {
     c->device = device;
     FVG_CUDA(cudaSetDevice(device));
     FVG_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
-    FVG_CUDA(cudaMalloc(&c->dev_err, 256));
-    FVG_CUDA(cudaMemset(c->dev_err, 0, 256));
+    FVG_CUDA(cudaHostAlloc(&c->host_page, 4096, cudaHostAllocMapped));
+    memset(c->host_page, 0, 4096);
+    void* dev_page = nullptr;
+    FVG_CUDA(cudaHostGetDevicePointer(&dev_page, c->host_page, 0));
+    c->dev_err = (unsigned*)dev_page;
+    c->host_words = (double*)((char*)c->host_page + 256);
+    c->dev_words = (double*)((char*)dev_page + 256);
     FVG_CUDA(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device));
     c->grid_spmv = c->num_sms * std::max(1, crs_blocks_per_sm());
     cudaMemPool_t pool;
@@ -121,6 +126,7 @@ FVG_API fvg_status fvg_ctx_create(int device, fvg_ctx** out) {
     fprintf(stderr, "fvg_ctx_create: %s\n", e.msg.c_str());
     if (c) {
       if (c->stream) cudaStreamDestroy(c->stream);
+      if (c->host_page) cudaFreeHost(c->host_page);
       delete c;
     }
     return e.code;
@@ -150,7 +156,7 @@ FVG_API void fvg_ctx_destroy(fvg_ctx* c) {
   }
   c->matrices.clear();
   cudaStreamSynchronize(c->stream);
-  if (c->dev_err) cudaFree(c->dev_err);
+  if (c->host_page) cudaFreeHost(c->host_page);
   prof_destroy(c);
   cudaStreamDestroy(c->stream);
   delete c;

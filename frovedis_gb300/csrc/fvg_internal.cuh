@@ -229,9 +229,16 @@ struct fvg_ctx {
   fvg::Profiler* prof = nullptr;  // owned; prof_create / prof_destroy
   // live matrices: destroying the context releases their device memory
   std::vector<fvg_matrix*> matrices;
-  // device error word: a kernel that must give up (a bounded wait that ran
-  // out) sets a bit here instead of trapping; read after each call
+  // One page of page-locked host memory that kernels write directly, so that
+  // the host reads it after a stream synchronisation without a copy:
+  // host_page the host's address, dev_err / dev_words the device's.
+  // Error word: a kernel that must give up (a bounded wait that ran out) sets
+  // a bit here instead of trapping; read after each call.
+  void* host_page = nullptr;
   unsigned* dev_err = nullptr;
+  // a call's scalars (the context serves one call at a time)
+  double* host_words = nullptr;
+  double* dev_words = nullptr;
   // poll budget of the bounded device-side waits (< 0: the defaults below)
   int64_t wait_limit = -1;
   // batched trainers: evaluations run (the line-search trials that had a
@@ -285,14 +292,15 @@ struct ProfScope {
 inline void count_launch(fvg_ctx* c, int n = 1) { c->launches += n; }
 void check_launch(const char* what);
 // Default poll budgets of the bounded device-side waits: the L-BFGS
-// direction's grid barriers (2^24 polls of ~32 ns) and the panel kernels'
+// direction's waits for all CTAs' sums (2^21 polls of ~0.5 us) and the panel kernels'
 // bulk-copy waits (2^16 polls, each a sleep of at most 20 us in the
 // barrier: ~1.3 s); a context may lower them for testing.
-constexpr unsigned kBarrierPolls = 1u << 24;
+constexpr unsigned kBarrierPolls = 1u << 21;
 constexpr unsigned kCopyPolls = 1u << 16;
 inline unsigned barrier_polls(const fvg_ctx* c) { return c->wait_limit < 0 ? kBarrierPolls : (unsigned)c->wait_limit; }
 inline unsigned copy_polls(const fvg_ctx* c) { return c->wait_limit < 0 ? kCopyPolls : (unsigned)c->wait_limit; }
-// Reads (and clears) the device error word; fails when a kernel reported one.
+// Reads (and clears) the error word, after the stream has been synchronised;
+// fails when a kernel reported one.
 void check_device_error(fvg_ctx* c);
 
 // ------------------------------------------------------------ utilities

@@ -259,12 +259,7 @@ void multinomial_train(fvg_ctx* c, fvg_matrix* M, const double* label_h, const d
   colpart.alloc(sizeof(double) * (size_t)nblk * K, s);
   sqpart.alloc(sizeof(double) * nblk, s);
   out.alloc(256, s);
-  double* hout = nullptr;
-  FVG_CUDA(cudaMallocHost(&hout, sizeof(double)));
-  struct Free {
-    double* p;
-    ~Free() { cudaFreeHost(p); }
-  } free_h{hout};
+  double* const hout = c->host_words;
   const unsigned dg = (unsigned)std::max<i64>(1, std::min<i64>(((i64)nk + 255) / 256, 4 * (i64)c->num_sms));
   const size_t es = mixed ? 4 : 8;
 

@@ -685,14 +685,17 @@ void crs_pass(fvg_ctx* c, DevCRS& a, int storage, int x_dt, const void* x, int y
   if (!a.val[storage].p) fail(FVG_ERR_INTERNAL, "missing value plane for the requested storage");
   const size_t at_size = (storage == FVG_F64) ? 8 : 4;
   DBuf tmp;
-  PassScratch ps;
-  if (!scratch) {
-    size_t bytes = carve(nullptr, s, c->grid_spmv, at_size, nullptr);
-    tmp.alloc(bytes, c->stream);
+  PassScratch ps = {};
+  if (scratch) {
+    carve((char*)scratch, s, c->grid_spmv, at_size, &ps);
+  } else if (epi == EPI_STORE) {  // a lone product: long rows' partials are all it needs
+    if (s.npieces > 0) tmp.alloc(at_size * (size_t)s.npieces, c->stream);
+    ps.partials = tmp.p;
+  } else {
+    tmp.alloc(carve(nullptr, s, c->grid_spmv, at_size, nullptr), c->stream);
     FVG_CUDA(cudaMemsetAsync(tmp.p, 0, 256, c->stream));  // ticket
-    scratch = tmp.p;
+    carve((char*)tmp.p, s, c->grid_spmv, at_size, &ps);
   }
-  carve((char*)scratch, s, c->grid_spmv, at_size, &ps);
   if (epi == EPI_LOGREG && storage != FVG_F64 && !(lr && lr->label_f))
     fail(FVG_ERR_INTERNAL, "FP32 logistic pass needs FP32 labels");
   ProfScope pr(c, prof_key);

@@ -23,11 +23,10 @@ void check_launch(const char* what) {
 }
 
 void check_device_error(fvg_ctx* c) {
-  unsigned h = 0;
-  FVG_CUDA(cudaMemcpyAsync(&h, c->dev_err, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
-  FVG_CUDA(cudaStreamSynchronize(c->stream));
+  volatile unsigned* word = (unsigned*)c->host_page;
+  const unsigned h = *word;
   if (h) {
-    FVG_CUDA(cudaMemsetAsync(c->dev_err, 0, sizeof(unsigned), c->stream));
+    *word = 0u;
     std::string what;
     if (h & 2u) what += " a bulk copy did not complete in its poll budget;";
     if (h & 4u) what += " a grid barrier was not reached in its poll budget;";
