@@ -94,7 +94,7 @@ FVG_API int64_t fvg_ctx_kernel_launches(fvg_ctx* ctx);
  * kernels' bulk-copy waits).  A wait that runs out is abandoned: the kernel
  * records it in the context's error word and finishes (a copy in flight is
  * still drained), and the call returns FVG_ERR_INTERNAL; the context stays
- * usable.  polls < 0 restores the defaults (2^24 barrier polls, 2^16 copy
+ * usable.  polls < 0 restores the defaults (2^21 grid-wait polls, 2^16 copy
  * polls of up to 20 us each — about a second, far beyond any healthy wait);
  * 0 makes every wait that is not already complete give up at once.  No reference counterpart (the
  * reference's ranks report failures through MPI, core/mpi_rpc.cc:471-491);
