@@ -32,10 +32,11 @@
 // identically for all active models, so its indices are host constants of
 // the iteration.  Control words on the device (models searching, models
 // active, the precision switch) gate every launch: a launch whose word is 0
-// returns at once, so the whole training is one fixed launch sequence,
-// captured once as a CUDA graph and launched once.  With BF16 values the
-// switch to FP32 values (the refinement phase) is decided on the device too,
-// once any model's gradient norm stalls.
+// returns at once.  The whole training is one CUDA graph, launched once; the
+// trials of a line search are a WHILE node of it that kb_decide ends (see
+// lbfgs_multi_train).  With BF16 values the switch to FP32 values (the
+// refinement phase) is decided on the device too, once any model's gradient
+// norm stalls.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -47,6 +48,7 @@ namespace fvg {
 constexpr int kBT = 256;
 constexpr int kBMaxHist = 32;
 constexpr int kBMaxModels = 256;
+constexpr int kBMaxTrials = 10;  // of one line search
 
 struct ColState {
   double rho[kBMaxHist], yy[kBMaxHist], al[kBMaxHist], beta[kBMaxHist];
@@ -73,7 +75,16 @@ enum BCtl {
   C_ONE,         // always 1
   C_NEVAL,       // evaluations run
   C_NMODEL,      // (dataset, model) evaluations run
+  C_T,           // the line search's trial, from 1
+  C_NTRIAL,      // trials run
   C_NCTL = 16
+};
+
+// The WHILE node a line search's trials run in (on == 0: no graph; the
+// trials are launched one after the other).
+struct TrialLoop {
+  cudaGraphConditionalHandle h = 0;
+  int on = 0;
 };
 
 __device__ __forceinline__ void set_flags(int* ctl) {
@@ -394,7 +405,7 @@ __global__ void __launch_bounds__(kBT, 4) kb_step_norm(const double* __restrict_
 }
 
 // models still searching: trial model + regulariser (see k_trial)
-__global__ void __launch_bounds__(kBT, 4) kb_trial(int t, const double* __restrict__ W, const double* __restrict__ STEP,
+__global__ void __launch_bounds__(kBT, 4) kb_trial(const double* __restrict__ W, const double* __restrict__ STEP,
                                                 double* __restrict__ NW, float* __restrict__ NWF,
                                                 const double* __restrict__ B0, double* __restrict__ B1, int rtype,
                                                 int eta_one, int no_eta, BArgs a) {
@@ -402,7 +413,7 @@ __global__ void __launch_bounds__(kBT, 4) kb_trial(int t, const double* __restri
   if (!on) return;
   const ColState& s = a.st[mj];
   if (!s.searching) return;
-  const double f = s.factor[t], fl = s.flip, lambda = s.lambda;
+  const double f = s.factor[__ldcg(a.ctl + C_T)], fl = s.flip, lambda = s.lambda;
   const double eta = eta_one ? 1.0 : f;
   const double scale = fmax(0.0, 1.0 - (lambda * eta));
   rows_grouped<kRowGroup>(r0, rstep, n, [&](i64 r) { const i64 e = e0 + r * ld; return V2{W[e], STEP[e]}; },
@@ -487,20 +498,25 @@ __device__ __forceinline__ void count_into(int n, int* ctl, int w) {
 
 // accept decision of trial t (LBFGS_SEARCH_TOL, lbfgs_parallelizer.hpp:
 // 155, 329; the 10th trial is taken whatever its loss)
-// (the models still searching: their masks in smask)
-__global__ void __launch_bounds__(kBT, 4) kb_decide(int t, const double* __restrict__ EV, int nd, int ld, int nwd,
-                                                 ColState* st, int* ctl, unsigned long long* smask) {
+// (the models still searching: their masks in smask).  The trial loop goes
+// on while a model searches; the tenth trial leaves none.
+__global__ void __launch_bounds__(kBT, 4) kb_decide(const double* __restrict__ EV, int nd, int ld, int nwd,
+                                                 ColState* st, int* ctl, unsigned long long* smask, TrialLoop loop) {
   if (ctl[C_TRIAL] == 0) return;
   const int nm = nd * ld;
+  const int t = ctl[C_T];
+  __syncthreads();
   if (threadIdx.x == 0) {  // the trial's evaluation ran
     ctl[C_NEVAL] += 1;
     ctl[C_NMODEL] += ctl[C_SEARCH];
+    ctl[C_NTRIAL] += 1;
+    ctl[C_T] = t + 1;
   }
   int n = 0;
   for (int j = threadIdx.x; j < nm; j += kBT) {
     ColState& s = st[j];
     if (!s.searching) continue;
-    if (EV[2 * j] - s.loss < 1e-4 || t == 10) {
+    if (EV[2 * j] - s.loss < 1e-4 || t >= kBMaxTrials) {
       s.searching = 0;
       s.trials = t;
     } else {
@@ -509,12 +525,14 @@ __global__ void __launch_bounds__(kBT, 4) kb_decide(int t, const double* __restr
   }
   count_into(n, ctl, C_SEARCH);
   __syncthreads();
+  if (loop.on && threadIdx.x == 0) cudaGraphSetConditional(loop.h, ctl[C_SEARCH] > 0);
   build_masks(st, nd, ld, nwd, 0, smask);
 }
 
 __global__ void __launch_bounds__(kBT, 4) kb_begin_search(int nd, int ld, int nwd, ColState* st, int* ctl,
-                                                       unsigned long long* smask) {
+                                                       unsigned long long* smask, TrialLoop loop) {
   const int nm = nd * ld;
+  if (threadIdx.x == 0) ctl[C_T] = 1;
   int n = 0;
   for (int j = threadIdx.x; j < nm; j += kBT) {
     st[j].searching = st[j].active;
@@ -522,6 +540,7 @@ __global__ void __launch_bounds__(kBT, 4) kb_begin_search(int nd, int ld, int nw
   }
   count_into(n, ctl, C_SEARCH);
   __syncthreads();
+  if (loop.on && threadIdx.x == 0) cudaGraphSetConditional(loop.h, ctl[C_SEARCH] > 0);
   build_masks(st, nd, ld, nwd, 0, smask);
 }
 
@@ -827,15 +846,67 @@ struct BatchEval {
   }
 };
 
-// Ends a stream capture that an exception interrupted.
-struct CaptureGuard {
+// A graph built from captured stretches of one stream and WHILE nodes.  The
+// trials of a line search end at a count only the device knows: as ten gated
+// copies of the trial's launches they cost 2 us a launch that finds its gate
+// closed, and 1.7 us a node to capture and instantiate (a fifth to a half of
+// a training of 200 000 rows); a WHILE node costs 3.5 us a pass over what its
+// launches take.
+struct LoopGraph {
   cudaStream_t s;
+  cudaGraph_t g = nullptr;
   bool open = false;
-  ~CaptureGuard() {
-    if (!open) return;
-    cudaGraph_t g = nullptr;
-    cudaStreamEndCapture(s, &g);
+  std::vector<cudaGraphNode_t> tail;  // what the next stretch of `g` follows
+
+  explicit LoopGraph(cudaStream_t s_) : s(s_) { FVG_CUDA(cudaGraphCreate(&g, 0)); }
+  LoopGraph(const LoopGraph&) = delete;
+  LoopGraph& operator=(const LoopGraph&) = delete;
+  ~LoopGraph() {
+    if (open) {  // a capture that an exception interrupted
+      cudaGraph_t x = nullptr;
+      cudaStreamEndCapture(s, &x);
+    }
     if (g) cudaGraphDestroy(g);
+  }
+  void begin(cudaGraph_t into, bool after_tail) {
+    FVG_CUDA(cudaStreamBeginCaptureToGraph(s, into, after_tail ? tail.data() : nullptr, nullptr,
+                                           after_tail ? tail.size() : 0, cudaStreamCaptureModeThreadLocal));
+    open = true;
+  }
+  void end(bool keep_tail) {
+    if (keep_tail) {
+      cudaStreamCaptureStatus st;
+      const cudaGraphNode_t* dep = nullptr;
+      const cudaGraphEdgeData* edge = nullptr;
+      size_t n = 0;
+      FVG_CUDA(cudaStreamGetCaptureInfo(s, &st, nullptr, nullptr, &dep, &edge, &n));
+      tail.assign(dep, dep + n);
+    }
+    open = false;
+    cudaGraph_t x = nullptr;
+    FVG_CUDA(cudaStreamEndCapture(s, &x));
+  }
+  cudaGraphConditionalHandle handle() {
+    cudaGraphConditionalHandle h = 0;
+    FVG_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, 0));
+    return h;
+  }
+  // inside a stretch: `body`'s launches again and again while the handle is set
+  template <class F>
+  void loop(cudaGraphConditionalHandle h, F body) {
+    end(true);
+    cudaGraphNodeParams p{};
+    p.type = cudaGraphNodeTypeConditional;
+    p.conditional.handle = h;
+    p.conditional.type = cudaGraphCondTypeWhile;
+    p.conditional.size = 1;
+    cudaGraphNode_t node = nullptr;
+    FVG_CUDA(cudaGraphAddNode(&node, g, tail.data(), nullptr, tail.size(), &p));
+    begin(p.conditional.phGraph_out[0], false);
+    body();
+    end(false);
+    tail.assign(1, node);
+    begin(g, true);
   }
 };
 
@@ -1021,13 +1092,20 @@ void lbfgs_multi_train(fvg_ctx* c, const std::vector<fvg_matrix*>& mats, const s
   };
   const int* one = ctl_i + C_ONE;
 
-  // the whole training as one launch sequence
-  auto run = [&]() {
+  // the whole training as one launch sequence; with a graph, the trials of an
+  // iteration as one loop of it
+  i64 trial_launches = 0, trial_copies = 0;  // of one trial; trials issued or captured
+  auto run = [&](LoopGraph* lg) {
     ev.eval(storage, weights_for(storage, W.as<double>(), one), B0, G.as<double>(), EV.as<double>(), one, nullptr);
     norms(G.as<double>(), 1, C_ONE, nullptr);
     int rear = 0, front = 0;
     for (i64 it = 1; it <= p->num_iteration; it++) {
       const int kh = (int)std::min<i64>(it - 1, h);
+      TrialLoop tl;
+      if (lg) {
+        tl.h = lg->handle();
+        tl.on = 1;
+      }
       {
         ProfScope ps(c, P_LBFGS);
         for (int q = kh - 1; q >= 0; q--)
@@ -1039,14 +1117,15 @@ void lbfgs_multi_train(fvg_ctx* c, const std::vector<fvg_matrix*>& mats, const s
         kb_step<<<vgrid, kBT, 0, s>>>(kh, rear, G.as<double>(), Z.as<double>(), STEP.as<double>(), S.as<double>(),
                                       gated(C_ACTIVE));
         kb_step_norm<<<vgrid, kBT, 0, s>>>(STEP.as<double>(), gated(C_ACTIVE));
-        kb_begin_search<<<1, kBT, 0, s>>>(nd, ld, nwd, a.st, ctl_i, smask);
+        kb_begin_search<<<1, kBT, 0, s>>>(nd, ld, nwd, a.st, ctl_i, smask, tl);
         check_launch("batched two-loop");
         count_launch(c, 2 * kh + 3);
       }
-      for (int t = 1; t <= 10; t++) {
+      auto trial = [&]() {
+        const int64_t l0 = c->launches;
         {
           ProfScope ps(c, P_LBFGS);
-          kb_trial<<<vgrid, kBT, 0, s>>>(t, W.as<double>(), STEP.as<double>(), NW.as<double>(),
+          kb_trial<<<vgrid, kBT, 0, s>>>(W.as<double>(), STEP.as<double>(), NW.as<double>(),
                                          mixed ? WF.as<float>() : nullptr, B0, B1, p->reg_type, 0, p->l2_no_eta,
                                          gated(C_TRIAL));
           check_launch("kb_trial");
@@ -1058,9 +1137,16 @@ void lbfgs_multi_train(fvg_ctx* c, const std::vector<fvg_matrix*>& mats, const s
         ev.eval(storage, x, B1, NG.as<double>(), EV.as<double>(), ctl_i + C_EVAL_LO, smask);
         if (refine) ev.eval(FVG_F32, x, B1, NG.as<double>(), EV.as<double>(), ctl_i + C_EVAL_HI, smask);
         norms(NG.as<double>(), 0, C_TRIAL, smask);
-        kb_decide<<<1, kBT, 0, s>>>(t, EV.as<double>(), nd, ld, nwd, a.st, ctl_i, smask);
+        kb_decide<<<1, kBT, 0, s>>>(EV.as<double>(), nd, ld, nwd, a.st, ctl_i, smask, tl);
         check_launch("kb_decide");
         count_launch(c);
+        trial_launches = c->launches - l0;
+        trial_copies++;
+      };
+      if (lg) {
+        lg->loop(tl.h, trial);
+      } else {
+        for (int t = 1; t <= kBMaxTrials; t++) trial();
       }
       const int nf = (kh == 0) ? 0 : (front + 1) % h;
       {
@@ -1092,18 +1178,14 @@ void lbfgs_multi_train(fvg_ctx* c, const std::vector<fvg_matrix*>& mats, const s
     }
   };
   if (c->profiling) {
-    run();  // per-phase timing needs the launches issued one by one
+    run(nullptr);  // per-phase timing needs the launches issued one by one
   } else {
-    CaptureGuard cg{s};
-    FVG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    cg.open = true;
-    run();
-    cudaGraph_t graph = nullptr;
-    cg.open = false;
-    FVG_CUDA(cudaStreamEndCapture(s, &graph));
+    LoopGraph lg(s);
+    lg.begin(lg.g, false);
+    run(&lg);
+    lg.end(false);
     cudaGraphExec_t exec = nullptr;
-    const cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
-    cudaGraphDestroy(graph);
+    const cudaError_t ie = cudaGraphInstantiate(&exec, lg.g, 0);
     if (ie != cudaSuccess) fail(FVG_ERR_INTERNAL, std::string("graph instantiation: ") + cudaGetErrorString(ie));
     const cudaError_t le = cudaGraphLaunch(exec, s);
     const cudaError_t se = cudaStreamSynchronize(s);
@@ -1127,6 +1209,7 @@ void lbfgs_multi_train(fvg_ctx* c, const std::vector<fvg_matrix*>& mats, const s
   FVG_CUDA(cudaMemcpyAsync(bb.data(), B0, sizeof(double) * nm, cudaMemcpyDeviceToHost, s));
   FVG_CUDA(cudaMemcpyAsync(hctl.data(), ctl_i, sizeof(int) * C_NCTL, cudaMemcpyDeviceToHost, s));
   FVG_CUDA(cudaStreamSynchronize(s));
+  if (!c->profiling) c->launches += trial_launches * (hctl[C_NTRIAL] - trial_copies);  // each loop was counted once
   c->batch_evals += hctl[C_NEVAL];
   c->batch_model_evals += hctl[C_NMODEL];
   for (int d = 0; d < nd; d++)
