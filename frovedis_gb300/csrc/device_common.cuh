@@ -23,6 +23,37 @@ template <class T> __device__ __forceinline__ T block_sum256(T v) {
   return t;  // valid in thread 0
 }
 
+// ---------------------------------------------------- Euclidean norms
+// The reference scales by the largest magnitude first (vector_operations.hpp:
+// 227-264), which takes two passes.  Here the squares are summed in three
+// ranges whose scaling (a power of two, exact) keeps them within FP64, after
+// J. L. Blue ("A portable Fortran program to find the Euclidean norm of a
+// vector", ACM TOMS 4(1), 1978): the exponent picks the range, one fused
+// multiply-add per element.  An infinity makes the norm NaN, and so does a NaN
+// beside an element other than 0; with zeros only it leaves 0 (the largest
+// magnitude ignores it).
+__device__ __forceinline__ void norm_add(double& tiny, double& mid, double& huge, double g) {
+  const int ex = (__double2hiint(g) >> 20) & 0x7ff;  // biased exponent
+  if (ex >= 1023 - 480 && ex <= 1023 + 480) {
+    mid = fma(g, g, mid);
+  } else if (ex < 1023 - 480) {
+    const double x = g * 0x1p+600;
+    tiny = fma(x, x, tiny);
+  } else if (ex < 0x7ff) {
+    const double x = g * 0x1p-600;
+    huge = fma(x, x, huge);
+  } else {
+    huge += g - g;          // NaN
+    if (g == g) mid += 1.0;  // an infinity: an element other than 0
+  }
+}
+__device__ __forceinline__ double norm_of(double tiny, double mid, double huge) {
+  if (huge != huge) return tiny > 0.0 || mid > 0.0 ? huge : 0.0;
+  if (huge > 0.0) return sqrt(huge + mid * 0x1p-600 * 0x1p-600) * 0x1p+600;
+  if (mid > 0.0) return sqrt(mid + tiny * 0x1p-600 * 0x1p-600);
+  return sqrt(tiny) * 0x1p-600;
+}
+
 // ---------------------------------------------------- compensated sums
 struct CSum {  // Neumaier, FP64 (the FP64 path)
   double s = 0.0, c = 0.0;

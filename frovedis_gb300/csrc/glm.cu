@@ -18,7 +18,7 @@
 #include <algorithm>
 #include <cmath>
 
-#include "fvg_internal.cuh"
+#include "device_common.cuh"
 
 namespace fvg {
 
@@ -398,32 +398,16 @@ __global__ void __launch_bounds__(kVecThreads) k_trial(int j, const double* __re
   if (blockIdx.x == 0 && threadIdx.x == 0) st->b[1] = __dadd_rn(st->b[0], __dmul_rn(f, st->bstep));
 }
 
-// |g| and rms = |g| / sqrt(n+1) of a gradient in one pass.  The reference
-// scales by max|g| first (vector_operations.hpp:227-264); here the squares are
-// summed in three ranges whose scaling (a power of two, exact) keeps them
-// within FP64, after J. L. Blue ("A portable Fortran program to find the
-// Euclidean norm of a vector", ACM TOMS 4(1), 1978): the exponent picks the
-// range, one fused multiply-add per element.  n = 20,000: 8.0 us, where the
-// maximum (5.5 us) and the scaled sum (6.9 us) were two kernels.
+// |g| and rms = |g| / sqrt(n+1) of a gradient in one pass (norm_add).
+// n = 20,000: 8.0 us, where the maximum (5.5 us) and the scaled sum (6.9 us)
+// were two kernels.
 __global__ void __launch_bounds__(kVecThreads) k_gnorm(const double* __restrict__ G, VecArgs a, int accepted) {
   LbState* st = a.st;
-  const double up = 0x1p+600, down = 0x1p-600;
-  double v[3] = {0.0, 0.0, 0.0};  // sums of squares: tiny (scaled up), ordinary, huge (scaled down)
-  VEC_LOOP(j, a.n1) {
-    const double g = G[j];
-    const int ex = (__double2hiint(g) >> 20) & 0x7ff;  // biased exponent
-    if (ex >= 1023 - 480 && ex <= 1023 + 480) v[1] = fma(g, g, v[1]);
-    else if (ex < 1023 - 480) v[0] = fma(g * up, g * up, v[0]);
-    else if (ex < 0x7ff) v[2] = fma(g * down, g * down, v[2]);
-    else v[1] += g - g;  // infinities and NaN: the scaled norm is NaN
-  }
+  double v[3] = {0.0, 0.0, 0.0};
+  VEC_LOOP(j, a.n1) norm_add(v[0], v[1], v[2], G[j]);
   const bool mx[3] = {false, false, false};
   grid_reduce<3>(v, mx, a.part, a.ticket, [&](double* t) {
-    double nrm;
-    if (t[2] > 0.0) nrm = sqrt(t[2] + t[1] * down * down) * up;
-    else if (t[1] > 0.0 || t[1] != t[1]) nrm = sqrt(t[1] + t[0] * down * down);
-    else nrm = sqrt(t[0]) * down;
-    if (t[1] != t[1]) nrm = t[1];
+    const double nrm = norm_of(t[0], t[1], t[2]);
     st->gnorm_t = nrm;
     st->rms_t = nrm / sqrt((double)a.n1);
     a.host[0] = st->eval[0];
