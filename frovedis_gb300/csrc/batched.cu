@@ -41,7 +41,7 @@
 #include <cmath>
 #include <vector>
 
-#include "fvg_internal.cuh"
+#include "device_common.cuh"
 
 namespace fvg {
 
@@ -53,10 +53,10 @@ constexpr int kBMaxTrials = 10;  // of one line search
 struct ColState {
   double rho[kBMaxHist], yy[kBMaxHist], al[kBMaxHist], beta[kBMaxHist];
   double factor[12];
-  double dot_gs, smax, stepsize, flip, bstep;
+  double dot_gs, stepsize, flip, bstep;
   double loss;                  // accepted loss
-  double gmax, gnorm, rms;      // of the accepted gradient
-  double gmax_t, gnorm_t, rms_t;  // of the last evaluated gradient
+  double gnorm, rms;      // of the accepted gradient
+  double gnorm_t, rms_t;  // of the last evaluated gradient
   double lambda;
   double rh[4];                 // gradient rms after the last four iterations
   int nrh;
@@ -98,8 +98,8 @@ struct BArgs {
   int k, ld, kp, rpb, h;
   const i64* doff;   // [nd+1] first vector row of each dataset
   i64 plane;         // elements of one vector (all datasets)
-  double* part;      // [nd][grid][k][NV]
-  unsigned* ticket;  // [nd]
+  double* part;      // [nd][grid + groups][k][NV]
+  unsigned* ticket;  // [nd][1 + groups]
   ColState* st;      // [nd][ld]
   const int* ctl;
   int gate;          // control word gating the launch (< 0: none)
@@ -134,14 +134,18 @@ __device__ __forceinline__ void build_masks(const ColState* st, int nd, int ld, 
 }
 
 // Fixed-order reduction of NV values per column; fin(j, totals) runs once
-// per column in the dataset's last CTA.
-template <int NV, class Fin>
-__device__ __forceinline__ void col_reduce(double (&v)[NV], const bool (&is_max)[NV], const BArgs& a, Fin fin) {
-  __shared__ double sm[NV][kBT];
-  __shared__ bool last;
-  const int j = threadIdx.x % a.kp, rr = threadIdx.x / a.kp;
-  double* part = a.part + (i64)blockIdx.y * gridDim.x * a.k * NV;
-  unsigned* ticket = a.ticket + blockIdx.y;
+// per column in the dataset's last CTA.  The CTAs' partial sums are combined
+// in two levels, kColGroup neighbouring CTAs and then the groups, each by the
+// last of its CTAs to arrive: one level over 608 CTAs was a chain of 19
+// batches of loads in one CTA, 20 of the 25 to 45 us of a kernel on a plane
+// of 20 000 rows x 64 models.
+constexpr int kColGroup = 32;
+
+// v[] of the CTA's rows -> sm[q][threadIdx.x] of the threads with rr == 0
+template <int NV>
+__device__ __forceinline__ void col_fold(const double (&v)[NV], const bool (&is_max)[NV], const BArgs& a, int rr,
+                                         double (&sm)[NV][kBT]) {
+  __syncthreads();
 #pragma unroll
   for (int q = 0; q < NV; q++) sm[q][threadIdx.x] = v[q];
   __syncthreads();
@@ -154,60 +158,79 @@ __device__ __forceinline__ void col_reduce(double (&v)[NV], const bool (&is_max)
       }
     __syncthreads();
   }
-  if (rr == 0 && j < a.k)
-#pragma unroll
-    for (int q = 0; q < NV; q++) part[((i64)blockIdx.x * a.k + j) * NV + q] = sm[q][threadIdx.x];
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = (atomicAdd(ticket, 1u) == gridDim.x - 1);
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  double t[NV];
+}
+
+// `cnt` partials from `part`, in order; eight loads issued before they are
+// combined
+template <int NV>
+__device__ __forceinline__ void col_gather(double (&t)[NV], const bool (&is_max)[NV], const BArgs& a, int rr, int j,
+                                           const double* part, int cnt) {
 #pragma unroll
   for (int q = 0; q < NV; q++) t[q] = 0.0;
-  if (j < a.k) {
-    // the CTAs' partials in CTA order; eight loads issued before they are
-    // combined (same order as one at a time)
-    i64 b = rr;
-    for (; b + 7 * a.rpb < gridDim.x; b += 8 * a.rpb) {
-      double x[8][NV];
+  if (j >= a.k) return;
+  constexpr int U = NV > 2 ? 4 : 8;
+  for (int b = rr; b < cnt; b += U * a.rpb) {
+    double x[U][NV];
 #pragma unroll
-      for (int u = 0; u < 8; u++)
+    for (int u = 0; u < U; u++)
 #pragma unroll
-        for (int q = 0; q < NV; q++) x[u][q] = __ldcg(&part[((b + u * a.rpb) * a.k + j) * NV + q]);
+      for (int q = 0; q < NV; q++)
+        x[u][q] = b + u * a.rpb < cnt ? __ldcg(&part[((i64)(b + u * a.rpb) * a.k + j) * NV + q]) : 0.0;
 #pragma unroll
-      for (int u = 0; u < 8; u++)
+    for (int u = 0; u < U; u++)
 #pragma unroll
-        for (int q = 0; q < NV; q++) t[q] = is_max[q] ? fmax(t[q], x[u][q]) : t[q] + x[u][q];
-    }
-    for (; b < gridDim.x; b += a.rpb)
-#pragma unroll
-      for (int q = 0; q < NV; q++) {
-        const double x = __ldcg(&part[(b * a.k + j) * NV + q]);
-        t[q] = is_max[q] ? fmax(t[q], x) : t[q] + x;
-      }
+      for (int q = 0; q < NV; q++) t[q] = is_max[q] ? fmax(t[q], x[u][q]) : t[q] + x[u][q];
   }
-#pragma unroll
-  for (int q = 0; q < NV; q++) sm[q][threadIdx.x] = t[q];
+}
+
+// true in the last of `cnt` CTAs to come here; what the others wrote before
+// is then visible to all its threads
+__device__ __forceinline__ bool col_last(unsigned* ticket, int cnt) {
+  __shared__ bool last;
+  __threadfence();
   __syncthreads();
-  for (int s = a.rpb / 2; s > 0; s >>= 1) {
-    if (rr < s)
-#pragma unroll
-      for (int q = 0; q < NV; q++) {
-        const double o = sm[q][threadIdx.x + s * a.kp];
-        sm[q][threadIdx.x] = is_max[q] ? fmax(sm[q][threadIdx.x], o) : sm[q][threadIdx.x] + o;
-      }
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(ticket, 1u) == (unsigned)cnt - 1;
+    if (last) *ticket = 0u;
   }
-  if (rr == 0 && j < a.k) {
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+
+template <int NV, class Fin>
+__device__ __forceinline__ void col_reduce(double (&v)[NV], const bool (&is_max)[NV], const BArgs& a, Fin fin) {
+  __shared__ double sm[NV][kBT];
+  const int j = threadIdx.x % a.kp, rr = threadIdx.x / a.kp;
+  const bool mine = rr == 0 && j < a.k;
+  const int grid = (int)gridDim.x, ng = (grid + kColGroup - 1) / kColGroup, grp = (int)blockIdx.x / kColGroup;
+  // per dataset: a slot per CTA, then one per group
+  double* part = a.part + (i64)blockIdx.y * (grid + ng) * a.k * NV;
+  double* gpart = part + (i64)grid * a.k * NV;
+  unsigned* ticket = a.ticket + (i64)blockIdx.y * (ng + 1);
+  auto put = [&](double* to) {
+    if (mine)
+#pragma unroll
+      for (int q = 0; q < NV; q++) to[(i64)j * NV + q] = sm[q][threadIdx.x];
+  };
+  col_fold<NV>(v, is_max, a, rr, sm);
+  put(part + (i64)blockIdx.x * a.k * NV);
+  const int b0 = grp * kColGroup, cnt = min(kColGroup, grid - b0);
+  if (!col_last(ticket + 1 + grp, cnt)) return;
+  col_gather<NV>(v, is_max, a, rr, j, part + (i64)b0 * a.k * NV, cnt);
+  col_fold<NV>(v, is_max, a, rr, sm);
+  if (ng > 1) {
+    put(gpart + (i64)grp * a.k * NV);
+    if (!col_last(ticket, ng)) return;
+    col_gather<NV>(v, is_max, a, rr, j, gpart, ng);
+    col_fold<NV>(v, is_max, a, rr, sm);
+  }
+  if (mine) {
     double tot[NV];
 #pragma unroll
     for (int q = 0; q < NV; q++) tot[q] = sm[q][threadIdx.x];
     fin(j, tot);
   }
-  __syncthreads();
-  if (threadIdx.x == 0) *ticket = 0u;
 }
 
 // thread -> (column j, first row r0 of dataset blockIdx.y); rows advance by
@@ -334,7 +357,8 @@ __global__ void __launch_bounds__(kBT, 4) kb_up(int i, int kh, int rear, const d
   });
 }
 
-// step = -z, or the no-history step (as in k_direction)
+// step = -z, or the no-history step (as in k_direction); its norm, the uphill
+// flip and the factors of the trials
 __global__ void __launch_bounds__(kBT, 4) kb_step(int kh, int rear, const double* __restrict__ G,
                                                const double* __restrict__ Z, double* __restrict__ STEP,
                                                const double* __restrict__ S, BArgs a) {
@@ -352,7 +376,7 @@ __global__ void __launch_bounds__(kBT, 4) kb_step(int kh, int rear, const double
       f = s.al[kh - 1] - s.beta[kh - 1];
     }
   }
-  double v[2] = {0.0, 0.0};
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
   if (act)
     rows_grouped<kRowGroup>(r0, rstep, n1,
                             [&](i64 r) {
@@ -364,43 +388,21 @@ __global__ void __launch_bounds__(kBT, 4) kb_step(int kh, int rear, const double
                               const double st = -z;
                               STEP[e0 + r * ld] = st;
                               v[0] += x.a * st;
-                              v[1] = fmax(v[1], fabs(st));
+                              norm_add(v[1], v[2], v[3], st);
                             });
-  const bool mx[2] = {false, true};
-  col_reduce<2>(v, mx, a, [&](int c2, double* t) {
+  const bool mx[4] = {false, false, false, false};
+  col_reduce<4>(v, mx, a, [&](int c2, double* t) {
     ColState& s = a.st[ds * ld + c2];
     if (!s.active) return;
+    const double ss = norm_of(t[1], t[2], t[3]);
     s.dot_gs = t[0];
-    s.smax = t[1];
-  });
-}
-
-// max-scaled step norm, uphill flip, factors of the 10 trials (as in k_direction)
-__global__ void __launch_bounds__(kBT, 4) kb_step_norm(const double* __restrict__ STEP, BArgs a) {
-  BCOL;
-  const bool act = on && a.st[mj].active;
-  const double mxv = act ? a.st[mj].smax : 0.0;
-  const double inv = mxv == 0 ? 0.0 : 1.0 / mxv;
-  double v[1] = {0.0};
-  if (act)
-    rows_grouped<kRowGroup>(r0, rstep, n1, [&](i64 r) { return STEP[e0 + r * ld]; },
-                            [&](i64, double x) {
-                              const double t = x * inv;
-                              v[0] += t * t;
-                            });
-  const bool mx[1] = {false};
-  col_reduce<1>(v, mx, a, [&](int c, double* t) {
-    ColState& s = a.st[ds * ld + c];
-    if (!s.active) return;
-    const double m = s.smax;
-    const double ss = (m == 0) ? 0.0 : sqrt(t[0]) * m;
     s.stepsize = ss;
-    s.flip = (s.dot_gs > 0) ? -1.0 : 1.0;
+    s.flip = (t[0] > 0) ? -1.0 : 1.0;
     double fac = 1.0;
     if (fac * ss > 1e20) fac = 1e20 / ss;
     s.factor[1] = fac;
     for (int q = 2; q <= 10; q++) s.factor[q] = s.factor[q - 1] / 10.0;
-    s.bstep = STEP[(rb + n1 - 1) * ld + c] * s.flip;
+    s.bstep = __ldcg(&STEP[(rb + n1 - 1) * ld + c2]) * s.flip;
   });
 }
 
@@ -432,50 +434,29 @@ __global__ void __launch_bounds__(kBT, 4) kb_trial(const double* __restrict__ W,
   if (r0 == 0) B1[mj] = __dadd_rn(B0[mj], __dmul_rn(f, s.bstep));
 }
 
+// gradient norm and rms in one pass (norm_add); `accepted`: the evaluation is
+// of the accepted model (the initial one, or the re-evaluation after a
+// precision switch)
 // (a.mask: only the models evaluated last; the others keep their norms)
-__global__ void __launch_bounds__(kBT, 4) kb_gmax(const double* __restrict__ G, BArgs a) {
-  BCOL;
-  if (!dataset_on(a, ds)) return;
-  const bool use = on && model_on(a, ds, j);
-  double v[1] = {0.0};
-  if (use)
-    rows_grouped<kRowGroup>(r0, rstep, n1, [&](i64 r) { return G[e0 + r * ld]; },
-                            [&](i64, double x) { v[0] = fmax(v[0], fabs(x)); });
-  const bool mx[1] = {true};
-  col_reduce<1>(v, mx, a, [&](int c, double* t) {
-    if (model_on(a, ds, c)) a.st[ds * ld + c].gmax_t = t[0];
-  });
-}
-
-// gradient norm and rms; `accepted`: the evaluation is of the accepted
-// model (the initial one, or the re-evaluation after a precision switch)
 __global__ void __launch_bounds__(kBT, 4) kb_gnorm(const double* __restrict__ G, const double* __restrict__ EV,
                                                 int accepted, BArgs a) {
   BCOL;
   if (!dataset_on(a, ds)) return;
   const bool use = on && model_on(a, ds, j);
-  const double mxv = use ? a.st[mj].gmax_t : 0.0;
-  const double inv = mxv == 0 ? 0.0 : 1.0 / mxv;
-  double v[1] = {0.0};
+  double v[3] = {0.0, 0.0, 0.0};
   if (use)
     rows_grouped<kRowGroup>(r0, rstep, n1, [&](i64 r) { return G[e0 + r * ld]; },
-                            [&](i64, double x) {
-                              const double t = x * inv;
-                              v[0] += t * t;
-                            });
-  const bool mx[1] = {false};
-  col_reduce<1>(v, mx, a, [&](int c, double* t) {
+                            [&](i64, double x) { norm_add(v[0], v[1], v[2], x); });
+  const bool mx[3] = {false, false, false};
+  col_reduce<3>(v, mx, a, [&](int c, double* t) {
     if (!model_on(a, ds, c)) return;
     const i64 mc = ds * ld + c;
     ColState& s = a.st[mc];
-    const double m = s.gmax_t;
-    const double nrm = (m == 0) ? 0.0 : sqrt(t[0]) * m;
-    s.gnorm_t = nrm;
-    s.rms_t = nrm / sqrt((double)n1);
+    s.gnorm_t = norm_of(t[0], t[1], t[2]);
+    s.rms_t = s.gnorm_t / sqrt((double)n1);
     if (accepted && s.active) {
-      s.gnorm = nrm;
+      s.gnorm = s.gnorm_t;
       s.rms = s.rms_t;
-      s.gmax = m;
       s.loss = EV[2 * mc];
     }
   });
@@ -1015,8 +996,10 @@ void lbfgs_multi_train(fvg_ctx* c, const std::vector<fvg_matrix*>& mats, const s
   const int vgx = (int)std::max<i64>(
       1, std::min<i64>((maxn1 + rpb - 1) / rpb, std::max<i64>(1, 4 * (i64)c->num_sms / nd)));
   const dim3 vgrid((unsigned)vgx, (unsigned)nd);
-  part.alloc(sizeof(double) * 2 * (size_t)vgx * kk * nd, s);
-  ctl.alloc(sizeof(int) * C_NCTL + sizeof(unsigned) * (size_t)nd, s);
+  const int vgroups = (vgx + kColGroup - 1) / kColGroup;
+  part.alloc(sizeof(double) * 4 * (size_t)(vgx + vgroups) * kk * nd, s);
+  const size_t tickets = sizeof(unsigned) * (size_t)nd * (vgroups + 1);
+  ctl.alloc(sizeof(int) * C_NCTL + tickets, s);
   dof.alloc(sizeof(i64) * (nd + 1), s);
   const int nwd = (ld + 63) / 64;
   MSK.alloc(sizeof(unsigned long long) * 2 * (size_t)nd * nwd, s);
@@ -1061,7 +1044,7 @@ void lbfgs_multi_train(fvg_ctx* c, const std::vector<fvg_matrix*>& mats, const s
     FVG_CUDA(cudaMemcpyAsync(ST.p, cs.data(), sizeof(ColState) * nm, cudaMemcpyHostToDevice, s));
     FVG_CUDA(cudaMemcpyAsync(B0, bb.data(), sizeof(double) * 2 * nm, cudaMemcpyHostToDevice, s));
     FVG_CUDA(cudaMemcpyAsync(ctl_i, hc.data(), sizeof(int) * C_NCTL, cudaMemcpyHostToDevice, s));
-    FVG_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned) * nd, s));
+    FVG_CUDA(cudaMemsetAsync(ticket, 0, tickets, s));
     FVG_CUDA(cudaMemcpyAsync(dof.p, doff.data(), sizeof(i64) * (nd + 1), cudaMemcpyHostToDevice, s));
     FVG_CUDA(cudaStreamSynchronize(s));  // the host vectors above go out of scope
   }
@@ -1085,10 +1068,9 @@ void lbfgs_multi_train(fvg_ctx* c, const std::vector<fvg_matrix*>& mats, const s
   };
   auto norms = [&](const double* g, int accepted, int gate, const unsigned long long* mask) {
     ProfScope ps(c, P_LBFGS);
-    kb_gmax<<<vgrid, kBT, 0, s>>>(g, gated(gate, mask));
     kb_gnorm<<<vgrid, kBT, 0, s>>>(g, EV.as<double>(), accepted, gated(gate, mask));
     check_launch("kb_gnorm");
-    count_launch(c, 2);
+    count_launch(c);
   };
   const int* one = ctl_i + C_ONE;
 
@@ -1116,10 +1098,9 @@ void lbfgs_multi_train(fvg_ctx* c, const std::vector<fvg_matrix*>& mats, const s
                                       gated(C_ACTIVE));
         kb_step<<<vgrid, kBT, 0, s>>>(kh, rear, G.as<double>(), Z.as<double>(), STEP.as<double>(), S.as<double>(),
                                       gated(C_ACTIVE));
-        kb_step_norm<<<vgrid, kBT, 0, s>>>(STEP.as<double>(), gated(C_ACTIVE));
         kb_begin_search<<<1, kBT, 0, s>>>(nd, ld, nwd, a.st, ctl_i, smask, tl);
         check_launch("batched two-loop");
-        count_launch(c, 2 * kh + 3);
+        count_launch(c, 2 * kh + 2);
       }
       auto trial = [&]() {
         const int64_t l0 = c->launches;
