@@ -414,6 +414,23 @@ template <class AT, int QN> struct SegWalk {
 // Long rows (a warp each): add the pieces' partials in piece order, apply the
 // epilogue; then (logistic) the last CTA reduces all loss / bias partials per
 // column in a fixed order.
+//
+// The hot rows of a transposed matrix have thousands of pieces, and the
+// latency of their loads bounds the kernel: the row's warp alone keeps 32 in
+// flight.  For a row of more than kFinShare pieces the whole CTA copies them
+// through a ring of tiles in shared memory, from which the row's warp adds
+// them in the same order; the rows are dealt across the CTAs, so neighbouring
+// hot rows meet different ones.  2,000 pieces of 32 columns: 34 us, 95 us
+// by one warp.
+constexpr int kFinShare = 64;
+constexpr int kFinTile = 8192;  // bytes
+constexpr int kFinTiles = 3;
+
+__device__ __forceinline__ void copy16_async(void* to, const void* from) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from)
+               : "memory");
+}
+
 template <class AT, class YT, int EPI, int CPL, bool VEC>
 __global__ void __launch_bounds__(kThreads) k_spmm_fin(const SpmmFin f) {
   using Sum = typename SumOf<AT>::type;
@@ -440,25 +457,17 @@ __global__ void __launch_bounds__(kThreads) k_spmm_fin(const SpmmFin f) {
   const i64 gw = (i64)blockIdx.x * (kThreads / 32) + wib, nw = (i64)gridDim.x * (kThreads / 32);
   SegWalk<AT, CPL> sw(p, seg ? f.seg_fpart : nullptr, gw, nw, NC);
   unsigned long long mw = mask_of(p, 0);
-  for (i64 i = gw; i < f.nlong; i += nw) {
-    const i64 q0 = f.long_piece0[i], q1 = f.long_piece0[i + 1];
-    const i32 row = f.long_rows[i];
-    if (track && sw.to_row(p, row, cols, ls, bs)) {
-      if (EPI == EPI_LOGREG) load_bias(p.bias + sw.d * p.ldb);
-      mw = mask_of(p, sw.d);
-    }
-    if (mw == 0) continue;
-    AT a[CPL];
-#pragma unroll
-    for (int q = 0; q < CPL; q++) a[q] = 0;
-    // added one after the other, loaded kBatch at a time: the hot rows of a
-    // transposed matrix have thousands of pieces, and the chain of their loads
-    // bounds the kernel (2,000 pieces of 32 columns: 95 us, 214 us one by one)
+  constexpr int kWarps = kThreads / 32;
+  __shared__ i32 s_piece[kWarps][2];  // the pieces of each warp's row, if shared
+  __shared__ __align__(16) AT s_tile[kFinTiles][kFinTile / sizeof(AT)];
+  constexpr int kPer = kFinTile / (int)sizeof(AT) / NC;  // pieces of a tile
+  // a row's pieces [q0, q1) one after the other, loaded kBatch at a time
+  auto add_pieces = [&](i32 q0, i32 q1, AT (&a)[CPL]) {
     constexpr int kBatch = 32 / CPL;
-    i64 pc = q0;
+    i32 pc = q0;
     for (; pc + kBatch <= q1; pc += kBatch) {
       AT v[kBatch][CPL];
-      const AT* part = (const AT*)p.partials + pc * NC;
+      const AT* part = (const AT*)p.partials + (i64)pc * NC;
 #pragma unroll
       for (int u = 0; u < kBatch; u++)
 #pragma unroll
@@ -469,11 +478,66 @@ __global__ void __launch_bounds__(kThreads) k_spmm_fin(const SpmmFin f) {
         for (int q = 0; q < CPL; q++) a[q] += v[u][q];
     }
     for (; pc < q1; pc++) {
-      const AT* part = (const AT*)p.partials + pc * NC;
+      const AT* part = (const AT*)p.partials + (i64)pc * NC;
 #pragma unroll
       for (int q = 0; q < CPL; q++) a[q] += __ldcg(part + colof<VEC, CPL>(lane, q));
     }
-    spmm_epi<AT, YT, EPI, CPL, VEC>(p, row, a, b, lane, ls, bs, mw);
+  };
+  for (i64 i0 = 0; i0 < f.nlong; i0 += nw) {
+    const i64 i = i0 + (i64)wib * gridDim.x + blockIdx.x;
+    i32 q0 = 0, q1 = 0, row = 0;
+    bool live = i < f.nlong;
+    if (live) {
+      q0 = f.long_piece0[i];
+      q1 = f.long_piece0[i + 1];
+      row = f.long_rows[i];
+      if (track && sw.to_row(p, row, cols, ls, bs)) {
+        if (EPI == EPI_LOGREG) load_bias(p.bias + sw.d * p.ldb);
+        mw = mask_of(p, sw.d);
+      }
+      live = mw != 0;
+    }
+    const bool shared = live && q1 - q0 > kFinShare;
+    if (lane == 0) {
+      s_piece[wib][0] = q0;
+      s_piece[wib][1] = shared ? q1 : q0;
+    }
+    AT a[CPL];
+#pragma unroll
+    for (int q = 0; q < CPL; q++) a[q] = 0;
+    if (live && !shared) add_pieces(q0, q1, a);
+    __syncthreads();
+    for (int w = 0; w < kWarps; w++) {
+      const i32 b0 = s_piece[w][0], n = s_piece[w][1] - b0;
+      if (n == 0) continue;
+      const i32 nt = (n + kPer - 1) / kPer;
+      auto fetch = [&](i32 t) {
+        if (t < nt) {
+          const i32 bytes = min(n - t * kPer, kPer) * NC * (int)sizeof(AT);
+          const char* from = (const char*)p.partials + (i64)(b0 + t * kPer) * NC * sizeof(AT);
+          for (i32 o = threadIdx.x * 16; o < bytes; o += kThreads * 16)
+            copy16_async((char*)s_tile[t % kFinTiles] + o, from + o);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      };
+      for (i32 t = 0; t < kFinTiles - 1; t++) fetch(t);
+      for (i32 t = 0; t < nt; t++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kFinTiles - 2) : "memory");
+        __syncthreads();  // tile t is there, tile t - 1 is read
+        fetch(t + kFinTiles - 1);
+        if (w == wib) {
+          const AT* tile = s_tile[t % kFinTiles];
+          const i32 cnt = min(n - t * kPer, kPer);
+#pragma unroll 8
+          for (i32 u = 0; u < cnt; u++)
+#pragma unroll
+            for (int q = 0; q < CPL; q++) a[q] += tile[u * NC + colof<VEC, CPL>(lane, q)];
+        }
+      }
+      __syncthreads();
+    }
+    if (live) spmm_epi<AT, YT, EPI, CPL, VEC>(p, row, a, b, lane, ls, bs, mw);
+    __syncthreads();  // s_piece is written by the next round
   }
   if (track && !seg) return;
   if (seg && p.nseg > 1) {
@@ -897,7 +961,7 @@ static int spmm_grid(fvg_ctx* c) {
 }
 
 static int spmm_fin_grid(fvg_ctx* c, i64 nlong) {
-  return (int)std::max<i64>(1, std::min<i64>((nlong + 7) / 8, 2 * c->num_sms));
+  return (int)std::max<i64>(1, std::min<i64>(nlong, 2 * c->num_sms));  // a CTA each while they last: rows are shared by its warps
 }
 
 // Scratch of one block pass (sized for 128 columns): ticket, per-CTA
