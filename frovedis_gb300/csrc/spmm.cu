@@ -645,22 +645,75 @@ __device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(v), "l"(x));
 }
 
-// A chunk of 32 entries staged for the warp: the row offset of the gathered
-// row of X (column id x stride) and the value, zero past the chunk's end.
-template <class AT> struct alignas(16) StageE {
-  long long off;
+// A chunk of 32 entries staged for the warp: the column (the row of X to
+// gather) and the value, both zero past the chunk's end.  8 bytes an entry
+// with FP32 values: the SM's shared-memory / L1 data path carries the gathers
+// (8 passes a step of 32 lanes x 32 bytes) and two thirds of it were busy; a
+// staged row offset (16 bytes) took 8 passes of it to write and 2 a step to
+// read.
+template <class AT> struct alignas(2 * sizeof(AT)) StageE {
+  i32 col;
   AT v;
 };
 
-template <class VT, class XT, class AT, int G>
+// The largest of the lanes' values (a NaN is ignored, as fmax does).
+__device__ __forceinline__ float warp_max(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ double warp_max(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+
+// The entries a warp takes next: lane L holds entry pos + L, loaded while the
+// chunk before is multiplied.  A chunk starts where the one before ended,
+// whatever row it belongs to, so 32 entries are fetched without a look at the
+// row bounds; at an item's end the next item's first ones.  pos tells a chunk
+// that comes after skipped rows that it has to load for itself.
+template <class AT> struct EntryPre {
+  i32 pos = -1;
+  i32 col = 0;
+  AT v = 0;
+};
+template <class VT, class AT>
+__device__ __forceinline__ void pre_fetch(const SpmmK& p, EntryPre<AT>& pre, i32 e, i32 end, int lane) {
+  pre.pos = e < end ? e : -1;  // an item without entries leaves nothing for one that starts at the same place
+  if (e + lane < end) {
+    pre.col = __ldcs(p.idx + e + lane);
+    pre.v = ld_val<VT, AT>((const VT*)p.val + e + lane);
+  }
+}
+
+// Entries [e0, e1) of one row (or piece) of `item`, `next` the item the warp
+// takes after it.  Group grp of the warp takes entries grp, grp + G, ... of
+// each chunk of 32.  FP32: the gathers of kStep steps are issued together, in
+// the last chunk under a predicate: a loop over the steps left it to the
+// compiler how many were under way, and the last chunk's went one by one,
+// padding included.  1M rows x 100 entries, 32 columns, BF16 values (with the
+// 8-byte stage): softmax pass 908 -> 780 us, transposed pass 722 -> 702 us.
+//
+// PRE (entries fetched a chunk ahead): plain products with FP32 values up to
+// 64 columns (300 000 rows x 50 entries, 64 columns: 217 us without, 192 with;
+// 128 columns of 100 000 rows: 151 without, 176 with) and FP64 ones (100 000
+// rows x 30 entries, 32 columns: 263 without, 255 with).  BF16 values are
+// faster without (60 000 rows x 20 entries, 64 columns: 55 without, 58 with),
+// and the epilogues' registers and the FP64 results of the transposed pass
+// leave no room for it (64 a thread): 796 -> 832, 702 -> 797 us.
+template <class VT, class XT, class AT, int G, bool PRE>
 __device__ __forceinline__ void row_dot_g(const SpmmK& p, i32 e0, i32 e1, int lane, AT (&a)[GLay<XT, G>::CPL],
-                                          StageE<AT>* st, bool lane_on = true) {
+                                          StageE<AT>* st, bool lane_on, EntryPre<AT>& pre, const Item& item,
+                                          const Item& next) {
   using L = GLay<XT, G>;
   constexpr int CPL = L::CPL;
   constexpr bool PACK = sizeof(XT) == 4 && sizeof(AT) == 4;
+  constexpr int kStep = PRE ? 2 : 4;
+  static_assert(32 / G >= kStep, "whole batches of steps in a chunk");
   const int sub = lane % L::LPR, grp = lane / L::LPR;
-  const XT* X = (const XT*)p.X + sub * CPL;
-  const int ldx = (int)p.ldx;  // a row stride of X fits 32 bits
+  const char* X = (const char*)((const XT*)p.X + sub * CPL);
+  const unsigned ldx = (unsigned)p.ldx * sizeof(XT);  // row stride of X in bytes: launch_grouped keeps it within 32 bits
   const VT* val = (const VT*)p.val;
   const bool mine = lane_on && sub * CPL < p.kb;
   unsigned long long acc[CPL / 2];  // packed FP32 pairs
@@ -670,44 +723,75 @@ __device__ __forceinline__ void row_dot_g(const SpmmK& p, i32 e0, i32 e1, int la
   for (int q = 0; q < CPL / 2; q++) acc[q] = 0ull;
   for (i32 e = e0; e < e1; e += 32) {
     const int cnt = min(32, e1 - e);
-    // stage the chunk (offsets computed once per entry); the padding
-    // entries (offset 0, value 0) round the chunk up to whole steps
     StageE<AT> se;
-    se.off = 0;
+    se.col = 0;
     se.v = 0;
-    if (lane < cnt) {
-      se.off = (long long)__ldcs(p.idx + e + lane) * ldx;
+    if constexpr (PRE) {
+      if (pre.pos != e) pre_fetch<VT, AT>(p, pre, e, item.e1, lane);
+      if (lane < cnt) {
+        se.col = pre.col;
+        se.v = pre.v;
+      }
+    } else if (lane < cnt) {
+      se.col = __ldcs(p.idx + e + lane);
       se.v = ld_val<VT, AT>(val + e + lane);
     }
     __syncwarp();
     st[lane] = se;
+    if constexpr (PRE) {
+      if (e + cnt < item.e1) pre_fetch<VT, AT>(p, pre, e + cnt, item.e1, lane);
+      else pre_fetch<VT, AT>(p, pre, next.e0, next.e1, lane);
+    }
     __syncwarp();
-    // group grp takes entries grp, grp + G, ...; lanes whose columns are
-    // not computed skip the chunk
-    if (mine) {
+    // lanes whose columns are not computed skip the chunk
+    if (!mine) continue;
+    if constexpr (!PACK) {
       const int steps = (cnt + G - 1) / G;
 #pragma unroll 4
       for (int k = 0; k < steps; k++) {
         const StageE<AT> t = st[k * G + grp];
-        const XT* xp = X + t.off;
-        if constexpr (PACK) {
-          // the lane's 8 FP32 columns in one 32-byte load, as 4 packed pairs
-          static_assert(CPL == 8, "one 32-byte load a lane");
-          unsigned long long x0, x1, x2, x3;
-          asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];"
-              : "=l"(x0), "=l"(x1), "=l"(x2), "=l"(x3)
-              : "l"(xp));
-          const unsigned long long vv = pack2((float)t.v, (float)t.v);
-          fma2(acc[0], vv, x0);
-          fma2(acc[1], vv, x1);
-          fma2(acc[2], vv, x2);
-          fma2(acc[3], vv, x3);
-        } else {
-          XT x[CPL];
-          VecLd<XT, CPL>::ld(xp, x);
+        XT x[CPL];
+        VecLd<XT, CPL>::ld((const XT*)(X + (unsigned long long)(unsigned)t.col * ldx), x);
 #pragma unroll
-          for (int q = 0; q < CPL; q++) a[q] += t.v * (AT)x[q];
+        for (int q = 0; q < CPL; q++) a[q] += t.v * (AT)x[q];
+      }
+    } else {
+      // the lane's 8 FP32 columns in one 32-byte load, as 4 packed pairs
+      static_assert(!PACK || CPL == 8, "one 32-byte load a lane");
+      auto steps = [&](int k0, auto full) {
+        StageE<AT> t[kStep];
+        unsigned long long x[kStep][4];
+#pragma unroll
+        for (int u = 0; u < kStep; u++) t[u] = st[(k0 + u) * G + grp];
+#pragma unroll
+        for (int u = 0; u < kStep; u++) {
+          const char* row = X + (unsigned long long)(unsigned)t[u].col * ldx;
+          if constexpr (decltype(full)::value) {
+            asm volatile("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];"
+                         : "=l"(x[u][0]), "=l"(x[u][1]), "=l"(x[u][2]), "=l"(x[u][3])
+                         : "l"(row));
+          } else {
+            const int on = (k0 + u) * G + grp < cnt;
+            asm volatile(
+                "{ .reg .pred p; setp.ne.s32 p, %5, 0;\n"
+                " mov.b64 %0, 0; mov.b64 %1, 0; mov.b64 %2, 0; mov.b64 %3, 0;\n"
+                " @p ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4]; }"
+                : "=&l"(x[u][0]), "=&l"(x[u][1]), "=&l"(x[u][2]), "=&l"(x[u][3])
+                : "l"(row), "r"(on));
+          }
         }
+#pragma unroll
+        for (int u = 0; u < kStep; u++) {
+          const unsigned long long vv = pack2((float)t[u].v, (float)t[u].v);
+#pragma unroll
+          for (int q = 0; q < 4; q++) fma2(acc[q], vv, x[u][q]);
+        }
+      };
+      if (cnt == 32) {
+#pragma unroll
+        for (int k = 0; k < 32 / G; k += kStep) steps(k, std::true_type());
+      } else {
+        for (int k = 0; k * G < cnt; k += kStep) steps(k, std::false_type());
       }
     }
   }
@@ -734,8 +818,15 @@ __device__ __forceinline__ void row_dot_g(const SpmmK& p, i32 e0, i32 e1, int la
   }
 }
 
+// CTAs per SM: four (64 registers a thread), three for the transposed pass of
+// the trainings (FP32 arithmetic, FP64 results) from 64 columns on, whose rows
+// of X of 256 bytes and more gain from fewer warps sharing the L1: 107 -> 98
+// us at 200 000 x 20 000, 10M entries, 64 columns (32 columns: 702 -> 780).
+template <class XT, class YT, int EPI, int G>
+constexpr int kGroupedCtas = EPI == EPI_STORE && sizeof(XT) == 4 && sizeof(YT) == 8 && G <= 4 ? 3 : 4;
+
 template <class VT, class XT, class AT, class YT, int EPI, int G>
-__global__ void __launch_bounds__(kThreads, 4) k_spmm_g(const SpmmK p) {
+__global__ void __launch_bounds__(kThreads, kGroupedCtas<XT, YT, EPI, G>) k_spmm_g(const SpmmK p) {
   using L = GLay<XT, G>;
   using Sum = typename SumOf<AT>::type;
   constexpr int CPL = L::CPL, NC = L::NC, QG = L::QG;
@@ -762,8 +853,14 @@ __global__ void __launch_bounds__(kThreads, 4) k_spmm_g(const SpmmK p) {
   __shared__ StageE<AT> stage[kThreads / 32][32];
   unsigned long long mw = mask_of(p, 0);
   AT lab = 0, w = 1;
+  // entries fetched ahead: see row_dot_g
+  constexpr bool PRE = EPI == EPI_STORE && sizeof(YT) == sizeof(AT) && sizeof(VT) == sizeof(AT) && (sizeof(AT) == 8 || G >= 4);
+  EntryPre<AT> pre;
+  Item next{0, 0, 0, 0};
+  if (PRE && gw < p.nitems) next = p.items[gw];
   for (i64 it = gw; it < p.nitems; it += nw) {
-    const Item item = p.items[it];
+    const Item item = PRE ? next : p.items[it];
+    if (PRE) next = it + nw < p.nitems ? p.items[it + nw] : Item{0, 0, 0, 0};
     AT a[CPL];
     // the store epilogue keeps no per-dataset sums, so its items may come in
     // any order (slab-ordered pieces): each item looks its dataset up
@@ -777,7 +874,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_spmm_g(const SpmmK p) {
         mw = mask_of(p, walk.d);
       }
       if (mw == 0) continue;  // the finalize skips the row too
-      row_dot_g<VT, XT, AT, G>(p, item.e0, item.e1, lane, a, stage[wib], cols_on(mw, lsh, CPL));
+      row_dot_g<VT, XT, AT, G, PRE>(p, item.e0, item.e1, lane, a, stage[wib], cols_on(mw, lsh, CPL), pre, item,
+                                    next);
       AT* part = (AT*)p.partials + (i64)(-1 - item.r1) * NC;
 #pragma unroll
       for (int q = 0; q < QG; q++) part[cols[q]] = a[q];
@@ -789,7 +887,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_spmm_g(const SpmmK p) {
         mw = mask_of(p, walk.d);
       }
       if (mw == 0) continue;  // no column of this dataset is computed
-      row_dot_g<VT, XT, AT, G>(p, __ldg(p.off + r), __ldg(p.off + r + 1), lane, a, stage[wib], cols_on(mw, lsh, CPL));
+      row_dot_g<VT, XT, AT, G, PRE>(p, __ldg(p.off + r), __ldg(p.off + r + 1), lane, a, stage[wib], cols_on(mw, lsh, CPL), pre, item,
+                                    next);
       if constexpr (EPI == EPI_STORE) {
         YT* y = (YT*)p.Y + (i64)r * p.ldy;
 #pragma unroll
@@ -835,8 +934,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_spmm_g(const SpmmK p) {
             z[q] = a[q] + b[q];
             if (cols[q] < p.kb) mx = fmax(mx, z[q]);
           }
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+          mx = warp_max(mx);
           AT zy = 0, sum = 0;
 #pragma unroll
           for (int q = 0; q < QG; q++) {
@@ -848,8 +946,9 @@ __global__ void __launch_bounds__(kThreads, 4) k_spmm_g(const SpmmK p) {
           for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
           // cross-entropy -log p[label] = log(sum) - (z_label - max), unweighted
           if (has_label && p.cta_part) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) zy += __shfl_xor_sync(0xffffffffu, zy, o);
+            // the label's lane alone holds a value other than 0
+            const unsigned own = __ballot_sync(0xffffffffu, zy != (AT)0);
+            zy = __shfl_sync(0xffffffffu, zy, own ? __ffs(own) - 1 : 0);
             if (lane == 0) ls[0].add(log_acc<AT>(sum) - zy);
           }
           const AT inv = (AT)1 / sum;
@@ -1106,7 +1205,7 @@ static bool launch_grouped(fvg_ctx* c, DevCRS& a, const Sched& s, int storage, c
   // vector loads: column blocks and strides in whole vectors (the FP32
   // lanes read 8 columns, the FP64 ones 2), 16-byte aligned bases
   constexpr int VW = 16 / (int)sizeof(XT);
-  bool ok = p.kb % VW == 0 && p.ldx % VW == 0 && aligned_to(p.X, 16);
+  bool ok = p.kb % VW == 0 && p.ldx % VW == 0 && aligned_to(p.X, 16) && p.ldx * (i64)sizeof(XT) < (i64)1 << 32;
   if (EPI == EPI_STORE) ok = ok && p.ldy % VW == 0 && aligned_to(p.Y, 16);
   else ok = ok && p.ldr % VW == 0 && aligned_to(p.R, 16);
   if (!ok) return false;
