@@ -157,100 +157,96 @@ __global__ void k_cold_fill(const i32* __restrict__ toff, const i64* __restrict_
   }
 }
 
-// Work items of a CRS, one warp per chunk of `step` rows (at most kPackRows),
+// Work items of a CRS, one CTA per chunk of `step` rows (at most kPackRows),
 // with the CRS schedule's packing rules
 // (tiles of short rows within `tile` entries, kTileRows rows and lane_work
 // products per lane; longer rows in pieces cut at 8-element boundaries).  The
-// greedy packing is sequential from tile to tile, but the rows of one tile
-// are found together: lane L tests whether the tile may reach to row
-// t0 + L (every limit, once passed, stays passed), and the first lane that
-// fails ends it, 32 rows a step.  Pass 0 counts each chunk's items, long rows
-// and pieces; pass 1 writes them at the scanned offsets `base` (chunk-major: a
-// chunk's items, long rows and pieces are contiguous and numbered globally).
-// Bound by the latency of the longest chunk's tile to tile chain (rows of
-// 200-500 entries: 100 tiles and more in 256 rows), so the chunk's offsets are
-// read from shared memory: 44 us a pass over the transposed 25,600 x 20,000
-// minibatches of a Zipf matrix (a thread walking each chunk row by row: 97 us).
-constexpr int kPackThreads = 128;
+// greedy packing is sequential from tile to tile, but where a tile ends
+// depends only on where it starts: thread t finds the end of a tile starting
+// at the chunk's row t (every limit, once passed, stays passed), one thread
+// follows the ends from row 0 and marks the starts met, and the marked rows
+// are counted and written side by side.  Pass 0 counts each chunk's items,
+// long rows and pieces; pass 1 writes them at the scanned offsets `base`
+// (chunk-major: a chunk's items, long rows and pieces are contiguous and
+// numbered globally).
+// Bound by the walk over the starts (up to 256 dependent reads of shared
+// memory): 12.7 us a pass over the transposed 25,600 x 20,000 minibatches of a
+// Zipf matrix; 44 us with the warp searching each tile's end in turn.
+constexpr int kPackThreads = (int)kPackRows;
 __global__ void __launch_bounds__(kPackThreads) k_pack(const i32* __restrict__ off, i64 nrows, i64 step, i64 np, int tile,
                                                     int write, i32* __restrict__ cnt,
                                                     const i32* __restrict__ base, Item* __restrict__ items,
                                                     i32* __restrict__ lrows, i32* __restrict__ lpiece0,
                                                     i32* __restrict__ lfirst, int lane_work) {
-  __shared__ i32 soff[kPackThreads / 32][kPackRows + 1];
-  const int lane = threadIdx.x & 31;
-  i32* so = soff[threadIdx.x >> 5];
-  PWARP_STRIDE(p, np) {
-    const i64 r0 = min(p * step, nrows), r1 = min(r0 + step, nrows);
-    __syncwarp();
-#pragma unroll 8
-    for (int q = lane; q <= (int)(r1 - r0); q += 32) so[q] = __ldg(off + r0 + q);
-    __syncwarp();
-    const i32 bi = write ? base[p] : 0, bl = write ? base[(np + 1) + p] : 0, bp = write ? base[2 * (np + 1) + p] : 0;
-    i32 ni = 0, nl = 0, npc = 0;
-    i64 t0 = r0;
-    while (t0 < r1) {
-      const i32 o0 = so[t0 - r0];
-      int n = 0;       // rows of the tile starting at t0
-      int mx = 0;      // longest of its rows so far
-      i32 o_end = o0;  // the offset where the tile ends
-      i32 ob, oe;      // offsets of this lane's row t0 + n + lane
-      bool lng;        // that row is longer than a tile
-      for (;;) {
-        const i64 r = t0 + n + lane;
-        const bool valid = r < r1;
-        ob = valid ? so[r - r0] : 0;
-        oe = valid ? so[r - r0 + 1] : 0;
-        const int len = oe - ob;
-        lng = len > tile;
-        int m = max(mx, len);  // longest row up to this one
+  constexpr int kWarps = kPackThreads / 32;
+  __shared__ i32 so[kPackThreads + 1];
+  __shared__ short nxt[kPackThreads];
+  __shared__ unsigned char start[kPackThreads];
+  __shared__ i32 wsum[3][kWarps];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  for (i64 p = blockIdx.x; p < np; p += gridDim.x) {
+    const i64 r0 = min(p * step, nrows);
+    const int R = (int)(min(r0 + step, nrows) - r0);  // rows of the chunk
+    __syncthreads();
+    if (t < R) so[t + 1] = __ldg(off + r0 + t + 1);
+    if (t == 0) so[0] = __ldg(off + r0);
+    start[t] = 0;
+    __syncthreads();
+    const i32 ob = t < R ? so[t] : 0, oe = t < R ? so[t + 1] : 0;
+    const bool lng = oe - ob > tile;
+    int e = t + 1;  // one past the last row of the item that starts at row t
+    if (t < R && !lng) {
+      i32 prev = oe;
+      int mx = oe - ob;
+      for (; e < R && e - t < kTileRows; e++) {
+        const i32 o = so[e + 1];
+        const int len = o - prev;
+        mx = max(mx, len);
+        if (len > tile || o - ob > tile || mx > lane_work * lanes_per_row(e - t + 1)) break;
+        prev = o;
+      }
+    }
+    nxt[t] = (short)e;
+    __syncthreads();
+    if (t == 0)
+      for (int q = 0; q < R; q = nxt[q]) start[q] = 1;
+    __syncthreads();
+    const bool mine = start[t] != 0;
+    const bool ml = mine && lng;
+    const i64 b8 = (i64)ob & ~7ll;
+    const i32 npr = ml ? (i32)(((i64)oe - b8 + tile - 1) / tile) : 0;  // pieces: b8 + k*tile < oe
+    // items, long rows and pieces up to this row
+    i32 v[3] = {ml ? npr : (mine ? 1 : 0), ml ? 1 : 0, npr}, x[3];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int u = __shfl_up_sync(0xffffffffu, m, o);
-          if (lane >= o) m = max(m, u);
-        }
-        const int R = n + lane + 1;
-        const bool ok = valid && !lng && oe - o0 <= tile && R <= kTileRows && m <= lane_work * lanes_per_row(R);
-        const unsigned bad = ~__ballot_sync(0xffffffffu, ok);
-        const int k = bad ? __ffs(bad) - 1 : 32;
-        if (k > 0) o_end = __shfl_sync(0xffffffffu, oe, k - 1);
-        n += k;
-        if (bad) break;
-        mx = __shfl_sync(0xffffffffu, m, 31);
-      }
-      if (n > 0) {
-        if (write && lane == 0) items[bi + ni] = Item{(int32_t)t0, (int32_t)(t0 + n), o0, o_end};
-        ni++;
-        t0 += n;
-        continue;
-      }
-      // t0 and the rows after it that are longer than a tile, a lane each
-      // (lane L holds row t0 + L): their pieces' items follow (k_long_pieces)
-      const unsigned sh = ~__ballot_sync(0xffffffffu, lng);
-      const int run = sh ? __ffs(sh) - 1 : 32;
-      const i64 b8 = (i64)ob & ~7ll;
-      const i32 npr = lane < run ? (i32)(((i64)oe - b8 + tile - 1) / tile) : 0;  // pieces: b8 + k*tile < oe
-      i32 incl = npr;
+    for (int q = 0; q < 3; q++) {
+      x[q] = v[q];
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const i32 u = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += u;
+        const i32 u = __shfl_up_sync(0xffffffffu, x[q], o);
+        if (lane >= o) x[q] += u;
       }
-      if (write && lane < run) {
-        lrows[bl + nl + lane] = (i32)(t0 + lane);
-        lpiece0[bl + nl + lane] = bp + npc + incl - npr;
-        lfirst[bl + nl + lane] = bi + ni + incl - npr;
-      }
-      const i32 all = __shfl_sync(0xffffffffu, incl, 31);
-      nl += run;
-      ni += all;
-      npc += all;
-      t0 += run;
+      if (lane == 31) wsum[q][w] = x[q];
     }
-    if (!write && lane == 0) {
-      cnt[p] = ni;
-      cnt[np + p] = nl;
-      cnt[2 * np + p] = npc;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+      for (int u = 0; u < w; u++) x[q] += wsum[q][u];
+    if (!write) {
+      if (t == kPackThreads - 1) {
+        cnt[p] = x[0];
+        cnt[np + p] = x[1];
+        cnt[2 * np + p] = x[2];
+      }
+      continue;
+    }
+    const i32 it = base[p] + x[0] - v[0];
+    if (ml) {
+      const i32 l = base[(np + 1) + p] + x[1] - 1;
+      lrows[l] = (i32)(r0 + t);
+      lpiece0[l] = base[2 * (np + 1) + p] + x[2] - npr;
+      lfirst[l] = it;  // its pieces' items follow (k_long_pieces)
+    } else if (mine) {
+      items[it] = Item{(int32_t)(r0 + t), (int32_t)(r0 + e), ob, so[e]};
     }
   }
 }
@@ -903,8 +899,7 @@ void device_pack(fvg_ctx* c, const i32* off, i64 nrows, i64 chunk, i64 nchunks, 
   DBuf cnt, basev;
   cnt.alloc(sizeof(i32) * 3 * np, c->stream);
   if (chunk > kPackRows) fail(FVG_ERR_INTERNAL, "packing chunk too long");
-  constexpr int kPw = kPackThreads / 32;  // a warp per chunk
-  const unsigned pg = (unsigned)std::min<i64>((np + kPw - 1) / kPw, 1 << 20);
+  const unsigned pg = (unsigned)std::min<i64>(np, 1 << 20);  // a CTA per chunk
   k_pack<<<pg, kPackThreads, 0, c->stream>>>(off, nrows, chunk, np, tile, 0, cnt.as<i32>(), nullptr, nullptr,
                                           nullptr, nullptr, nullptr, lane_work);
   check_launch("pack");
