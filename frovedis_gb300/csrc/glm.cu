@@ -1046,10 +1046,23 @@ struct SgdArgs {
   double n_used0;
 };
 
-// w -= ra * g; b -= ra * bias  (update_model, gradient_descent.hpp:242-259)
-__global__ void k_sgd_update(double* __restrict__ LW, const double* __restrict__ G, double ra, int icpt, SgdArgs a) {
+// w -= ra * g; b -= ra * bias  (update_model, gradient_descent.hpp:242-259),
+// and the minibatch's loss into its rank's running loss (gradient_descent::
+// optimize passes one loss variable through the rank's minibatches,
+// gradient_descent.hpp:128-145).  The squared loss halves the whole running
+// value after each batch (gradient.hpp:70-73); out[0] already holds the
+// batch's halved sum, and halving commutes with rounding, so
+// 0.5 * running + out[0] equals the reference's 0.5 * (running + sum).
+// (A minibatch of 25,600 rows takes 35 us of short kernels: one launch for
+// both saves the 2.5 us of the loss's own.)
+__global__ void k_sgd_update(double* __restrict__ LW, const double* __restrict__ G, double ra, int icpt,
+                             const double* __restrict__ out, int first, int halve, SgdArgs a) {
   VEC_LOOP(j, a.n) LW[j] = __dsub_rn(LW[j], __dmul_rn(ra, G[j]));
-  if (icpt && blockIdx.x == 0 && threadIdx.x == 0) a.scal[2] = __dsub_rn(a.scal[2], __dmul_rn(ra, G[a.n]));
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (icpt) a.scal[2] = __dsub_rn(a.scal[2], __dmul_rn(ra, G[a.n]));
+    const double prev = first ? 0.0 : a.scal[6];
+    a.scal[6] = __dadd_rn(halve ? 0.5 * prev : prev, out[0]);
+  }
 }
 
 // rank delta LW - W accumulated into TOT in rank order (calc_diff_inplace +
@@ -1120,17 +1133,6 @@ __global__ void k_mark_used(const i32* __restrict__ idx, i64 nnz, int* __restric
 __global__ void k_zero_unused(double* __restrict__ W, const int* __restrict__ used, i64 n) {
   for (i64 j = (i64)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (i64)gridDim.x * blockDim.x)
     if (!used[j]) W[j] = 0.0;
-}
-
-// One minibatch's loss into its rank's running loss (gradient_descent::
-// optimize passes one loss variable through the rank's minibatches,
-// gradient_descent.hpp:128-145).  The squared loss halves the whole running
-// value after each batch (gradient.hpp:70-73); out[0] already holds the
-// batch's halved sum, and halving commutes with rounding, so
-// 0.5 * running + out[0] equals the reference's 0.5 * (running + sum).
-__global__ void k_sgd_loss(const double* __restrict__ out, double* __restrict__ scal, int first, int halve) {
-  const double prev = first ? 0.0 : scal[6];
-  scal[6] = __dadd_rn(halve ? 0.5 * prev : prev, out[0]);
 }
 
 void sgd_train(fvg_ctx* c, fvg_matrix* M, const double* label_h, const double* sw_h, const fvg_glm_params* p,
@@ -1245,11 +1247,11 @@ void sgd_train(fvg_ctx* c, fvg_matrix* M, const double* label_h, const double* s
           x = LWF.p;
         }
         b->ev.eval(x, scal.as<double>() + 2, G.as<double>(), out.as<double>());
-        k_sgd_loss<<<1, 1, 0, s>>>(out.as<double>(), scal.as<double>(), first_loss ? 1 : 0,
-                                   p->loss == FVG_LOSS_SQUARED ? 1 : 0);
-        k_sgd_update<<<vgrid, kVecThreads, 0, s>>>(LW.as<double>(), G.as<double>(), ra, p->intercept, sa);
+        k_sgd_update<<<vgrid, kVecThreads, 0, s>>>(LW.as<double>(), G.as<double>(), ra, p->intercept,
+                                                   out.as<double>(), first_loss ? 1 : 0,
+                                                   p->loss == FVG_LOSS_SQUARED ? 1 : 0, sa);
         check_launch("sgd_update");
-        count_launch(c, 2);
+        count_launch(c);
         first_loss = false;
       }
       k_sgd_delta<<<vgrid, kVecThreads, 0, s>>>(LW.as<double>(), W.as<double>(), TOT.as<double>(), first_rank ? 1 : 0,
