@@ -4,6 +4,7 @@
 #pragma once
 
 #include "fvg_internal.cuh"
+#include "logistic64.cuh"
 
 namespace fvg {
 
@@ -113,7 +114,7 @@ __device__ __forceinline__ void logistic_row(double wtx, double lab, double& los
   const double z = lab * wtx;
   const double neg = -lab;
   const double az = __hiloint2double(__double2hiint(z) & 0x7fffffff, __double2loint(z));
-  const double e = exp(-az);
+  const double e = dbl_at_least(az, 0x4085e000) ? exp(-az) : logi::exp_neg(az);  // 700 and above
   const bool up = __double2hiint(z) >= 0;  // z >= 0
   if (dbl_at_least(z, 0x40320000) && z > 18.0) {
     loss = e;
@@ -122,10 +123,10 @@ __device__ __forceinline__ void logistic_row(double wtx, double lab, double& los
     loss = az;
     d = neg;
   } else {
-    const double u = 1.0 + e;
-    loss = log(u);
+    double q;
+    logi::log_and_quotient(1.0 + e, up ? e : 1.0, loss, q);
     if (!up) loss += az;
-    d = neg * ((up ? e : 1.0) / u);
+    d = neg * q;
   }
   if (dbl_at_least(d, 0x426d1a94)) {  // 1e12 and above
     if (d > 1e12) d = 1e12;
