@@ -40,29 +40,29 @@ METRIC = "sparse LogReg L-BFGS iters/s + SpMV HBM GB/s: BF16/batched vs FP64 GPU
 PEAKS = os.path.join(ROOT, "MEASURED_PEAKS.json")
 # dram__bytes_read.sum + dram__bytes_write.sum over the algorithmic bytes of
 # the same pass (the CRS formulas of eval_bytes), per value storage, from ncu
-# captures of the benchmark matrix's kernels (profiles/ holds the summaries).
-# BF16 values, the 1,000,000-row version: pass 1 with the forward head
-# (k_panel + tail k_crs + k_finalize) 285.42 MB / 380.01 MB; pass 2 with the
-# row panels (rare-column k_crs + k_panel + k_panel_colsum) 288.54 MB /
-# 376.01 MB.  FP32 values, full size: pass 1 4060.5 MB / 4964.0 MB, pass 2
-# 4150.6 MB / 4852.0 MB.
-NCU_TRAFFIC_RATIO = {"split": {"pass1": 537.6 / 620.81, "pass2": 534.7 / 609.21},
-                     "bf16": {"pass1": 285.42 / 380.01, "pass2": 288.54 / 376.01},
-                     "f32": {"pass1": 4060.5 / 4964.0, "pass2": 4150.6 / 4852.0}}
+# captures of the benchmark matrix's kernels, the 1,000,000-row version
+# (profiles/ holds the summaries).  BF16 values: pass 1 with the forward head
+# (k_panel_stream + tail k_crs + k_finalize) 299.6 MB / 380.01 MB; pass 2 with
+# the row panels (rare-column k_crs + k_panel_stream + k_panel_colsum) 318.5
+# MB / 376.01 MB.  FP32 values: pass 1 425.0 MB / 500.0 MB, pass 2 446.8 MB /
+# 496.0 MB.
+NCU_TRAFFIC_RATIO = {"split": {"pass1": 574.1 / 620.81, "pass2": 594.1 / 609.21},
+                     "bf16": {"pass1": 299.6 / 380.01, "pass2": 318.5 / 376.01},
+                     "f32": {"pass1": 425.0 / 500.0, "pass2": 446.8 / 496.0}}
 TRAFFIC_SOURCE = {"split": "ncu dram bytes of every kernel of a pass / algorithmic bytes per pass (1/10-row "
                            "capture, all columns), x this run's algorithmic bytes per launch",
                   "bf16": "ncu dram bytes / algorithmic bytes per pass (1/10-row capture), x this run's "
                           "algorithmic bytes per launch",
-                  "f32": "ncu dram bytes / algorithmic bytes per pass (full-size capture), x this run's "
+                  "f32": "ncu dram bytes / algorithmic bytes per pass (1/10-row capture), x this run's "
                          "algorithmic bytes per launch"}
 PASS_KERNELS = {
-    "split": "pass1 A*w: forward head k_panel_split (the frequent columns' w as FP32 pairs in shared memory) + "
+    "split": "pass1 A*w: forward head k_panel_stream (the frequent columns' w as FP32 pairs in shared memory) + "
              "k_crs_split over the row tails + k_fin_split + k_glm_split (df64 logistic rows); pass2 A^T*r: row "
-             "panels k_panel_split + k_panel_colsum_split + k_crs_split over the rare columns + k_fin_split",
-    "bf16": "pass1 A*w: k_panel (forward head) + k_crs (row tails, logistic epilogue); pass2 A^T*r: k_panel "
+             "panels k_panel_stream + k_panel_colsum_split + k_crs_split over the rare columns + k_fin_split",
+    "bf16": "pass1 A*w: k_panel_stream (forward head) + k_crs (row tails, logistic epilogue); pass2 A^T*r: k_panel_stream "
             "(row panels) + k_crs (rare columns) + k_panel_colsum",
     "f32": "as bf16, FP32 values",
-    "f64": "k_crs (pass1 A*w + logistic epilogue, pass2 A^T*r on the transposed copy)",
+    "f64": "k_crs64 (pass1 A*w, pass2 A^T*r on the transposed copy) + k_finalize + k_logreg_rows (logistic rows)",
 }
 
 

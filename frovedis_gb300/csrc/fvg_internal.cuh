@@ -164,7 +164,7 @@ struct DevHYB {  // jds_crs_hybrid_local (jds_crs_hybrid.hpp:8-153)
   bool all_crs = false;  // m <= threshold: the whole matrix is the CRS part
 };
 
-// Row-panel layout of the backward product g = A^T r (FP32 arithmetic).
+// Row-panel layout of the backward product g = A^T r (FP32 and split arithmetic).
 // A's rows are cut into panels of `rows` consecutive rows; a CTA stages one
 // panel's slice of r in shared memory and sums, for every hot column h, the
 // products of the column's entries that fall in the panel ("panel row"

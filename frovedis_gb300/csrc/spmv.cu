@@ -1,23 +1,24 @@
 // Sparse products on the device.
 //
-// CRS (crs_matrix_spmv_impl, crs_matrix.hpp:1505-1516): one persistent
-// kernel walks the matrix in row order as warp work items of at most 512
-// nonzeros, built once per matrix on the host from the row offsets.  An item
-// is either a tile of consecutive short rows (up to 248 rows, a bounded
-// number of products per lane) or a piece of a long row (the finalize kernel
-// adds the pieces in order).  A warp streams the item's values and column ids
-// with coalesced evict-first loads, gathers x through the read-only path,
-// stages the products in its own shared-memory slice and sums each row with
-// 1..32 lanes.  All reductions have a fixed order, so results are
-// deterministic run to run.
+// CRS (crs_matrix_spmv_impl, crs_matrix.hpp:1505-1516): persistent kernels
+// walk the matrix in row order as warp work items of at most 512 nonzeros,
+// packed once per matrix on the device from the row offsets.  An item is
+// either a tile of consecutive short rows (up to 248 rows; for k_crs a bounded
+// number of products per lane) or a piece of a long row (k_finalize adds the
+// pieces in order).  FP32 arithmetic (k_crs): a warp streams the item's values
+// and column ids with coalesced evict-first loads, gathers x through the
+// read-only path, stages the products in its own shared-memory slice and sums
+// each row with 1..32 lanes.  FP64 arithmetic (k_crs64): the rows are cut
+// among the lanes by entries, so that every FP64 instruction serves 32 lanes.
+// All reductions have a fixed order, so results are deterministic run to run.
 //
-// The optional logistic epilogue fuses compute_wtx + logistic_gradient::
+// The optional logistic epilogue is compute_wtx + logistic_gradient::
 // compute_dloss + `* sample_weight` + bias sum (gradient_descent.hpp:196-211,
-// gradient.hpp:15-53) into the same pass: it writes dloss*sw per row and
-// per-CTA compensated partial sums of the loss and of dloss*sw (FP32 Kahan
-// sums on the FP32-arithmetic path, which keep GB300's narrow FP64 unit out of
-// the per-row work; FP64 Neumaier sums on the FP64 path), which the finalize
-// kernel reduces in FP64 in a fixed order.
+// gradient.hpp:15-53): dloss*sw per row and per-CTA compensated partial sums of
+// the loss and of dloss*sw.  FP32 arithmetic: fused into k_crs (FP32 Kahan sums,
+// which keep GB300's narrow FP64 unit out of the per-row work), the partials
+// reduced in FP64 by k_finalize.  FP64 arithmetic: a kernel of its own over the
+// finished product (k_logreg_rows).
 #include <algorithm>
 #include <mutex>
 #include <vector>
@@ -198,8 +199,8 @@ __global__ void __launch_bounds__(kThreads, FVG_CRS_MIN_BLOCKS) k_crs(const CrsK
 // 24 warps (222 KB of slices) took 1.21 ms where 12 (111 KB) take 0.44.
 // Measured (before: k_crs's rows by lanes, and its loss rows): 2M x 2M
 // power-law 558 -> 442 us; 1M x 100,000, 6.0e7 nonzeros, A w with hinge loss
-// 372 -> 221 + 60, A^T r 238 -> 221; 100,000 x 20,000, 4.0e6 nonzeros, A w
-// with logistic loss 81 -> 18 + 26, A^T r 22.6 -> 18.3.  At 6.0e7 nonzeros L1's
+// 372 -> 221 + 42, A^T r 238 -> 221; 100,000 x 20,000, 4.0e6 nonzeros, A w
+// with logistic loss 81 -> 18 + 20, A^T r 22.6 -> 18.3.  At 6.0e7 nonzeros L1's
 // data pipe is 74% and the FP64 pipe 59% busy.
 static_assert(kWarpTile == 512, "k_crs64: 16 entries a lane, a 16-word row map");
 constexpr int kC64 = 16;                               // entries per lane
@@ -483,7 +484,7 @@ __global__ void __launch_bounds__(kThreads) k_finalize(const FinK f) {
 //
 // FP64: bound by the FP64 unit (64 clocks a warp instruction) and, on small
 // matrices, by the launch and the reduction.  With the loss of logistic64.cuh
-// and a thread's first row stored as its sum (the compensated add costs 7
+// and a thread's first row stored as its sum (the compensated add costs 4
 // FP64 instructions, and up to 311,000 rows a thread has one): 100,000
 // logistic rows 20.4 us, 26.3 with the library's exp, log and division.
 template <class V> struct FirstRow {

@@ -90,7 +90,7 @@ FVG_API fvg_status fvg_ctx_reset_profile(fvg_ctx* ctx);
 /* Number of CUDA kernels this context launched since creation. */
 FVG_API int64_t fvg_ctx_kernel_launches(fvg_ctx* ctx);
 /* Poll budget of the bounded device-side waits of this context's kernels
- * (the L-BFGS direction's grid barriers, the row-panel and forward-head
+ * (the L-BFGS direction's waits for the other CTAs' sums, the row-panel and forward-head
  * kernels' bulk-copy waits).  A wait that runs out is abandoned: the kernel
  * records it in the context's error word and finishes (a copy in flight is
  * still drained), and the call returns FVG_ERR_INTERNAL; the context stays
@@ -134,8 +134,7 @@ FVG_API fvg_status fvg_matrix_add_storage(fvg_ctx* ctx, fvg_matrix* mat, fvg_dty
  * copy of r's slice, the rest through the transposed CRS.
  * rows < 0: chosen from the matrix (the default; off for small matrices or
  * when few entries fall in such columns); 0: off; > 0: panels of that many
- * rows (a multiple of 4, at most what four CTAs per SM can hold in shared
- * memory).  min_per_panel <= 0 takes the default (2).  Drops a layout built
+ * rows (a multiple of 4, at most what a CTA can hold in shared memory).  min_per_panel <= 0 takes the default (2).  Drops a layout built
  * earlier; the next FP32 / BF16 backward product builds the new one. */
 FVG_API fvg_status fvg_matrix_set_panels(fvg_ctx* ctx, fvg_matrix* mat, int64_t rows, double min_per_panel);
 /* The layout in use (built if needed): info[0] rows per panel (0: none),
