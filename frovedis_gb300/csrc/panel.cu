@@ -770,31 +770,60 @@ __global__ void k_fill_records(const i32* __restrict__ coff, const i32* __restri
 }
 
 // g[hot[h]] = sum over panels of ypan[panel*nhot + h] in a fixed order:
-// 32 columns per CTA of 1024 threads; warp w adds panels w, w+32, ... in two
-// compensated FP32 sums (GB300's FP64 unit is too narrow for one FP64 add per
-// partial), then warp 0 adds the 32 warp sums in FP64, in order.
+// 32 columns per CTA of kSumWarps warps; warp w adds panels w, w + kSumWarps,
+// ... in two compensated FP32 sums (GB300's FP64 unit is too narrow for one
+// FP64 add per partial; Knuth's TwoSum, because the partials' signs differ and
+// Kahan's form loses the remainder where an addend is larger than the sum:
+// 1.2e-7 against 0.95e-7 from the exact product), then warp 0 adds the warps' sums in FP64, in order.
+// Bound by that FP64 tail where the panels are few (2M rows: 152, 25,000
+// columns): 7.3 us with 8 warps, 19.6 with 32.
+constexpr int kSumWarps = 8;
+struct PairSum {
+  float s = 0.f, c = 0.f;
+  __device__ __forceinline__ void add(float v) {
+    const float t = s + v, bb = t - s;
+    c += (s - (t - bb)) + (v - bb);
+    s = t;
+  }
+  __device__ __forceinline__ double total() const { return (double)s + (double)c; }
+};
 template <class YT>
-__global__ void __launch_bounds__(1024) k_panel_colsum(const float* __restrict__ ypan, const i32* __restrict__ hot,
-                                                       i64 nhot, i64 np, YT* __restrict__ y) {
-  __shared__ double part[32][33];
+__global__ void __launch_bounds__(32 * kSumWarps) k_panel_colsum(const float* __restrict__ ypan,
+                                                                 const i32* __restrict__ hot, i64 nhot, i64 np,
+                                                                 YT* __restrict__ y) {
+  __shared__ double part[kSumWarps][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (i64 h0 = (i64)blockIdx.x * 32; h0 < nhot; h0 += (i64)gridDim.x * 32) {
     const i64 h = h0 + lane;
-    FSum a, b;
+    PairSum a, b;
     if (h < nhot) {
+      constexpr int U = 8;  // loads under way together
       i64 pn = w;
-      for (; pn + 32 < np; pn += 64) {
-        a.add(__ldcs(ypan + pn * nhot + h));
-        b.add(__ldcs(ypan + (pn + 32) * nhot + h));
+      for (; pn + (U - 1) * kSumWarps < np; pn += U * kSumWarps) {
+        float v[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) v[u] = __ldcs(ypan + (pn + u * kSumWarps) * nhot + h);
+#pragma unroll
+        for (int u = 0; u < U; u += 2) {
+          a.add(v[u]);
+          b.add(v[u + 1]);
+        }
       }
-      if (pn < np) a.add(__ldcs(ypan + pn * nhot + h));
+      float v[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) v[u] = pn + u * kSumWarps < np ? __ldcs(ypan + (pn + u * kSumWarps) * nhot + h) : 0.f;
+#pragma unroll
+      for (int u = 0; u < U; u += 2) {
+        a.add(v[u]);
+        b.add(v[u + 1]);
+      }
     }
     part[w][lane] = a.total() + b.total();
     __syncthreads();
     if (w == 0 && h < nhot) {
       double s = 0.0;
-#pragma unroll 8
-      for (int q = 0; q < 32; q++) s += part[q][lane];
+#pragma unroll
+      for (int q = 0; q < kSumWarps; q++) s += part[q][lane];
       y[hot[h]] = (YT)s;
     }
     __syncthreads();
@@ -1322,13 +1351,14 @@ void panel_trans_mv(fvg_ctx* c, DevPanels& pn, int storage, const float* r, int 
   crs_pass(c, pn.cold, storage, FVG_F32, r, y_dt, y, EPI_STORE, nullptr, scratch, P_NKEYS);
   if (storage == FVG_F32) launch_stream<FVG_F32>(c, pn, r, pn.ypan.p, pn.partials.p);
   else launch_stream<FVG_BF16>(c, pn, r, pn.ypan.p, pn.partials.p);
-  const unsigned cg = (unsigned)std::max<i64>(1, std::min<i64>((pn.nhot + 31) / 32, 2 * c->num_sms));
+  const unsigned cg = (unsigned)std::max<i64>(1, std::min<i64>((pn.nhot + 31) / 32, 8 * c->num_sms));
+  const int ct = 32 * kSumWarps;
   if (y_dt == FVG_F64)
-    k_panel_colsum<double><<<cg, 1024, 0, c->stream>>>(pn.ypan.as<float>(), pn.hot_cols.as<i32>(), pn.nhot,
-                                                        pn.npanels, (double*)y);
+    k_panel_colsum<double><<<cg, ct, 0, c->stream>>>(pn.ypan.as<float>(), pn.hot_cols.as<i32>(), pn.nhot, pn.npanels,
+                                                     (double*)y);
   else
-    k_panel_colsum<float><<<cg, 1024, 0, c->stream>>>(pn.ypan.as<float>(), pn.hot_cols.as<i32>(), pn.nhot,
-                                                       pn.npanels, (float*)y);
+    k_panel_colsum<float><<<cg, ct, 0, c->stream>>>(pn.ypan.as<float>(), pn.hot_cols.as<i32>(), pn.nhot, pn.npanels,
+                                                    (float*)y);
   check_launch("k_panel_colsum");
   count_launch(c);
 }
