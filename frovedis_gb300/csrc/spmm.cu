@@ -697,8 +697,9 @@ __device__ __forceinline__ void pre_fetch(const SpmmK& p, EntryPre<AT>& pre, i32
 //
 // PRE (entries fetched a chunk ahead): plain products with FP32 values up to
 // 64 columns (300 000 rows x 50 entries, 64 columns: 217 us without, 192 with;
-// 128 columns of 100 000 rows: 151 without, 176 with) and FP64 ones (100 000
-// rows x 30 entries, 32 columns: 263 without, 255 with).  BF16 values are
+// 128 columns of 100 000 rows: 151 without, 176 with) and FP64 ones up to 32
+// (150 000 rows x 60 entries, 32 columns: 545 without, 540 with; 64 columns:
+// 955 without, 1,011 with).  BF16 values are
 // faster without (60 000 rows x 20 entries, 64 columns: 55 without, 58 with),
 // and the epilogues' registers and the FP64 results of the transposed pass
 // leave no room for it (64 a thread): 796 -> 832, 702 -> 797 us.
@@ -854,7 +855,7 @@ __global__ void __launch_bounds__(kThreads, kGroupedCtas<XT, YT, EPI, G>) k_spmm
   unsigned long long mw = mask_of(p, 0);
   AT lab = 0, w = 1;
   // entries fetched ahead: see row_dot_g
-  constexpr bool PRE = EPI == EPI_STORE && sizeof(YT) == sizeof(AT) && sizeof(VT) == sizeof(AT) && (sizeof(AT) == 8 || G >= 4);
+  constexpr bool PRE = EPI == EPI_STORE && sizeof(YT) == sizeof(AT) && sizeof(VT) == sizeof(AT) && G >= (sizeof(AT) == 8 ? 2 : 4);
   EntryPre<AT> pre;
   Item next{0, 0, 0, 0};
   if (PRE && gw < p.nitems) next = p.items[gw];
