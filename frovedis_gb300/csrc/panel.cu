@@ -1070,8 +1070,16 @@ template <int ST> void fill_records(fvg_ctx* c, DevPanels& pn) {
   pn.rec[ST] = std::move(rec);
 }
 
+// The buffers of the panel rows' and the pieces' sums, each on its own: the
+// layout outlives a call in which only the first could be allocated.
+void sum_buffers(fvg_ctx* c, DevPanels& pn, DBuf& ypan, DBuf& partials, size_t elem) {
+  if (!ypan.p) ypan.alloc(elem * std::max<i64>(pn.npanels * pn.nhot, 1), c->stream);
+  if (!partials.p) partials.alloc(elem * std::max<i64>(pn.npieces, 1), c->stream);
+}
+
 // ypan (and the long rows' partials) of the layout for a vector x.
 template <int ST> void launch_stream(fvg_ctx* c, DevPanels& pn, const void* x, void* ypan, void* partials) {
+  if (!pn.rec[ST].p || !ypan || !partials) fail(FVG_ERR_INTERNAL, "a panel layout without its records or sums");
   auto kfn = k_panel_stream<ST>;
   static std::mutex mu;  // contexts of different host threads launch concurrently
   static std::vector<int> attr_set;
@@ -1331,10 +1339,7 @@ void panel_ensure_plane(fvg_ctx* c, DevPanels& pn, int dt) {
     else fill_records<FVG_BF16>(c, pn);
     if (dt != pn.master) pn.val[dt].release();  // the records hold them
   }
-  if (!pn.ypan.p) {
-    pn.ypan.alloc(sizeof(float) * std::max<i64>(pn.npanels * pn.nhot, 1), c->stream);
-    pn.partials.alloc(sizeof(float) * std::max<i64>(pn.npieces, 1), c->stream);
-  }
+  sum_buffers(c, pn, pn.ypan, pn.partials, sizeof(float));
   crs_ensure_plane(c, pn.cold, dt, pn.master);
   crs_sched(c, pn.cold, kWarpTile);  // the cold product's work items
 }
@@ -1410,10 +1415,7 @@ void panel_ensure_split(fvg_ctx* c, DevPanels& pn) {
     pn.lo.release();
   }
   crs_ensure_split(c, pn.cold, pn.master);
-  if (!pn.ypan2.p) {
-    pn.ypan2.alloc(sizeof(float2) * std::max<i64>(pn.npanels * pn.nhot, 1), c->stream);
-    pn.partials2.alloc(sizeof(float2) * std::max<i64>(pn.npieces, 1), c->stream);
-  }
+  sum_buffers(c, pn, pn.ypan2, pn.partials2, sizeof(float2));
 }
 
 i64 panel_split_scratch_bytes(fvg_ctx* c, DevPanels& pn, bool y_df) {

@@ -1,0 +1,69 @@
+"""A call whose device allocations fail, whichever of them fails first: it reports FVG_ERR_OUT_OF_MEMORY and leaves
+nothing half made on the matrix, so that the same call made again gives what it gives on a matrix that never failed.
+The failures are injected on the host; no kernel runs on a buffer that was not allocated."""
+import numpy as np
+import pytest
+
+import oracle
+
+fv = pytest.importorskip("frovedis_gb300")
+
+pytestmark = pytest.mark.gpu
+
+FVG_ERR_OUT_OF_MEMORY = 5
+
+
+def _every_failure(make, call):
+    """call(A) on matrices from make(): the n-th allocation fails, for every n until none is left to fail."""
+    inject = fv.load().fvg_debug_inject_alloc_failure
+    A = make()
+    good = call(A)
+    A.close()
+    n = 0
+    while True:
+        A = make()
+        inject(n)
+        try:
+            got = call(A)
+        except fv.FvgError as e:
+            assert e.code == FVG_ERR_OUT_OF_MEMORY, (n, str(e))
+            got = None
+        finally:
+            inject(-1)
+        done = got is not None  # the call needs no more than n allocations
+        again = call(A)
+        for a, b in zip(again, good):
+            assert np.array_equal(a, b), n
+        A.close()
+        if done:
+            return n
+        n += 1
+
+
+def _matrix(m=2000, n=300, lam=15.0, seed=4):
+    from frovedis_gb300 import datagen
+    off, idx, val, label = datagen.generate(datagen.Spec(m=m, n=n, lam=lam, seed=seed))
+    return oracle.CRS(m, n, off, idx, val), label
+
+
+@pytest.mark.parametrize("storage", ["f32", "bf16", "split"])
+def test_panel_and_head_layouts(storage):
+    a, label = _matrix()
+    w = np.random.default_rng(1).standard_normal(a.n) * 0.2
+    # the most frequent column has more than 64 entries in a panel of 1000 rows: sums of several segments
+    assert np.bincount(a.idx[:a.off[1000]], minlength=a.n).max() > 64
+
+    with fv.Context(0) as ctx:
+        def make():
+            A = ctx.matrix(a.m, a.n, a.off, a.idx, a.val)
+            A.prepare("CRS", transpose=True)
+            A.set_panels(1000, 1.0)
+            A.set_head(64)
+            return A
+
+        def call(A):
+            g, loss = fv.logreg_eval(A, label, w, b=0.3, intercept=True, storage=storage)
+            assert A.panel_info()[2] > 0 and A.head_info()[0] == 64
+            return [g, loss]
+
+        assert _every_failure(make, call) > 30
