@@ -935,10 +935,7 @@ void lbfgs_multi_train(fvg_ctx* c, const std::vector<fvg_matrix*>& mats, const s
   std::vector<int> planes{storage};
   if (refine) planes.push_back(FVG_F32);
   for (fvg_matrix* M : mats) {
-    if (!M->AT) {
-      M->AT.reset(new DevCRS());
-      crs_build_transpose(c, M->A, *M->AT, M->master);
-    }
+    transpose_of(c, M);
     for (int st : planes) {
       crs_ensure_plane(c, M->A, st, M->master);
       crs_ensure_plane(c, *M->AT, st, M->master);

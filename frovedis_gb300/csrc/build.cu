@@ -688,4 +688,32 @@ void hyb_build(fvg_ctx* c, const DevCRS& a, DevHYB& h, int master, i64 thr) {
   FVG_CUDA(cudaStreamSynchronize(c->stream));  // hcoff host buffer
 }
 
+// ------------------------------------------------------ a matrix's layouts
+template <class L, class Build> static L& built(std::unique_ptr<L>& at, Build build) {
+  if (!at) {
+    auto l = std::make_unique<L>();
+    build(*l);
+    at = std::move(l);
+  }
+  return *at;
+}
+
+DevCRS& transpose_of(fvg_ctx* c, fvg_matrix* M) {
+  return built(M->AT, [&](DevCRS& t) { crs_build_transpose(c, M->A, t, M->master); });
+}
+
+DevELL& ell_of(fvg_ctx* c, fvg_matrix* M) {
+  return built(M->ell, [&](DevELL& e) { ell_build(c, M->A, e, M->master); });
+}
+
+DevJDS& jds_of(fvg_ctx* c, fvg_matrix* M, bool trans) {
+  return built(trans ? M->tjds : M->jds,
+               [&](DevJDS& j) { jds_build(c, trans ? transpose_of(c, M) : M->A, j, M->master); });
+}
+
+DevHYB& hyb_of(fvg_ctx* c, fvg_matrix* M, bool trans) {
+  return built(trans ? M->thyb : M->hyb,
+               [&](DevHYB& h) { hyb_build(c, trans ? transpose_of(c, M) : M->A, h, M->master, 256); });
+}
+
 }  // namespace fvg

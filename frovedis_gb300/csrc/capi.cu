@@ -274,13 +274,6 @@ FVG_API fvg_status fvg_matrix_info(const fvg_matrix* M, int64_t* m, int64_t* n, 
   return FVG_OK;
 }
 
-static void ensure_transpose(fvg_ctx* c, fvg_matrix* M) {
-  if (!M->AT) {
-    M->AT.reset(new DevCRS());
-    crs_build_transpose(c, M->A, *M->AT, M->master);
-  }
-}
-
 // The CRS kernels' work schedules for the value planes the matrix has.
 static void crs_scheds(fvg_ctx* c, fvg_matrix* M, DevCRS& a) {
   for (int dt : {FVG_F64, FVG_F32, FVG_BF16})
@@ -289,35 +282,18 @@ static void crs_scheds(fvg_ctx* c, fvg_matrix* M, DevCRS& a) {
 
 static void prepare(fvg_ctx* c, fvg_matrix* M, int fmt, bool trans) {
   if (fmt == FVG_CRS) {
-    if (trans) ensure_transpose(c, M);
+    if (trans) transpose_of(c, M);
     crs_scheds(c, M, M->A);
     if (trans) crs_scheds(c, M, *M->AT);
   } else if (fmt == FVG_ELL) {
-    if (!M->ell) {
-      M->ell.reset(new DevELL());
-      ell_build(c, M->A, *M->ell, M->master);
-    }
-    if (trans) ensure_transpose(c, M);
+    ell_of(c, M);
+    if (trans) transpose_of(c, M);
   } else if (fmt == FVG_JDS) {
-    if (!M->jds) {
-      M->jds.reset(new DevJDS());
-      jds_build(c, M->A, *M->jds, M->master);
-    }
-    if (trans && !M->tjds) {
-      ensure_transpose(c, M);
-      M->tjds.reset(new DevJDS());
-      jds_build(c, *M->AT, *M->tjds, M->master);
-    }
+    jds_of(c, M, false);
+    if (trans) jds_of(c, M, true);
   } else if (fmt == FVG_HYBRID) {
-    if (!M->hyb) {
-      M->hyb.reset(new DevHYB());
-      hyb_build(c, M->A, *M->hyb, M->master, 256);
-    }
-    if (trans && !M->thyb) {
-      ensure_transpose(c, M);
-      M->thyb.reset(new DevHYB());
-      hyb_build(c, *M->AT, *M->thyb, M->master, 256);
-    }
+    hyb_of(c, M, false);
+    if (trans) hyb_of(c, M, true);
   } else {
     fail(FVG_ERR_UNSUPPORTED, "Unsupported input matrix type!!\n");
   }
@@ -496,8 +472,7 @@ FVG_API fvg_status fvg_matrix_get_transpose(fvg_ctx* c, fvg_matrix* M, int32_t* 
   if (!c || !M) return FVG_ERR_INVALID_ARG;
   API_BEGIN
   own(c, M);
-  ensure_transpose(c, M);
-  const DevCRS& t = *M->AT;
+  const DevCRS& t = transpose_of(c, M);
   if (toff) FVG_CUDA(cudaMemcpyAsync(toff, t.off.p, sizeof(int32_t) * (t.m + 1), cudaMemcpyDeviceToHost, c->stream));
   if (tidx && t.nnz)
     FVG_CUDA(cudaMemcpyAsync(tidx, t.idx.p, sizeof(int32_t) * t.nnz, cudaMemcpyDeviceToHost, c->stream));

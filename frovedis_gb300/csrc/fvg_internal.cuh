@@ -340,6 +340,12 @@ const Sched& crs_sched_slabs(fvg_ctx* c, DevCRS& a, int storage, i64 slab);
 void ell_build(fvg_ctx* c, const DevCRS& a, DevELL& e, int master);
 void jds_build(fvg_ctx* c, const DevCRS& a, DevJDS& j, int master);
 void hyb_build(fvg_ctx* c, const DevCRS& a, DevHYB& h, int master, i64 threshold);
+// The matrix's transposed copy and other layouts (of A, or of A^T), built on
+// their first use.  A build that fails leaves nothing on the matrix.
+DevCRS& transpose_of(fvg_ctx* c, fvg_matrix* M);
+DevELL& ell_of(fvg_ctx* c, fvg_matrix* M);
+DevJDS& jds_of(fvg_ctx* c, fvg_matrix* M, bool trans);
+DevHYB& hyb_of(fvg_ctx* c, fvg_matrix* M, bool trans);
 void ensure_plane_generic(fvg_ctx* c, DBuf* planes, i64 n, int dt, int master);
 
 // ------------------------------------------------------------ products

@@ -706,52 +706,16 @@ static void build_operand(fvg_ctx* c, fvg_matrix* M, int fmt, Operand& o) {
   o.m = M->A.m;
   o.n = M->A.n;
   o.master = M->master;
-  if (fmt == FVG_CRS || fmt == FVG_ELL) {
-    if (!M->AT) {
-      M->AT.reset(new DevCRS());
-      crs_build_transpose(c, M->A, *M->AT, M->master);
-    }
-    o.AT = M->AT.get();
-  }
+  if (fmt == FVG_CRS || fmt == FVG_ELL) o.AT = &transpose_of(c, M);
   if (fmt == FVG_CRS) o.A = &M->A;
-  if (fmt == FVG_ELL) {
-    if (!M->ell) {
-      M->ell.reset(new DevELL());
-      ell_build(c, M->A, *M->ell, M->master);
-    }
-    o.E = M->ell.get();
-  }
+  if (fmt == FVG_ELL) o.E = &ell_of(c, M);
   if (fmt == FVG_HYBRID) {
-    if (!M->hyb) {
-      M->hyb.reset(new DevHYB());
-      hyb_build(c, M->A, *M->hyb, M->master, 256);
-    }
-    if (!M->thyb) {
-      if (!M->AT) {
-        M->AT.reset(new DevCRS());
-        crs_build_transpose(c, M->A, *M->AT, M->master);
-      }
-      M->thyb.reset(new DevHYB());
-      hyb_build(c, *M->AT, *M->thyb, M->master, 256);
-    }
-    o.H = M->hyb.get();
-    o.HT = M->thyb.get();
+    o.H = &hyb_of(c, M, false);
+    o.HT = &hyb_of(c, M, true);
   }
   if (fmt == FVG_JDS) {
-    if (!M->jds) {
-      M->jds.reset(new DevJDS());
-      jds_build(c, M->A, *M->jds, M->master);
-    }
-    if (!M->tjds) {
-      if (!M->AT) {
-        M->AT.reset(new DevCRS());
-        crs_build_transpose(c, M->A, *M->AT, M->master);
-      }
-      M->tjds.reset(new DevJDS());
-      jds_build(c, *M->AT, *M->tjds, M->master);
-    }
-    o.J = M->jds.get();
-    o.JT = M->tjds.get();
+    o.J = &jds_of(c, M, false);
+    o.JT = &jds_of(c, M, true);
   }
 }
 

@@ -226,10 +226,7 @@ void multinomial_train(fvg_ctx* c, fvg_matrix* M, const double* label_h, const d
     fail(FVG_ERR_UNSUPPORTED, "Unsupported input matrix type!!\n");
   const i64 m = M->A.m, n = M->A.n;
   cudaStream_t s = c->stream;
-  if (!M->AT) {
-    M->AT.reset(new DevCRS());
-    crs_build_transpose(c, M->A, *M->AT, M->master);
-  }
+  transpose_of(c, M);
   const int storage = p->storage;
   if (storage == FVG_SPLIT) fail(FVG_ERR_UNSUPPORTED, "split storage is offered by the L-BFGS trainers, single evaluations and the products");
   const bool mixed = storage != FVG_F64;
@@ -361,10 +358,7 @@ void multinomial_lbfgs_train(fvg_ctx* c, fvg_matrix* M, const double* label_h, c
   if (storage == FVG_SPLIT) fail(FVG_ERR_UNSUPPORTED, "split storage is offered by the binary L-BFGS trainers, single evaluations and the products");
   const i64 m = M->A.m, n = M->A.n;
   cudaStream_t s = c->stream;
-  if (!M->AT) {
-    M->AT.reset(new DevCRS());
-    crs_build_transpose(c, M->A, *M->AT, M->master);
-  }
+  transpose_of(c, M);
   crs_ensure_plane(c, *M->AT, storage, M->master);
   DBuf label, sw;
   label.alloc(sizeof(double) * m, s);

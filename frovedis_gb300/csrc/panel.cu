@@ -1321,10 +1321,7 @@ DevPanels* panels_for(fvg_ctx* c, fvg_matrix* M) {
   if (M->panel_rows == 0) return nullptr;
   if (M->pan) return M->pan.get();
   if (M->pan_tried) return nullptr;
-  if (!M->AT) {
-    M->AT.reset(new DevCRS());
-    crs_build_transpose(c, M->A, *M->AT, M->master);
-  }
+  transpose_of(c, M);
   // a forced layout that cannot be built throws here, on every call
   std::unique_ptr<DevPanels> pn = panel_build(c, *M->AT, M->master, M->panel_rows, M->panel_min);
   M->pan_tried = true;
@@ -1376,10 +1373,7 @@ DevPanels* head_for(fvg_ctx* c, fvg_matrix* M) {
   if (M->head_cols == 0) return nullptr;
   if (M->head) return M->head.get();
   if (M->head_tried) return nullptr;
-  if (!M->AT) {
-    M->AT.reset(new DevCRS());
-    crs_build_transpose(c, M->A, *M->AT, M->master);
-  }
+  transpose_of(c, M);
   std::unique_ptr<DevPanels> hd = head_build(c, M->A, *M->AT, M->master, M->head_cols);
   M->head_tried = true;
   M->head = std::move(hd);

@@ -42,11 +42,11 @@ void inject_alloc_failure(long long after) { g_alloc_fail_after.store(after); }
 void DBuf::alloc(size_t nbytes, cudaStream_t s) {
   release();
   stream = s;
-  bytes = nbytes;
   if (nbytes == 0) return;
   if (g_alloc_fail_after.load() >= 0 && g_alloc_fail_after.fetch_sub(1) == 0)
     throw_cuda(cudaErrorMemoryAllocation, "cudaMallocAsync (injected failure)", __FILE__, __LINE__);
   FVG_CUDA(cudaMallocAsync(&p, nbytes, s));
+  bytes = nbytes;
   // the SpMV kernels issue 16-byte vector loads from the start of every
   // index/value array
   if (reinterpret_cast<uintptr_t>(p) & 255u) fail(FVG_ERR_INTERNAL, "device allocation is not 256-byte aligned");

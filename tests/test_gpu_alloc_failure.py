@@ -67,3 +67,39 @@ def test_panel_and_head_layouts(storage):
             return [g, loss]
 
         assert _every_failure(make, call) > 30
+
+
+@pytest.mark.parametrize("fmt", ["CRS", "ELL", "JDS", "HYBRID"])
+def test_first_use_of_a_format(fmt):
+    """The transposed copy and the format's own layouts, built by the call itself; also the bytes the matrix reports."""
+    a, _ = _matrix(m=700, n=90, lam=8.0)
+    x = np.random.default_rng(2).standard_normal(a.n)
+    r = np.random.default_rng(3).standard_normal(a.m)
+    with fv.Context(0) as ctx:
+        def call(A):
+            y = [A.spmv(x, fmt=fmt), A.trans_mv(r, fmt=fmt)]
+            return y + [A.device_bytes]
+
+        assert _every_failure(lambda: ctx.matrix(a.m, a.n, a.off, a.idx, a.val), call) > 10
+
+
+@pytest.mark.parametrize("what", ["batched", "multinomial", "probability", "sgd"])
+def test_first_use_by_a_trainer(what):
+    a, label = _matrix(m=600, n=80, lam=8.0)
+    kinds = (np.arange(a.m) % 3).astype(np.float64)
+    W = np.random.default_rng(5).standard_normal((a.n, 3))
+
+    def call(A):
+        if what == "batched":
+            r = fv.logreg_lbfgs_batched(A, label, [1e-3, 1e-1], num_iter=3, reg_type="L2")
+            return [r["w"], r["loss"]]
+        if what == "multinomial":
+            r = fv.multinomial_lbfgs(A, kinds, 3, num_iter=2, reg_type="L2", reg_param=1e-3)
+            return [r["W"], r["loss"]]
+        if what == "probability":
+            return [fv.multinomial_probability(A, W, np.zeros(3))]
+        r = fv.logreg_sgd(A, label, num_iter=2, alpha=0.01, mini_batch_fraction=0.5)
+        return [r["w"], r["loss"]]
+
+    with fv.Context(0) as ctx:
+        assert _every_failure(lambda: ctx.matrix(a.m, a.n, a.off, a.idx, a.val), call) > 2
