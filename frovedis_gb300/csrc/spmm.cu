@@ -747,15 +747,17 @@ __device__ __forceinline__ void row_dot_g(const SpmmK& p, i32 e0, i32 e1, int la
     // lanes whose columns are not computed skip the chunk
     if (!mine) continue;
     if constexpr (!PACK) {
-      const int steps = (cnt + G - 1) / G;
-#pragma unroll 4
-      for (int k = 0; k < steps; k++) {
+      auto step = [&](int k) {
         const StageE<AT> t = st[k * G + grp];
         XT x[CPL];
         VecLd<XT, CPL>::ld((const XT*)(X + (unsigned long long)(unsigned)t.col * ldx), x);
 #pragma unroll
         for (int q = 0; q < CPL; q++) a[q] += t.v * (AT)x[q];
-      }
+      };
+      const int whole = cnt / G;
+#pragma unroll 4
+      for (int k = 0; k < whole; k++) step(k);
+      if (whole * G + grp < cnt) step(whole);  // the padding is no entry: 0 * infinity would be one
     } else {
       // the lane's 8 FP32 columns in one 32-byte load, as 4 packed pairs
       static_assert(!PACK || CPL == 8, "one 32-byte load a lane");
