@@ -401,6 +401,17 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// Compensated FP32 sum (Knuth's TwoSum).
+struct PairSum {
+  float s = 0.f, c = 0.f;
+  __device__ __forceinline__ void add(float v) {
+    const float t = s + v, bb = t - s;
+    c += (s - (t - bb)) + (v - bb);
+    s = t;
+  }
+  __device__ __forceinline__ double total() const { return (double)s + (double)c; }
+};
+
 struct StreamK {
   const unsigned char* rec;
   const i32* coff;    // first chunk of each slice
@@ -424,15 +435,18 @@ __device__ __forceinline__ df shfl_xor_df(df a, int o) {
   return {__shfl_xor_sync(0xffffffffu, a.h, o), __shfl_xor_sync(0xffffffffu, a.l, o)};
 }
 
-// One lane's 4 products of a chunk, and a segment's running sum.  FP32: one
-// sum per entry of a chunk, so chains stay at 16 adds; split: exact products
-// p + t, df sums (TwoSum).
+// One lane's 4 entries of a chunk, and a segment's running sum.  FP32: one
+// chain of fused multiply-adds per entry of a chunk and chunk of a copy, so
+// chains stay at 8; split: exact products p + t, df sums (TwoSum).
+// (FP32 error of A^T x, 2M x 200,000 BF16 values, five draws, from the 64-bit
+// product: 1.03e-7 with rounded products in chains of 16 and plain sums over a
+// long row's segments; 7.8e-8 with this and compensated sums over them, in the
+// same time: 231 and 232 us.)
 template <int ST> struct ChunkProd {
-  float p[4];
+  float v[4], x[4];
   __device__ __forceinline__ void load(const unsigned char* rec, int lane, const float* xs) {
     using R = StreamRec<ST>;
     const uint2 q = reinterpret_cast<const uint2*>(rec + R::kValB)[lane];
-    float v[4];
     if constexpr (ST == FVG_F32) {
       const float4 h = reinterpret_cast<const float4*>(rec)[lane];
       v[0] = h.x; v[1] = h.y; v[2] = h.z; v[3] = h.w;
@@ -441,10 +455,10 @@ template <int ST> struct ChunkProd {
       v[0] = __uint_as_float(h.x << 16); v[1] = __uint_as_float(h.x & 0xffff0000u);
       v[2] = __uint_as_float(h.y << 16); v[3] = __uint_as_float(h.y & 0xffff0000u);
     }
-    p[0] = v[0] * xs[q.x & 0xffffu];
-    p[1] = v[1] * xs[q.x >> 16];
-    p[2] = v[2] * xs[q.y & 0xffffu];
-    p[3] = v[3] * xs[q.y >> 16];
+    x[0] = xs[q.x & 0xffffu];
+    x[1] = xs[q.x >> 16];
+    x[2] = xs[q.y & 0xffffu];
+    x[3] = xs[q.y >> 16];
   }
 };
 template <> struct ChunkProd<FVG_SPLIT> {
@@ -462,16 +476,21 @@ template <> struct ChunkProd<FVG_SPLIT> {
   }
 };
 template <int ST> struct SegSum {
-  float s[4] = {0.f, 0.f, 0.f, 0.f};
-  __device__ __forceinline__ void add(const ChunkProd<ST>& c) {
+  float s[kStreamChunks][4] = {};
+  __device__ __forceinline__ void add(const ChunkProd<ST>& c, int of) {
 #pragma unroll
-    for (int k = 0; k < 4; k++) s[k] += c.p[k];
+    for (int k = 0; k < 4; k++) s[of][k] = fmaf(c.v[k], c.x[k], s[of][k]);
   }
-  __device__ __forceinline__ float get() const { return (s[0] + s[1]) + (s[2] + s[3]); }
+  __device__ __forceinline__ float get() const {
+    float t = 0.f;
+#pragma unroll
+    for (int q = 0; q < kStreamChunks; q++) t += (s[q][0] + s[q][1]) + (s[q][2] + s[q][3]);
+    return t;
+  }
 };
 template <> struct SegSum<FVG_SPLIT> {
   DfAcc a;
-  __device__ __forceinline__ void add(const ChunkProd<FVG_SPLIT>& c) {
+  __device__ __forceinline__ void add(const ChunkProd<FVG_SPLIT>& c, int) {
 #pragma unroll
     for (int k = 0; k < 4; k++) a.add(c.p[k], c.t[k]);
   }
@@ -581,7 +600,7 @@ __global__ void __launch_bounds__(kStreamWarps * 32, 1) k_panel_stream(const Str
         dead = true;
         break;
       }
-      // all the copy's products first (their shared loads overlap), so that
+      // all the copy's entries first (their shared loads overlap), so that
       // the ring slot is free for the next copy before the sums
       const unsigned char* cur = ring + us * (SC * R::kB);
       ChunkProd<ST> c[SC];
@@ -599,7 +618,7 @@ __global__ void __launch_bounds__(kStreamWarps * 32, 1) k_panel_stream(const Str
       for (int k = 0; k < SC; k++) {
         if (g >= ge) break;
         while (g == ce) next_slice();
-        sum.add(c[k]);
+        sum.add(c[k], k);
         g++;
       }
     }
@@ -617,11 +636,15 @@ __global__ void __launch_bounds__(kStreamWarps * 32, 1) k_panel_stream(const Str
         for (int o = 16; o > 0; o >>= 1) a = df_add(a, shfl_xor_df(a, o));
         if (lane == 0) ypan[p.long_rows[L]] = df_pack(a);
       } else {
-        float a = 0.f;
-        for (int j = c0 + lane; j < c1; j += 32) a += __ldcg(partials + j);
+        PairSum a;
+        for (int j = c0 + lane; j < c1; j += 32) a.add(__ldcg(partials + j));
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (lane == 0) ypan[p.long_rows[L]] = a;
+        for (int o = 16; o > 0; o >>= 1) {
+          const float v = __shfl_xor_sync(0xffffffffu, a.s, o), r = __shfl_xor_sync(0xffffffffu, a.c, o);
+          a.add(v);
+          a.c += r;
+        }
+        if (lane == 0) ypan[p.long_rows[L]] = a.s + a.c;
       }
     }
   }
@@ -772,21 +795,12 @@ __global__ void k_fill_records(const i32* __restrict__ coff, const i32* __restri
 // g[hot[h]] = sum over panels of ypan[panel*nhot + h] in a fixed order:
 // 32 columns per CTA of kSumWarps warps; warp w adds panels w, w + kSumWarps,
 // ... in two compensated FP32 sums (GB300's FP64 unit is too narrow for one
-// FP64 add per partial; Knuth's TwoSum, because the partials' signs differ and
-// Kahan's form loses the remainder where an addend is larger than the sum:
-// 1.2e-7 against 0.95e-7 from the exact product), then warp 0 adds the warps' sums in FP64, in order.
+// FP64 add per partial; TwoSum, because the partials' signs differ and Kahan's
+// form loses the remainder where an addend is larger than the sum), then warp
+// 0 adds the warps' sums in FP64, in order.
 // Bound by that FP64 tail where the panels are few (2M rows: 152, 25,000
 // columns): 7.3 us with 8 warps, 19.6 with 32.
 constexpr int kSumWarps = 8;
-struct PairSum {
-  float s = 0.f, c = 0.f;
-  __device__ __forceinline__ void add(float v) {
-    const float t = s + v, bb = t - s;
-    c += (s - (t - bb)) + (v - bb);
-    s = t;
-  }
-  __device__ __forceinline__ double total() const { return (double)s + (double)c; }
-};
 template <class YT>
 __global__ void __launch_bounds__(32 * kSumWarps) k_panel_colsum(const float* __restrict__ ypan,
                                                                  const i32* __restrict__ hot, i64 nhot, i64 np,
