@@ -313,9 +313,9 @@ FVG_API fvg_status fvg_matrix_prepare(fvg_ctx* c, fvg_matrix* M, fvg_format fmt,
     const bool split = M->A.lo.p != nullptr;  // its FP32 plane belongs to the split values
     for (DevPanels* p : {pt, hd}) {
       if (!p) continue;
-      if (split) panel_ensure_split(c, *p);
+      if (split) panel_ensure_split(c, M, *p);
       for (int dt : {FVG_F32, FVG_BF16})
-        if (M->A.val[dt].p && !(split && dt == FVG_F32)) panel_ensure_plane(c, *p, dt);
+        if (M->A.val[dt].p && !(split && dt == FVG_F32)) panel_ensure_plane(c, M, *p, dt);
     }
   }
   FVG_CUDA(cudaStreamSynchronize(c->stream));
@@ -443,12 +443,11 @@ FVG_API int64_t fvg_matrix_device_bytes(const fvg_matrix* M) {
   for (const DevPanels* p : {M->pan.get(), M->head.get()}) {
     if (!p) continue;
     b += crs_bytes(p->cold);
-    for (const DBuf* d : {&p->hot_cols, &p->poff, &p->prow, &p->lo, &p->coff, &p->vout, &p->vsrc, &p->vlen, &p->wstart,
-                          &p->ulong0, &p->long_rows, &p->long_piece0, &p->ypan, &p->partials, &p->ypan2,
+    for (const DBuf* d : {&p->hot_cols, &p->src, &p->poff, &p->coff, &p->vout, &p->voff, &p->spos, &p->wstart, &p->ulong0,
+                          &p->long_rows, &p->long_piece0, &p->ypan, &p->partials, &p->ypan2,
                           &p->partials2})
       b += (int64_t)d->bytes;
     for (auto& r : p->rec) b += (int64_t)r.bytes;
-    for (auto& v : p->val) b += (int64_t)v.bytes;
   }
   return b;
 }
@@ -666,6 +665,7 @@ static void run_product_split(fvg_ctx* c, fvg_matrix* M, int fmt, const void* x,
   }
   DevPanels* pt = trans ? panels_for(c, M) : nullptr;
   if (pt) {
+    panel_ensure_split(c, M, *pt);
     ProfScope ps(c, P_SPMV_CRS);
     panel_trans_mv_split(c, *pt, x2.p, dy, nullptr);
   } else {
@@ -700,9 +700,10 @@ static void run_product(fvg_ctx* c, fvg_matrix* M, int fmt, int storage, int vec
     else hyb_spmv(c, *M->hyb, storage, v.kdt, v.dx, out_dt, v.dy);
   } else {
     DevPanels* pt = (storage != FVG_F64 && (fmt == FVG_CRS || fmt == FVG_ELL)) ? panels_for(c, M) : nullptr;
-    if (pt)
+    if (pt) {
+      panel_ensure_plane(c, M, *pt, storage);
       panel_trans_mv(c, *pt, storage, (const float*)v.dx, out_dt, v.dy, nullptr, P_SPMV_CRS);
-    else if (fmt == FVG_CRS || fmt == FVG_ELL)
+    } else if (fmt == FVG_CRS || fmt == FVG_ELL)
       crs_pass(c, *M->AT, storage, v.kdt, v.dx, out_dt, v.dy, EPI_STORE, nullptr, nullptr, P_SPMV_CRS);
     else if (fmt == FVG_JDS) jds_spmv(c, *M->tjds, storage, v.kdt, v.dx, out_dt, v.dy, false);
     else hyb_spmv(c, *M->thyb, storage, v.kdt, v.dx, out_dt, v.dy);

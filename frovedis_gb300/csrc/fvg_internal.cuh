@@ -179,16 +179,15 @@ struct DevPanels {
   double min_per_panel = 0.0;
   int master = FVG_F64;
   DBuf hot_cols;                    // int32 [nhot], ascending
-  DBuf poff;                        // int32 [npanels*nhot + 1]
-  DBuf prow;                        // uint16 [E + kPad]: row within the panel
-  DBuf val[3];                      // [E + kPad] per dtype
-  DBuf lo;                          // bf16 [E + kPad]: residual of the FP32 values (split storage)
+  DBuf src;                         // int32 [nhot][npanels + 1]: where A^T's entries of (hot column, panel) start
+  DBuf poff;                        // forward head: int32 [npanels*nhot + 1], offsets of the rows' head entries
   DevCRS cold;                      // n rows, hot rows empty
   // streamed layout of the panel rows (panel.cu): segments of at most 64
   // entries, sorted by length within a panel, in slices of 32 lanes
   i64 group = 1, nunits = 0;        // panels a CTA takes at a time, such units
   i64 nslices = 0, nchunks = 0;
-  DBuf coff, vout, vsrc, vlen, wstart;
+  DBuf coff, vout, wstart;
+  DBuf voff, spos;                  // int32: first segment of each panel row; a segment's slice * 32 + lane
   i64 nlong = 0, npieces = 0;       // panel rows of several segments
   DBuf ulong0, long_rows, long_piece0;
   DBuf rec[4];                      // records by value storage (FVG_F32, FVG_BF16, FVG_SPLIT)
@@ -434,7 +433,9 @@ void crs_spmm_store_seg(fvg_ctx* c, DevCRS& a, int storage, const void* X, i64 l
 // matrix's column counts make it pay (or as forced); returns null when the
 // plain transposed CRS is used.
 DevPanels* panels_for(fvg_ctx* c, fvg_matrix* M);
-void panel_ensure_plane(fvg_ctx* c, DevPanels& pn, int dt);
+// The records of a value storage (panels or head) and the products' buffers;
+// a product needs them made first.
+void panel_ensure_plane(fvg_ctx* c, fvg_matrix* M, DevPanels& pn, int dt);
 i64 panel_scratch_bytes(fvg_ctx* c, DevPanels& pn, int storage);
 // y[0..n) = A^T r for FP32 r; y FP64 or FP32.
 void panel_trans_mv(fvg_ctx* c, DevPanels& pn, int storage, const float* r, int y_dt, void* y, void* scratch,
@@ -443,14 +444,13 @@ void panel_trans_mv(fvg_ctx* c, DevPanels& pn, int storage, const float* r, int 
 // is used), and that pass: head partials, then the tail's CRS pass with the
 // logistic epilogue over head + tail.
 DevPanels* head_for(fvg_ctx* c, fvg_matrix* M);
-void head_ensure_plane(fvg_ctx* c, DevPanels& hd, int dt);
 i64 head_scratch_bytes(fvg_ctx* c, DevPanels& hd, int storage);
 void head_logreg_pass(fvg_ctx* c, DevPanels& hd, int storage, const float* w, const LogregEpi& lr, void* scratch,
                       int prof_key);
 // Split storage on the same layouts: g = A^T r (r df pairs, g FP64: hot
 // columns from the panels, the rest from the cold CRS); the forward head's
 // partial per row into hd.ypan2 and the tail's product into wtx (df pairs).
-void panel_ensure_split(fvg_ctx* c, DevPanels& pn);
+void panel_ensure_split(fvg_ctx* c, fvg_matrix* M, DevPanels& pn);
 i64 panel_split_scratch_bytes(fvg_ctx* c, DevPanels& pn, bool y_df);
 void panel_trans_mv_split(fvg_ctx* c, DevPanels& pn, const void* r, double* y, void* scratch);
 void head_pass_split(fvg_ctx* c, DevPanels& hd, const void* w, void* wtx, void* scratch);

@@ -583,12 +583,12 @@ struct Evaluator {
     if (op->M && op->fmt == FVG_CRS) {
       PT = panels_for(c, op->M);
       if (PT) {
-        panel_ensure_split(c, *PT);
+        panel_ensure_split(c, op->M, *PT);
         s3.alloc(panel_split_scratch_bytes(c, *PT, false), c->stream);
       }
       HD = head_for(c, op->M);
       if (HD) {
-        panel_ensure_split(c, *HD);
+        panel_ensure_split(c, op->M, *HD);
         s4.alloc(panel_split_scratch_bytes(c, *HD, true), c->stream);
       }
     }
@@ -633,7 +633,7 @@ struct Evaluator {
     if (!PT && op->AT) {
       PT = panels_for(c, op->M);
       if (PT) {
-        panel_ensure_plane(c, *PT, storage);
+        panel_ensure_plane(c, op->M, *PT, storage);
         s3.alloc(panel_scratch_bytes(c, *PT, storage), c->stream);
         FVG_CUDA(cudaMemsetAsync(s3.p, 0, 256, c->stream));
       }
@@ -641,7 +641,7 @@ struct Evaluator {
     if (!HD && op->fmt == FVG_CRS && op->A) {
       HD = head_for(c, op->M);
       if (HD) {
-        head_ensure_plane(c, *HD, storage);
+        panel_ensure_plane(c, op->M, *HD, storage);
         s4.alloc(head_scratch_bytes(c, *HD, storage), c->stream);
         FVG_CUDA(cudaMemsetAsync(s4.p, 0, 256, c->stream));
       }
@@ -651,8 +651,8 @@ struct Evaluator {
     storage = st;
     ensure_storage(c, *op, storage);
     use_panels();
-    if (PT && storage != FVG_F64) panel_ensure_plane(c, *PT, storage);
-    if (HD && storage != FVG_F64) head_ensure_plane(c, *HD, storage);
+    if (PT && storage != FVG_F64) panel_ensure_plane(c, op->M, *PT, storage);
+    if (HD && storage != FVG_F64) panel_ensure_plane(c, op->M, *HD, storage);
   }
   // x: weights (FP64 for FP64 storage, FP32 otherwise); b: device intercept
   void eval(const void* x, const double* b, double* grad, double* out) {

@@ -28,11 +28,13 @@
 #include <algorithm>
 #include <cmath>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "bulk_copy.cuh"
 #include "device_common.cuh"
 #include "df64.cuh"
+#include "split_bits.h"
 
 namespace fvg {
 
@@ -118,24 +120,6 @@ struct SidePlanes {
     if (slo) dlo[to] = slo[from];
   }
 };
-
-// a warp per panel row: its entries copied with the row made panel-local
-template <class T>
-__global__ void k_panel_fill(const i32* __restrict__ B, const i64* __restrict__ poff, const i32* __restrict__ tidx,
-                             const T* __restrict__ tval, i64 nhot, i64 np, i64 rows, uint16_t* __restrict__ prow,
-                             T* __restrict__ pval, const SidePlanes sp) {
-  const int lane = threadIdx.x & 31;
-  PWARP_STRIDE(q, np * nhot) {
-    const i64 p = q / nhot, h = q - p * nhot;
-    const i64 s = B[h * (np + 1) + p], e = B[h * (np + 1) + p + 1], d = poff[q];
-    const i64 r0 = p * rows;
-    for (i64 k = lane; k < e - s; k += 32) {
-      prow[d + k] = (uint16_t)(tidx[s + k] - r0);
-      pval[d + k] = tval[s + k];
-      sp.copy(s + k, d + k);
-    }
-  }
-}
 
 __global__ void k_cold_lens(const i32* __restrict__ toff, const i64* __restrict__ flag, i64 n, i64* __restrict__ len) {
   PGRID_STRIDE(c, n) len[c] = flag[c] ? 0 : (i64)toff[c + 1] - toff[c];
@@ -315,39 +299,27 @@ __global__ void k_head_off(const i64* __restrict__ hoff, i64 m, i64 Q, i32* __re
   PGRID_STRIDE(q, Q + 1) poff[q] = (i32)hoff[q < m ? q : m];
 }
 
-// a warp per row: head entries (slot, value) and tail entries (column,
-// value), each in the row's order
+// a warp per row: its tail entries (column, value), in the row's order
 template <class T>
-__global__ void k_head_fill(const i32* __restrict__ off, const i32* __restrict__ idx, const T* __restrict__ val,
-                            i64 m, const i32* __restrict__ slot, const i64* __restrict__ hoff,
-                            const i64* __restrict__ toff, uint16_t* __restrict__ hslot, T* __restrict__ hval,
-                            i32* __restrict__ tidx, T* __restrict__ tval, const SidePlanes sph,
-                            const SidePlanes spt) {
+__global__ void k_tail_fill(const i32* __restrict__ off, const i32* __restrict__ idx, const T* __restrict__ val,
+                            i64 m, const i32* __restrict__ slot, const i64* __restrict__ toff,
+                            i32* __restrict__ tidx, T* __restrict__ tval, const SidePlanes sp) {
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   PWARP_STRIDE(r, m) {
     const i64 s0 = off[r], e0 = off[r + 1];
-    i64 hp = hoff[r], tp = toff[r];
+    i64 tp = toff[r];
     for (i64 b = s0; b < e0; b += 32) {
       const i64 e = b + lane;
-      const bool ok = e < e0;
-      const i32 col = ok ? idx[e] : 0;
-      const i32 sl = ok ? slot[col] : -1;
-      const bool head = ok && sl >= 0;
-      const unsigned hb = __ballot_sync(0xffffffffu, head);
-      const unsigned tb = __ballot_sync(0xffffffffu, ok && !head);
-      if (head) {
-        const i64 q = hp + __popc(hb & lt);
-        hslot[q] = (uint16_t)sl;
-        hval[q] = val[e];
-        sph.copy(e, q);
-      } else if (ok) {
+      const i32 col = e < e0 ? idx[e] : 0;
+      const bool tail = e < e0 && slot[col] < 0;
+      const unsigned tb = __ballot_sync(0xffffffffu, tail);
+      if (tail) {
         const i64 q = tp + __popc(tb & lt);
         tidx[q] = col;
         tval[q] = val[e];
-        spt.copy(e, q);
+        sp.copy(e, q);
       }
-      hp += __popc(hb);
       tp += __popc(tb);
     }
   }
@@ -700,12 +672,12 @@ __global__ void k_take_every(const i64* __restrict__ src, i64 step, i64 limit, i
   PGRID_STRIDE(i, n) out[i] = src[min(i * step, limit)];
 }
 
-// per (slice, lane): where the segment's sum goes, its first entry and its
-// entries; per slice its chunks (lane 0 holds the longest segment)
+// per (slice, lane): where the segment's sum goes; per segment its slice and
+// lane; per slice its chunks (lane 0 holds the longest segment)
 __global__ void k_slices(const i32* __restrict__ poff, const i64* __restrict__ voff, const i64* __restrict__ lpc,
                          const uint32_t* __restrict__ ids, const i32* __restrict__ vq, const i64* __restrict__ sbase,
                          const i64* __restrict__ pstart, i64 np, i64 ns, i32* __restrict__ vout,
-                         i32* __restrict__ vsrc, unsigned char* __restrict__ vlen, i64* __restrict__ width) {
+                         i32* __restrict__ spos, i64* __restrict__ width) {
   PGRID_STRIDE(t, ns * 32) {
     const i64 s = t >> 5;
     i64 a = 0, b = np;  // the panel holding slice s: sbase[a] <= s < sbase[a + 1]
@@ -715,19 +687,16 @@ __global__ void k_slices(const i32* __restrict__ poff, const i64* __restrict__ v
       else b = mid;
     }
     const i64 i = pstart[a] + (s - sbase[a]) * 32 + (t & 31);
-    i32 out = kNoRow, src = 0, cnt = 0, c0 = 0, c1 = 0;
+    i32 out = kNoRow, c0 = 0, c1 = 0;
     if (i < pstart[a + 1]) {
       const i64 v = ids[i];
       const i32 q = vq[v];
       const i32 n = (i32)(voff[q + 1] - voff[q]), j = (i32)(v - voff[q]), len = poff[q + 1] - poff[q];
       seg_chunks(len, j, n, c0, c1);
       out = n > 1 ? ~(i32)(lpc[q] + j) : q;
-      src = poff[q] + 4 * c0;
-      cnt = min(4 * c1, len) - 4 * c0;
+      spos[v] = (i32)t;
     }
     vout[t] = out;
-    vsrc[t] = src;
-    vlen[t] = (unsigned char)cnt;
     if ((t & 31) == 0) width[s] = c1 - c0;
   }
 }
@@ -759,35 +728,111 @@ __global__ void k_warp_starts(const i32* __restrict__ coff, const i64* __restric
   }
 }
 
-// a warp per slice: its records from the packed entries
+// Records are written straight from the CRS values the layout is made of (A^T
+// for row panels, A for the head), so no second copy of the entries is kept or
+// needed while a layout is built: first every record as padding, then each
+// panel row's entries at their segments' places.  Neighbouring entries of a
+// row share a chunk, and the chunks of a panel stay in L2 until all its rows
+// are in.
 template <int ST>
-__global__ void k_fill_records(const i32* __restrict__ coff, const i32* __restrict__ vsrc,
-                               const unsigned char* __restrict__ vlen, i64 ns, const uint16_t* __restrict__ prow,
-                               const float* __restrict__ v32, const unsigned short* __restrict__ v16,
-                               const unsigned short* __restrict__ lo, unsigned pad, unsigned char* __restrict__ rec) {
+__global__ void k_blank_records(unsigned char* __restrict__ rec, i64 nrec, unsigned pad) {
   using R = StreamRec<ST>;
-  const int lane = threadIdx.x & 31;
-  PWARP_STRIDE(s, ns) {
-    const i32 src = vsrc[s * 32 + lane];
-    const int n = vlen[s * 32 + lane], c0 = coff[s], w = coff[s + 1] - c0;
-    for (int c = 0; c < w; c++) {
-      unsigned char* r = rec + (i64)(c0 + c) * R::kB;
-      float v[4];
-      unsigned h[4], l[4], q[4];
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        const bool in = 4 * c + k < n;
-        const i64 e = (i64)src + 4 * c + k;
-        q[k] = in ? prow[e] : pad;
-        if (ST == FVG_BF16) h[k] = in ? v16[e] : 0u;
-        else v[k] = in ? v32[e] : 0.f;
-        if (ST == FVG_SPLIT) l[k] = in ? lo[e] : 0u;
+  constexpr int kW = R::kB / 16;
+  const unsigned pp = pad | (pad << 16);
+  PGRID_STRIDE(i, nrec * kW)
+    reinterpret_cast<uint4*>(rec)[i] = (i % kW) * 16 >= R::kValB + R::kLoB ? make_uint4(pp, pp, pp, pp) : uint4{};
+}
+
+// Entry e (0..3) of a lane's chunk: the value as `ST` stores it (the same
+// roundings as the value planes') and its slot.
+template <int ST, class T>
+__device__ __forceinline__ void put_entry(unsigned char* chunk, int lane, int e, T v, unsigned slot) {
+  using R = StreamRec<ST>;
+  const int o = lane * 4 + e;
+  if constexpr (ST == FVG_BF16) {
+    bf16 b;
+    if constexpr (std::is_same_v<T, double>) b = __double2bfloat16(v);
+    else if constexpr (std::is_same_v<T, float>) b = __float2bfloat16_rn(v);
+    else b = v;
+    reinterpret_cast<bf16*>(chunk)[o] = b;
+  } else {
+    float h;
+    unsigned short lo = 0;
+    if constexpr (std::is_same_v<T, double>) {
+      uint32_t hb;
+      if (ST == FVG_SPLIT && split_bits((uint64_t)__double_as_longlong(v), &hb, &lo)) {
+        h = __uint_as_float(hb);
+      } else {
+        h = (float)v;
+        if (ST == FVG_SPLIT) lo = __bfloat16_as_ushort(__double2bfloat16(isinf(h) ? 0.0 : v - (double)h));
       }
-      if (ST == FVG_BF16) reinterpret_cast<uint2*>(r)[lane] = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
-      else reinterpret_cast<float4*>(r)[lane] = make_float4(v[0], v[1], v[2], v[3]);
-      if (ST == FVG_SPLIT)
-        reinterpret_cast<uint2*>(r + R::kValB)[lane] = make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
-      reinterpret_cast<uint2*>(r + R::kValB + R::kLoB)[lane] = make_uint2(q[0] | (q[1] << 16), q[2] | (q[3] << 16));
+    } else {
+      h = (float)v;
+    }
+    reinterpret_cast<float*>(chunk)[o] = h;
+    if (ST == FVG_SPLIT) reinterpret_cast<unsigned short*>(chunk + R::kValB)[o] = lo;
+  }
+  reinterpret_cast<unsigned short*>(chunk + R::kValB + R::kLoB)[o] = (unsigned short)slot;
+}
+
+// where the segments' records are
+struct RecAt {
+  const i32* coff;  // first chunk of each slice
+  const i32* voff;  // first segment of each panel row
+  const i32* spos;  // slice * 32 + lane of each segment
+  unsigned char* rec;
+};
+
+// row panels: a warp per panel row, a segment after the other
+template <int ST, class T>
+__global__ void k_panel_records(const i32* __restrict__ B, const i32* __restrict__ tidx, const T* __restrict__ tval,
+                                i64 nhot, i64 np, i64 rows, const RecAt at) {
+  const int lane = threadIdx.x & 31;
+  PWARP_STRIDE(q, np * nhot) {
+    const i64 p = q / nhot, h = q - p * nhot;
+    const i64 s = B[h * (np + 1) + p];
+    const i32 len = (i32)(B[h * (np + 1) + p + 1] - s);
+    const i32 v0 = at.voff[q], n = at.voff[q + 1] - v0;
+    for (i32 j = 0; j < n; j++) {
+      i32 c0, c1;
+      seg_chunks(len, j, n, c0, c1);
+      const i32 pos = at.spos[v0 + j];
+      unsigned char* first = at.rec + (i64)at.coff[pos >> 5] * StreamRec<ST>::kB;
+      const i32 k1 = min(4 * c1, len);
+      for (i32 k = 4 * c0 + lane; k < k1; k += 32)
+        put_entry<ST, T>(first + (i64)((k >> 2) - c0) * StreamRec<ST>::kB, pos & 31, k & 3, tval[s + k],
+                         (unsigned)(tidx[s + k] - p * rows));
+    }
+  }
+}
+
+// forward head: a warp per row of A, its entries in head columns
+template <int ST, class T>
+__global__ void k_head_records(const i32* __restrict__ off, const i32* __restrict__ idx, const T* __restrict__ val,
+                               i64 m, const i32* __restrict__ slot, const i32* __restrict__ poff, const RecAt at) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  PWARP_STRIDE(r, m) {
+    const i64 s0 = off[r], e0 = off[r + 1];
+    const i32 len = poff[r + 1] - poff[r], v0 = at.voff[r], n = at.voff[r + 1] - v0;
+    const i64 c = (len + 3) / 4;
+    i32 k0 = 0;
+    for (i64 b = s0; b < e0; b += 32) {
+      const i64 e = b + lane;
+      const i32 sl = e < e0 ? slot[idx[e]] : -1;
+      const unsigned hb = __ballot_sync(0xffffffffu, sl >= 0);
+      if (sl >= 0) {
+        const i32 k = k0 + __popc(hb & lt), ck = k >> 2;
+        i32 j = 0, c0 = 0, c1;
+        if (n > 1) {
+          j = (i32)(((i64)(ck + 1) * n - 1) / c);  // the last segment that starts at or before chunk ck
+          seg_chunks(len, j, n, c0, c1);
+        }
+        const i32 pos = at.spos[v0 + j];
+        put_entry<ST, T>(at.rec + ((i64)at.coff[pos >> 5] + ck - c0) * StreamRec<ST>::kB, pos & 31, k & 3, val[e],
+                         (unsigned)sl);
+      }
+      k0 += __popc(hb);
     }
   }
 }
@@ -915,19 +960,13 @@ SidePlanes side_planes(fvg_ctx* c, const DBuf* src, const DBuf& slo, int master,
 }
 
 template <class T>
-void fill_planes(fvg_ctx* c, const DevCRS& at, DevPanels& pn, const i32* B, const i64* poff64, const i64* flag,
-                 const i64* coff) {
-  const T* tv = at.val[pn.master].as<T>();
-  const SidePlanes spp = side_planes(c, at.val, at.lo, pn.master, pn.val, pn.lo, pn.E);
-  const SidePlanes spc = side_planes(c, at.val, at.lo, pn.master, pn.cold.val, pn.cold.lo, pn.cold.nnz);
-  k_panel_fill<T><<<grid_n(32 * pn.npanels * pn.nhot), 256, 0, c->stream>>>(
-      B, poff64, at.idx.as<i32>(), tv, pn.nhot, pn.npanels, pn.rows, pn.prow.as<uint16_t>(), pn.val[pn.master].as<T>(),
-      spp);
-  check_launch("panel_fill");
-  k_cold_fill<T><<<grid_n(32 * pn.n), 256, 0, c->stream>>>(at.off.as<i32>(), flag, coff, pn.n, at.idx.as<i32>(), tv,
-                                                           pn.cold.idx.as<i32>(), pn.cold.val[pn.master].as<T>(), spc);
+void fill_cold(fvg_ctx* c, const DevCRS& at, DevPanels& pn, const i64* flag, const i64* coff) {
+  const SidePlanes sp = side_planes(c, at.val, at.lo, pn.master, pn.cold.val, pn.cold.lo, pn.cold.nnz);
+  k_cold_fill<T><<<grid_n(32 * pn.n), 256, 0, c->stream>>>(at.off.as<i32>(), flag, coff, pn.n, at.idx.as<i32>(),
+                                                           at.val[pn.master].as<T>(), pn.cold.idx.as<i32>(),
+                                                           pn.cold.val[pn.master].as<T>(), sp);
   check_launch("cold_fill");
-  count_launch(c, 2);
+  count_launch(c);
 }
 
 }  // namespace
@@ -989,8 +1028,8 @@ void device_pack(fvg_ctx* c, const i32* off, i64 nrows, i64 chunk, i64 nchunks, 
 
 namespace {
 
-// The streamed layout of the packed panel rows (poff); false when it would
-// not fit its index types.
+// The streamed layout of the panel rows (poff: their entries' offsets); false
+// when it would not fit its index types.
 bool stream_layout(fvg_ctx* c, DevPanels& pn) {
   cudaStream_t st = c->stream;
   const i64 np = pn.npanels, nhot = pn.nhot, Q = np * nhot;
@@ -1003,6 +1042,8 @@ bool stream_layout(fvg_ctx* c, DevPanels& pn) {
   scan_i64(c, nv.as<i64>(), voff.as<i64>(), Q);
   scan_i64(c, lng.as<i64>(), lpos.as<i64>(), Q);
   scan_i64(c, lpcn.as<i64>(), lpc.as<i64>(), Q);
+  nv.release();
+  lpcn.release();
   // per panel: its first segment; per unit: its first long row
   pn.nunits = (np + pn.group - 1) / pn.group;
   DBuf pstart, ul;
@@ -1038,18 +1079,19 @@ bool stream_layout(fvg_ctx* c, DevPanels& pn) {
   sbase.alloc(sizeof(i64) * (np + 1), st);
   FVG_CUDA(cudaMemcpyAsync(sbase.p, sb.data(), sizeof(i64) * (np + 1), cudaMemcpyHostToDevice, st));
   pn.vout.alloc(sizeof(i32) * std::max<i64>(ns * 32, 1), st);
-  pn.vsrc.alloc(sizeof(i32) * std::max<i64>(ns * 32, 1), st);
-  pn.vlen.alloc(std::max<i64>(ns * 32, 1), st);
+  pn.spos.alloc(sizeof(i32) * std::max<i64>(V, 1), st);
   width.alloc(sizeof(i64) * std::max<i64>(ns, 1), st);
   coff.alloc(sizeof(i64) * (ns + 1), st);
   k_slices<<<grid_n(ns * 32), 256, 0, st>>>(poff, voff.as<i64>(), lpc.as<i64>(), ids.as<uint32_t>(), vq.as<i32>(),
                                             sbase.as<i64>(), pstart.as<i64>(), np, ns, pn.vout.as<i32>(),
-                                            pn.vsrc.as<i32>(), pn.vlen.as<unsigned char>(), width.as<i64>());
+                                            pn.spos.as<i32>(), width.as<i64>());
   check_launch("slices");
   scan_i64(c, width.as<i64>(), coff.as<i64>(), ns);
   FVG_CUDA(cudaMemcpyAsync(&pn.nchunks, coff.as<i64>() + ns, sizeof(i64), cudaMemcpyDeviceToHost, st));
   FVG_CUDA(cudaStreamSynchronize(st));
   if (pn.nchunks + ns >= (1ll << 31) - 1) return false;
+  pn.voff.alloc(sizeof(i32) * (Q + 1), st);
+  k_i64_to_i32<<<grid_n(Q + 1), 256, 0, st>>>(voff.as<i64>(), pn.voff.as<i32>(), Q + 1);
   pn.coff.alloc(sizeof(i32) * (ns + 1), st);
   k_i64_to_i32<<<grid_n(ns + 1), 256, 0, st>>>(coff.as<i64>(), pn.coff.as<i32>(), ns + 1);
   pn.ulong0.alloc(sizeof(i32) * (pn.nunits + 1), st);
@@ -1064,23 +1106,45 @@ bool stream_layout(fvg_ctx* c, DevPanels& pn) {
   k_warp_starts<<<grid_n(pn.nunits * (kStreamWarps + 1)), 256, 0, st>>>(pn.coff.as<i32>(), sbase.as<i64>(), pn.group,
                                                                         np, pn.nunits, pn.wstart.as<i32>());
   check_launch("stream_layout");
-  count_launch(c, 9);
+  count_launch(c, 10);
   FVG_CUDA(cudaStreamSynchronize(st));  // host values go out of scope
   return true;
 }
 
-// The records of a value storage, from the packed entries' planes.
-template <int ST> void fill_records(fvg_ctx* c, DevPanels& pn) {
-  DBuf rec;
-  rec.alloc((size_t)(pn.nchunks + kStreamChunks) * StreamRec<ST>::kB, c->stream);  // a copy may read past the last
-  FVG_CUDA(cudaMemsetAsync(rec.as<unsigned char>() + (size_t)pn.nchunks * StreamRec<ST>::kB, 0,
-                           (size_t)kStreamChunks * StreamRec<ST>::kB, c->stream));
-  k_fill_records<ST><<<grid_n(32 * std::max<i64>(pn.nslices, 1)), 256, 0, c->stream>>>(
-      pn.coff.as<i32>(), pn.vsrc.as<i32>(), pn.vlen.as<unsigned char>(), pn.nslices, pn.prow.as<uint16_t>(),
-      pn.val[FVG_F32].as<float>(), pn.val[FVG_BF16].as<unsigned short>(), pn.lo.as<unsigned short>(),
-      (unsigned)pn.rows, rec.as<unsigned char>());
+// The records of a value storage, from the matrix's own values.
+template <int ST> void fill_records(fvg_ctx* c, fvg_matrix* M, DevPanels& pn) {
+  DBuf rec, slot;
+  const i64 nrec = pn.nchunks + kStreamChunks;  // a copy may read past the last
+  rec.alloc((size_t)nrec * StreamRec<ST>::kB, c->stream);
+  k_blank_records<ST><<<grid_n(nrec * (StreamRec<ST>::kB / 16)), 256, 0, c->stream>>>(rec.as<unsigned char>(), nrec,
+                                                                                     (unsigned)pn.rows);
+  check_launch("blank_records");
+  if (pn.shared) {  // column -> slot
+    slot.alloc(sizeof(i32) * pn.n, c->stream);
+    fill_i32(c, slot.as<i32>(), -1, pn.n);
+    k_head_slots<<<grid_n(pn.rows), 256, 0, c->stream>>>(pn.hot_cols.as<uint32_t>(), pn.rows, slot.as<i32>());
+    check_launch("head_slots");
+    count_launch(c);
+  }
+  const RecAt at{pn.coff.as<i32>(), pn.voff.as<i32>(), pn.spos.as<i32>(), rec.as<unsigned char>()};
+  auto fill = [&](auto tag) {
+    using T = decltype(tag);
+    if (pn.shared) {
+      const DevCRS& a = M->A;
+      k_head_records<ST, T><<<grid_n(32 * a.m), 256, 0, c->stream>>>(a.off.as<i32>(), a.idx.as<i32>(),
+                                                                    a.val[pn.master].as<T>(), a.m, slot.as<i32>(),
+                                                                    pn.poff.as<i32>(), at);
+    } else {
+      const DevCRS& t = *M->AT;
+      k_panel_records<ST, T><<<grid_n(32 * pn.npanels * pn.nhot), 256, 0, c->stream>>>(
+          pn.src.as<i32>(), t.idx.as<i32>(), t.val[pn.master].as<T>(), pn.nhot, pn.npanels, pn.rows, at);
+    }
+  };
+  if (pn.master == FVG_F64) fill(double{});
+  else if (pn.master == FVG_F32) fill(float{});
+  else fill(bf16{});
   check_launch("fill_records");
-  count_launch(c);
+  count_launch(c, 2);
   pn.rec[ST] = std::move(rec);
 }
 
@@ -1180,15 +1244,16 @@ std::unique_ptr<DevPanels> panel_build(fvg_ctx* c, const DevCRS& at, int master,
   check_launch("hot_list");
   count_launch(c);
   // per (panel, hot column) ranges and their offsets
-  DBuf B, len, poff64;
-  B.alloc(sizeof(i32) * nhot * (np + 1), c->stream);
+  DBuf len, poff64;
+  pn->src.alloc(sizeof(i32) * nhot * (np + 1), c->stream);
+  i32* const B = pn->src.as<i32>();
   k_panel_bounds<<<grid_n(nhot * (np + 1)), 256, 0, c->stream>>>(at.off.as<i32>(), at.idx.as<i32>(),
-                                                                  pn->hot_cols.as<i32>(), nhot, np, rows, B.as<i32>());
+                                                                  pn->hot_cols.as<i32>(), nhot, np, rows, B);
   check_launch("panel_bounds");
   const i64 Q = np * nhot;
   len.alloc(sizeof(i64) * Q, c->stream);
   poff64.alloc(sizeof(i64) * (Q + 1), c->stream);
-  k_panel_lens<<<grid_n(Q), 256, 0, c->stream>>>(B.as<i32>(), nhot, np, len.as<i64>());
+  k_panel_lens<<<grid_n(Q), 256, 0, c->stream>>>(B, nhot, np, len.as<i64>());
   check_launch("panel_lens");
   count_launch(c, 2);
   scan_i64(c, len.as<i64>(), poff64.as<i64>(), Q);
@@ -1201,8 +1266,8 @@ std::unique_ptr<DevPanels> panel_build(fvg_ctx* c, const DevCRS& at, int master,
   k_i64_to_i32<<<grid_n(Q + 1), 256, 0, c->stream>>>(poff64.as<i64>(), pn->poff.as<i32>(), Q + 1);
   check_launch("poff");
   count_launch(c);
-  alloc_padded(c, pn->prow, E, 2);
-  alloc_padded(c, pn->val[master], E, dtype_size(master));
+  len.release();
+  poff64.release();
   // cold columns: A^T with the hot rows emptied
   DevCRS& cold = pn->cold;
   cold.m = n;
@@ -1222,11 +1287,12 @@ std::unique_ptr<DevPanels> panel_build(fvg_ctx* c, const DevCRS& at, int master,
   count_launch(c);
   alloc_padded(c, cold.idx, cold.nnz, 4);
   alloc_padded(c, cold.val[master], cold.nnz, dtype_size(master));
-  if (master == FVG_F64) fill_planes<double>(c, at, *pn, B.as<i32>(), poff64.as<i64>(), flag.as<i64>(), coff64.as<i64>());
-  else if (master == FVG_F32) fill_planes<float>(c, at, *pn, B.as<i32>(), poff64.as<i64>(), flag.as<i64>(), coff64.as<i64>());
-  else fill_planes<bf16>(c, at, *pn, B.as<i32>(), poff64.as<i64>(), flag.as<i64>(), coff64.as<i64>());
+  if (master == FVG_F64) fill_cold<double>(c, at, *pn, flag.as<i64>(), coff64.as<i64>());
+  else if (master == FVG_F32) fill_cold<float>(c, at, *pn, flag.as<i64>(), coff64.as<i64>());
+  else fill_cold<bf16>(c, at, *pn, flag.as<i64>(), coff64.as<i64>());
   cold.max_row = 0;  // not used by the product
   if (!stream_layout(c, *pn)) return nullptr;
+  pn->poff.release();  // the records are filled by src
   FVG_CUDA(cudaStreamSynchronize(c->stream));  // host vectors go out of scope
   return pn;
 }
@@ -1297,8 +1363,6 @@ std::unique_ptr<DevPanels> head_build(fvg_ctx* c, const DevCRS& a, const DevCRS&
   k_head_off<<<grid_n(Q + 1), 256, 0, c->stream>>>(hoff.as<i64>(), m, Q, hd->poff.as<i32>());
   check_launch("head_off");
   count_launch(c);
-  alloc_padded(c, hd->prow, hd->E, 2);
-  alloc_padded(c, hd->val[master], hd->E, dtype_size(master));
   DevCRS& tail = hd->cold;
   tail.m = m;
   tail.n = n;
@@ -1309,14 +1373,13 @@ std::unique_ptr<DevPanels> head_build(fvg_ctx* c, const DevCRS& a, const DevCRS&
   count_launch(c);
   alloc_padded(c, tail.idx, tail.nnz, 4);
   alloc_padded(c, tail.val[master], tail.nnz, dtype_size(master));
-  const SidePlanes sph = side_planes(c, a.val, a.lo, master, hd->val, hd->lo, hd->E);
   const SidePlanes spt = side_planes(c, a.val, a.lo, master, tail.val, tail.lo, tail.nnz);
   auto fill = [&](auto tag) {
     using T = decltype(tag);
-    k_head_fill<T><<<grid_n(32 * m), 256, 0, c->stream>>>(
-        a.off.as<i32>(), a.idx.as<i32>(), a.val[master].as<T>(), m, dslot.as<i32>(), hoff.as<i64>(), tof.as<i64>(),
-        hd->prow.as<uint16_t>(), hd->val[master].as<T>(), tail.idx.as<i32>(), tail.val[master].as<T>(), sph, spt);
-    check_launch("head_fill");
+    k_tail_fill<T><<<grid_n(32 * m), 256, 0, c->stream>>>(a.off.as<i32>(), a.idx.as<i32>(), a.val[master].as<T>(), m,
+                                                         dslot.as<i32>(), tof.as<i64>(), tail.idx.as<i32>(),
+                                                         tail.val[master].as<T>(), spt);
+    check_launch("tail_fill");
     count_launch(c);
   };
   if (master == FVG_F64) fill(double{});
@@ -1343,12 +1406,10 @@ DevPanels* panels_for(fvg_ctx* c, fvg_matrix* M) {
   return M->pan.get();
 }
 
-void panel_ensure_plane(fvg_ctx* c, DevPanels& pn, int dt) {
+void panel_ensure_plane(fvg_ctx* c, fvg_matrix* M, DevPanels& pn, int dt) {
   if (!pn.rec[dt].p) {
-    ensure_plane_generic(c, pn.val, pn.E, dt, pn.master);
-    if (dt == FVG_F32) fill_records<FVG_F32>(c, pn);
-    else fill_records<FVG_BF16>(c, pn);
-    if (dt != pn.master) pn.val[dt].release();  // the records hold them
+    if (dt == FVG_F32) fill_records<FVG_F32>(c, M, pn);
+    else fill_records<FVG_BF16>(c, M, pn);
   }
   sum_buffers(c, pn, pn.ypan, pn.partials, sizeof(float));
   crs_ensure_plane(c, pn.cold, dt, pn.master);
@@ -1361,7 +1422,6 @@ void panel_trans_mv(fvg_ctx* c, DevPanels& pn, int storage, const float* r, int 
                     int prof_key) {
   if (storage == FVG_F64) fail(FVG_ERR_INTERNAL, "the panel product runs on FP32 or BF16 values");
   if (y_dt != FVG_F64 && y_dt != FVG_F32) fail(FVG_ERR_INTERNAL, "panel product output must be FP64 or FP32");
-  panel_ensure_plane(c, pn, storage);
   ProfScope pr(c, prof_key);
   // cold columns (and zeros for the hot ones) by the transposed CRS kernel
   crs_pass(c, pn.cold, storage, FVG_F32, r, y_dt, y, EPI_STORE, nullptr, scratch, P_NKEYS);
@@ -1394,14 +1454,11 @@ DevPanels* head_for(fvg_ctx* c, fvg_matrix* M) {
   return M->head.get();
 }
 
-void head_ensure_plane(fvg_ctx* c, DevPanels& hd, int dt) { panel_ensure_plane(c, hd, dt); }
-
 i64 head_scratch_bytes(fvg_ctx* c, DevPanels& hd, int storage) { return crs_pass_scratch_bytes(c, hd.cold, storage); }
 
 void head_logreg_pass(fvg_ctx* c, DevPanels& hd, int storage, const float* w, const LogregEpi& lr, void* scratch,
                       int prof_key) {
   if (storage == FVG_F64) fail(FVG_ERR_INTERNAL, "the head pass runs on FP32 or BF16 values");
-  head_ensure_plane(c, hd, storage);
   ProfScope pr(c, prof_key);
   if (storage == FVG_F32) launch_stream<FVG_F32>(c, hd, w, hd.ypan.p, hd.partials.p);
   else launch_stream<FVG_BF16>(c, hd, w, hd.ypan.p, hd.partials.p);
@@ -1415,13 +1472,8 @@ void head_logreg_pass(fvg_ctx* c, DevPanels& hd, int storage, const float* w, co
 // ------------------------------------------------------------ split storage
 namespace fvg {
 
-void panel_ensure_split(fvg_ctx* c, DevPanels& pn) {
-  if (!pn.rec[FVG_SPLIT].p) {
-    ensure_split_planes(c, pn.val, pn.E, pn.master, pn.lo);
-    fill_records<FVG_SPLIT>(c, pn);
-    if (pn.master != FVG_F32) pn.val[FVG_F32].release();  // the records hold both
-    pn.lo.release();
-  }
+void panel_ensure_split(fvg_ctx* c, fvg_matrix* M, DevPanels& pn) {
+  if (!pn.rec[FVG_SPLIT].p) fill_records<FVG_SPLIT>(c, M, pn);
   crs_ensure_split(c, pn.cold, pn.master);
   sum_buffers(c, pn, pn.ypan2, pn.partials2, sizeof(float2));
 }
@@ -1431,7 +1483,6 @@ i64 panel_split_scratch_bytes(fvg_ctx* c, DevPanels& pn, bool y_df) {
 }
 
 void panel_trans_mv_split(fvg_ctx* c, DevPanels& pn, const void* r, double* y, void* scratch) {
-  panel_ensure_split(c, pn);
   // cold columns (and zeros for the hot ones) by the transposed CRS kernel
   crs_pass_split(c, pn.cold, r, false, y, scratch, P_NKEYS);
   launch_stream<FVG_SPLIT>(c, pn, r, pn.ypan2.p, pn.partials2.p);
@@ -1443,7 +1494,6 @@ void panel_trans_mv_split(fvg_ctx* c, DevPanels& pn, const void* r, double* y, v
 }
 
 void head_pass_split(fvg_ctx* c, DevPanels& hd, const void* w, void* wtx, void* scratch) {
-  panel_ensure_split(c, hd);
   launch_stream<FVG_SPLIT>(c, hd, w, hd.ypan2.p, hd.partials2.p);
   crs_pass_split(c, hd.cold, w, true, wtx, scratch, P_NKEYS);
 }
