@@ -304,18 +304,23 @@ FVG_API fvg_status fvg_matrix_prepare(fvg_ctx* c, fvg_matrix* M, fvg_format fmt,
   API_BEGIN
   own(c, M);
   prepare(c, M, fmt, with_transpose != 0);
-  if (with_transpose && M->A.lo.p && M->AT) crs_ensure_split(c, *M->AT, M->master);
+  if (with_transpose && M->AT) {  // the transposed copy's planes beside A's
+    if (M->A.lo.p) crs_ensure_split(c, *M->AT, M->master);
+    for (int dt : {FVG_F32, FVG_BF16})
+      if (M->A.val[dt].p) crs_ensure_plane(c, *M->AT, dt, M->master);
+  }
   // a matrix that already holds FP32 / BF16 values gets its row-panel
   // backward layout and its forward head now rather than at the first product
   if (with_transpose && (fmt == FVG_CRS || fmt == FVG_ELL) && (M->A.val[FVG_F32].p || M->A.val[FVG_BF16].p)) {
     DevPanels* pt = panels_for(c, M);
     DevPanels* hd = fmt == FVG_CRS ? head_for(c, M) : nullptr;
-    const bool split = M->A.lo.p != nullptr;  // its FP32 plane belongs to the split values
+    // beside split values an FP32 plane may be there for them alone
+    const bool split = M->A.lo.p != nullptr, f32 = !split || M->wants_f32 || M->master == FVG_F32;
     for (DevPanels* p : {pt, hd}) {
       if (!p) continue;
       if (split) panel_ensure_split(c, M, *p);
       for (int dt : {FVG_F32, FVG_BF16})
-        if (M->A.val[dt].p && !(split && dt == FVG_F32)) panel_ensure_plane(c, M, *p, dt);
+        if (M->A.val[dt].p && (dt != FVG_F32 || f32)) panel_ensure_plane(c, M, *p, dt);
     }
   }
   FVG_CUDA(cudaStreamSynchronize(c->stream));
@@ -410,6 +415,7 @@ FVG_API fvg_status fvg_matrix_add_storage(fvg_ctx* c, fvg_matrix* M, fvg_dtype s
   own(c, M);
   need(storage >= FVG_F64 && storage <= FVG_SPLIT, FVG_ERR_INVALID_ARG, "unknown storage dtype");
   ensure_plane_all(c, M, storage);
+  if (storage == FVG_F32) M->wants_f32 = true;
   FVG_CUDA(cudaStreamSynchronize(c->stream));
   API_END(c)
 }

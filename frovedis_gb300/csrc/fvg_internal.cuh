@@ -249,6 +249,7 @@ struct fvg_ctx {
 struct fvg_matrix {
   fvg_ctx* ctx = nullptr;
   int master = FVG_F64;           // dtype of the uploaded values
+  bool wants_f32 = false;         // FP32 products were asked for (beside split values, which hold an FP32 plane too)
   fvg::DevCRS A;
   std::unique_ptr<fvg::DevCRS> AT;
   std::unique_ptr<fvg::DevELL> ell;
