@@ -36,7 +36,16 @@ void ensure_plane_generic(fvg_ctx* c, DBuf* planes, i64 n, int dt, int master) {
   convert_values(c, planes[master].p, master, planes[dt].p, dt, n);
 }
 
-void crs_ensure_plane(fvg_ctx* c, DevCRS& a, int dt, int master) { ensure_plane_generic(c, a.val, a.nnz, dt, master); }
+// A matrix with work items for one storage keeps them for every storage it
+// has values of: what a product without allocations relies on.
+void crs_plane_added(fvg_ctx* c, DevCRS& a, int dt) {
+  if (a.sched[0] || a.sched[2]) pass_sched(c, a, dt);
+}
+
+void crs_ensure_plane(fvg_ctx* c, DevCRS& a, int dt, int master) {
+  ensure_plane_generic(c, a.val, a.nnz, dt, master);
+  crs_plane_added(c, a, dt);
+}
 
 // ------------------------------------------------------------------ upload
 // Counts and the longest row are combined per warp first: one atomic per

@@ -396,9 +396,6 @@ static void ensure_plane_all(fvg_ctx* c, fvg_matrix* M, int dt) {
   }
   crs_ensure_plane(c, M->A, dt, M->master);
   if (M->AT) crs_ensure_plane(c, *M->AT, dt, M->master);
-  // a matrix prepared before it had this plane: its schedule too
-  for (DevCRS* a : {&M->A, M->AT.get()})
-    if (a && (a->sched[0] || a->sched[2])) pass_sched(c, *a, dt);
   if (M->ell) ensure_plane_generic(c, M->ell->val, M->ell->m * M->ell->width, dt, M->master);
   for (DevJDS* j : {M->jds.get(), M->tjds.get()})
     if (j) ensure_plane_generic(c, j->val, j->nnz, dt, M->master);

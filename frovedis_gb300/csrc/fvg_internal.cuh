@@ -326,6 +326,7 @@ void gather_values(fvg_ctx* c, const void* src, const uint32_t* perm, void* dst,
 void crs_upload(fvg_ctx* c, DevCRS& a, i64 m, i64 n, const i32* off, const i32* idx, const void* val, int dt,
                 bool on_device);
 void crs_ensure_plane(fvg_ctx* c, DevCRS& a, int dt, int master);
+void crs_plane_added(fvg_ctx* c, DevCRS& a, int dt);  // after a's values of storage dt were made
 void crs_build_transpose(fvg_ctx* c, const DevCRS& a, DevCRS& t, int master);
 const Sched& crs_sched(fvg_ctx* c, DevCRS& a, int tile);
 const Sched& crs_sched64(fvg_ctx* c, DevCRS& a);  // the FP64 kernel's items (slot 2)

@@ -444,7 +444,10 @@ void ensure_split_planes(fvg_ctx* c, DBuf* planes, i64 n, int master, DBuf& lo) 
   if (!lo.p) split_residual_plane(c, planes, n, master, lo);
 }
 
-void crs_ensure_split(fvg_ctx* c, DevCRS& a, int master) { ensure_split_planes(c, a.val, a.nnz, master, a.lo); }
+void crs_ensure_split(fvg_ctx* c, DevCRS& a, int master) {
+  ensure_split_planes(c, a.val, a.nnz, master, a.lo);
+  crs_plane_added(c, a, FVG_F32);
+}
 
 void split_vector(fvg_ctx* c, const double* x, void* y, i64 n) {
   if (n <= 0) return;

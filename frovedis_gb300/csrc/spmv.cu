@@ -750,7 +750,10 @@ void crs_pass(fvg_ctx* c, DevCRS& a, int storage, int x_dt, const void* x, int y
 // Returns the scratch bytes the pass needs when scratch is null.
 size_t crs_spmv_no_alloc(fvg_ctx* c, DevCRS& a, int storage, const void* x, void* y, void* scratch,
                          size_t scratch_bytes) {
-  const Sched* s = a.sched[storage == FVG_F64 ? 2 : 0].get();
+  // its own work items; where another storage's first use made the matrix's
+  // only ones, those (both kernels take either list)
+  const int own = storage == FVG_F64 ? 2 : 0;
+  const Sched* s = a.sched[a.sched[own] ? own : 2 - own].get();
   if (!s) fail(FVG_ERR_INVALID_ARG, "matrix not prepared: call fvg_matrix_prepare(ctx, mat, FVG_CRS, ...) first");
   if (!a.val[storage].p) fail(FVG_ERR_INVALID_ARG, "value plane missing: call fvg_matrix_add_storage first");
   const size_t at_size = (storage == FVG_F64) ? 8 : 4;
