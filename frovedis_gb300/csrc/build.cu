@@ -298,8 +298,8 @@ __global__ void k_gather_items(const Item* __restrict__ src, const uint32_t* __r
 }
 
 const Sched& crs_sched_slabs(fvg_ctx* c, DevCRS& a, int storage, i64 slab) {
-  if (a.slab_sched && a.slab_rows == slab) return *a.slab_sched;
   const Sched& s0 = pass_sched(c, a, storage);
+  if (a.slab_sched && a.slab_rows == slab && a.slab_of == &s0) return *a.slab_sched;
   const int tile = s0.tile;
   ProfScope ps(c, P_SCHED);
   auto s = std::make_unique<Sched>();
@@ -366,6 +366,7 @@ const Sched& crs_sched_slabs(fvg_ctx* c, DevCRS& a, int storage, i64 slab) {
   FVG_CUDA(cudaStreamSynchronize(st));  // host vectors go out of scope
   a.slab_sched = std::move(s);
   a.slab_rows = slab;
+  a.slab_of = &s0;
   return *a.slab_sched;
 }
 

@@ -123,6 +123,7 @@ struct DevCRS {
   std::unique_ptr<Sched> sched[3];
   std::unique_ptr<Sched> slab_sched;  // long rows in slab-ordered pieces (crs_sched_slabs)
   i64 slab_rows = 0;
+  const Sched* slab_of = nullptr;  // of which of sched[] its tiles are
   i64 max_row = 0;
 };
 
