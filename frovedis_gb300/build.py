@@ -31,8 +31,8 @@ def nvcc() -> str:
 
 def _deps():
     files = [os.path.join(CSRC, s) for s in SOURCES]
-    files += [os.path.join(CSRC, "fvg_internal.cuh"), os.path.join(CSRC, "device_common.cuh"), os.path.join(CSRC, "df64.cuh"), os.path.join(CSRC, "logistic64.cuh"), os.path.join(INCLUDE, "fvg.h"), __file__]
-    return files
+    files += [os.path.join(CSRC, f) for f in sorted(os.listdir(CSRC)) if f.endswith((".cuh", ".h"))]
+    return files + [os.path.join(INCLUDE, "fvg.h"), __file__]
 
 
 def up_to_date() -> bool:
