@@ -62,8 +62,17 @@ unsigned grid_n(i64 n, int threads = 256) {
        q += ((i64)gridDim.x * blockDim.x) >> 5)
 
 constexpr i64 kPanelMinRows = 4096;      // auto: shortest panels
-constexpr i64 kPanelMinMatrix = 76800;   // auto: rows of a matrix that gets panels
-constexpr i64 kHeadMinMatrix = 311296;   // auto: rows of a matrix that gets a head
+// auto: rows of a matrix that gets panels, 22 of the shortest.  A^T x, 50
+// entries a row, BF16 values: the plain product takes 31 us at 89,000 rows, the
+// panels 60; 46 and 65 at 200,000; 71 and 70 at 400,000; 153 and 104 at
+// 1,000,000.  Between the line and 400,000 rows the panels are there for their
+// error: 6e-8 to 9e-8 of the 64-bit product, 9e-8 to 1.3e-7 without.
+constexpr i64 kPanelMinMatrix = 22 * kPanelMinRows;
+// auto: rows per SM of a matrix that gets a head.  A w and the loss rows, 50
+// entries a row, with / without: BF16 values 40 / 34 us at 100,000 rows, 54 / 53
+// at 300,000, 60 / 67 at 450,000, 73 / 92 at 700,000; split values 39 / 38, 67 /
+// 76, 80 / 105 and 106 / 153.
+constexpr i64 kHeadMinPerSm = 2048;
 constexpr double kPanelMinAuto = 2.0;    // hot: >= this many entries per panel on average
 
 // ------------------------------------------------------------------ build
@@ -1349,7 +1358,7 @@ std::unique_ptr<DevPanels> head_build(fvg_ctx* c, const DevCRS& a, const DevCRS&
   if (forced && force_cols > cap)
     fail(FVG_ERR_INVALID_ARG, "head columns must be at most " + std::to_string(cap));
   const i64 grid = c->num_sms;  // one CTA (one stretch of rows) per SM
-  if (!forced && m < kHeadMinMatrix) return nullptr;
+  if (!forced && m < kHeadMinPerSm * grid) return nullptr;
   const i64 H = std::min<i64>(n, forced ? force_cols : cap);
   // the H largest column counts (from the transposed offsets), on the
   // device: a stable sort of the columns by decreasing count (ties keep
