@@ -143,8 +143,7 @@ constexpr int kColGroup = 32;
 
 // v[] of the CTA's rows -> sm[q][threadIdx.x] of the threads with rr == 0
 template <int NV>
-__device__ __forceinline__ void col_fold(const double (&v)[NV], const bool (&is_max)[NV], const BArgs& a, int rr,
-                                         double (&sm)[NV][kBT]) {
+__device__ __forceinline__ void col_fold(const double (&v)[NV], const BArgs& a, int rr, double (&sm)[NV][kBT]) {
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < NV; q++) sm[q][threadIdx.x] = v[q];
@@ -152,10 +151,7 @@ __device__ __forceinline__ void col_fold(const double (&v)[NV], const bool (&is_
   for (int s = a.rpb / 2; s > 0; s >>= 1) {
     if (rr < s)
 #pragma unroll
-      for (int q = 0; q < NV; q++) {
-        const double o = sm[q][threadIdx.x + s * a.kp];
-        sm[q][threadIdx.x] = is_max[q] ? fmax(sm[q][threadIdx.x], o) : sm[q][threadIdx.x] + o;
-      }
+      for (int q = 0; q < NV; q++) sm[q][threadIdx.x] += sm[q][threadIdx.x + s * a.kp];
     __syncthreads();
   }
 }
@@ -163,7 +159,7 @@ __device__ __forceinline__ void col_fold(const double (&v)[NV], const bool (&is_
 // `cnt` partials from `part`, in order; eight loads issued before they are
 // combined
 template <int NV>
-__device__ __forceinline__ void col_gather(double (&t)[NV], const bool (&is_max)[NV], const BArgs& a, int rr, int j,
+__device__ __forceinline__ void col_gather(double (&t)[NV], const BArgs& a, int rr, int j,
                                            const double* part, int cnt) {
 #pragma unroll
   for (int q = 0; q < NV; q++) t[q] = 0.0;
@@ -179,7 +175,7 @@ __device__ __forceinline__ void col_gather(double (&t)[NV], const bool (&is_max)
 #pragma unroll
     for (int u = 0; u < U; u++)
 #pragma unroll
-      for (int q = 0; q < NV; q++) t[q] = is_max[q] ? fmax(t[q], x[u][q]) : t[q] + x[u][q];
+      for (int q = 0; q < NV; q++) t[q] += x[u][q];
   }
 }
 
@@ -199,7 +195,7 @@ __device__ __forceinline__ bool col_last(unsigned* ticket, int cnt) {
 }
 
 template <int NV, class Fin>
-__device__ __forceinline__ void col_reduce(double (&v)[NV], const bool (&is_max)[NV], const BArgs& a, Fin fin) {
+__device__ __forceinline__ void col_reduce(double (&v)[NV], const BArgs& a, Fin fin) {
   __shared__ double sm[NV][kBT];
   const int j = threadIdx.x % a.kp, rr = threadIdx.x / a.kp;
   const bool mine = rr == 0 && j < a.k;
@@ -213,17 +209,17 @@ __device__ __forceinline__ void col_reduce(double (&v)[NV], const bool (&is_max)
 #pragma unroll
       for (int q = 0; q < NV; q++) to[(i64)j * NV + q] = sm[q][threadIdx.x];
   };
-  col_fold<NV>(v, is_max, a, rr, sm);
+  col_fold<NV>(v, a, rr, sm);
   put(part + (i64)blockIdx.x * a.k * NV);
   const int b0 = grp * kColGroup, cnt = min(kColGroup, grid - b0);
   if (!col_last(ticket + 1 + grp, cnt)) return;
-  col_gather<NV>(v, is_max, a, rr, j, part + (i64)b0 * a.k * NV, cnt);
-  col_fold<NV>(v, is_max, a, rr, sm);
+  col_gather<NV>(v, a, rr, j, part + (i64)b0 * a.k * NV, cnt);
+  col_fold<NV>(v, a, rr, sm);
   if (ng > 1) {
     put(gpart + (i64)grp * a.k * NV);
     if (!col_last(ticket, ng)) return;
-    col_gather<NV>(v, is_max, a, rr, j, gpart, ng);
-    col_fold<NV>(v, is_max, a, rr, sm);
+    col_gather<NV>(v, a, rr, j, gpart, ng);
+    col_fold<NV>(v, a, rr, sm);
   }
   if (mine) {
     double tot[NV];
@@ -305,8 +301,7 @@ __global__ void __launch_bounds__(kBT, 4) kb_down(int i, int kh, int rear, const
                               Q[e0 + r * ld] = q;
                               v[0] += x.c * q;
                             });
-  const bool mx[1] = {false};
-  col_reduce<1>(v, mx, a, [&](int c, double* t) {
+  col_reduce<1>(v, a, [&](int c, double* t) {
     ColState& s = a.st[ds * ld + c];
     if (s.active) s.al[i] = s.rho[hslot(rear, i, a.h)] * t[0];
   });
@@ -350,8 +345,7 @@ __global__ void __launch_bounds__(kBT, 4) kb_up(int i, int kh, int rear, const d
                               Z[e0 + r * ld] = z;
                               v[0] += x.c * z;
                             });
-  const bool mx[1] = {false};
-  col_reduce<1>(v, mx, a, [&](int c, double* t) {
+  col_reduce<1>(v, a, [&](int c, double* t) {
     ColState& s = a.st[ds * ld + c];
     if (s.active) s.beta[i] = s.rho[hslot(rear, i, a.h)] * t[0];
   });
@@ -390,8 +384,7 @@ __global__ void __launch_bounds__(kBT, 4) kb_step(int kh, int rear, const double
                               v[0] += x.a * st;
                               norm_add(v[1], v[2], v[3], st);
                             });
-  const bool mx[4] = {false, false, false, false};
-  col_reduce<4>(v, mx, a, [&](int c2, double* t) {
+  col_reduce<4>(v, a, [&](int c2, double* t) {
     ColState& s = a.st[ds * ld + c2];
     if (!s.active) return;
     const double ss = norm_of(t[1], t[2], t[3]);
@@ -447,8 +440,7 @@ __global__ void __launch_bounds__(kBT, 4) kb_gnorm(const double* __restrict__ G,
   if (use)
     rows_grouped<kRowGroup>(r0, rstep, n1, [&](i64 r) { return G[e0 + r * ld]; },
                             [&](i64, double x) { norm_add(v[0], v[1], v[2], x); });
-  const bool mx[3] = {false, false, false};
-  col_reduce<3>(v, mx, a, [&](int c, double* t) {
+  col_reduce<3>(v, a, [&](int c, double* t) {
     if (!model_on(a, ds, c)) return;
     const i64 mc = ds * ld + c;
     ColState& s = a.st[mc];
@@ -556,8 +548,7 @@ __global__ void __launch_bounds__(kBT, 4) kb_accept(int nf, int it, double tol, 
                       v[0] += s * y;
                       v[1] += y * y;
                     });
-  const bool mx[2] = {false, false};
-  col_reduce<2>(v, mx, a, [&](int c, double* t) {
+  col_reduce<2>(v, a, [&](int c, double* t) {
     const i64 mc = ds * ld + c;
     ColState& s = a.st[mc];
     if (!s.active) return;

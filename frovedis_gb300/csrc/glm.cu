@@ -49,23 +49,21 @@ struct VecArgs {
 
 __device__ __forceinline__ int slot(const LbState* st, int i) { return (st->rear + i) % st->h; }
 
-// Fixed-order grid reduction of NV values (sum or max per value); the last
-// CTA calls fin(totals) with thread 0.
+// Fixed-order grid reduction of NV sums; the last CTA calls fin(totals) with
+// thread 0.
 template <int NV, class Fin>
-__device__ __forceinline__ void grid_reduce(double (&v)[NV], const bool (&is_max)[NV], double* part,
-                                            unsigned* ticket, Fin fin) {
+__device__ __forceinline__ void grid_reduce(double (&v)[NV], double* part, unsigned* ticket, Fin fin) {
   constexpr unsigned kFull = 0xffffffffu;
   constexpr int kWarps = kVecThreads / 32;
   __shared__ double sm[NV][kWarps];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  auto join = [&](int q, double x, double y) { return is_max[q] ? fmax(x, y) : x + y; };
   // the CTA's total into every lane of warp 0
   auto cta = [&](double(&t)[NV]) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-      for (int q = 0; q < NV; q++) t[q] = join(q, t[q], __shfl_xor_sync(kFull, t[q], o));
+      for (int q = 0; q < NV; q++) t[q] += __shfl_xor_sync(kFull, t[q], o);
     if (lane == 0)
 #pragma unroll
       for (int q = 0; q < NV; q++) sm[q][w] = t[q];
@@ -76,7 +74,7 @@ __device__ __forceinline__ void grid_reduce(double (&v)[NV], const bool (&is_max
 #pragma unroll
     for (int o = kWarps / 2; o > 0; o >>= 1)
 #pragma unroll
-      for (int q = 0; q < NV; q++) t[q] = join(q, t[q], __shfl_xor_sync(kFull, t[q], o));
+      for (int q = 0; q < NV; q++) t[q] += __shfl_xor_sync(kFull, t[q], o);
   };
   cta(v);
   if (threadIdx.x == 0) {
@@ -93,7 +91,7 @@ __device__ __forceinline__ void grid_reduce(double (&v)[NV], const bool (&is_max
   for (int q = 0; q < NV; q++) t[q] = 0.0;
   for (i64 b = threadIdx.x; b < gridDim.x; b += kVecThreads)
 #pragma unroll
-    for (int q = 0; q < NV; q++) t[q] = join(q, t[q], __ldcg(&part[b * NV + q]));
+    for (int q = 0; q < NV; q++) t[q] += __ldcg(&part[b * NV + q]);
   cta(t);
   if (threadIdx.x == 0) {
     fin(t);
@@ -405,8 +403,7 @@ __global__ void __launch_bounds__(kVecThreads) k_gnorm(const double* __restrict_
   LbState* st = a.st;
   double v[3] = {0.0, 0.0, 0.0};
   VEC_LOOP(j, a.n1) norm_add(v[0], v[1], v[2], G[j]);
-  const bool mx[3] = {false, false, false};
-  grid_reduce<3>(v, mx, a.part, a.ticket, [&](double* t) {
+  grid_reduce<3>(v, a.part, a.ticket, [&](double* t) {
     const double nrm = norm_of(t[0], t[1], t[2]);
     st->gnorm_t = nrm;
     st->rms_t = nrm / sqrt((double)a.n1);
@@ -447,8 +444,7 @@ __global__ void __launch_bounds__(kVecThreads) k_accept(double* __restrict__ W, 
     v[0] += s * y;
     v[1] += y * y;
   }
-  const bool mx[2] = {false, false};
-  grid_reduce<2>(v, mx, a.part, a.ticket, [&](double* t) {
+  grid_reduce<2>(v, a.part, a.ticket, [&](double* t) {
     double dv = t[0];
     if (dv == 0) dv = 1;
     st->rho[nf] = 1.0 / dv;
@@ -1068,8 +1064,7 @@ __global__ void __launch_bounds__(kVecThreads) k_sgd_apply(double* __restrict__ 
     double df = a.used ? TOT[j] : prev - w;
     v[0] += df * df;
   }
-  const bool mx[1] = {false};
-  grid_reduce<1>(v, mx, a.part, a.ticket, [&](double* t) {
+  grid_reduce<1>(v, a.part, a.ticket, [&](double* t) {
     double pb = a.scal[1];
     double nb = __dadd_rn(pb, a.scal[3]);
     a.scal[1] = nb;

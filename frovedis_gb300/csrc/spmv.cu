@@ -35,7 +35,6 @@ struct CrsK {
   const void* x;
   const Item* items;
   i64 nitems;
-  int tile;
   void* y;
   void* partials;
   // logistic epilogue
@@ -47,7 +46,6 @@ struct CrsK {
   int icpt;
   void* r;
   double* cta_part;
-  unsigned* err;
   int loss;    // GLM loss kind
   double eps;  // its epsilon
   const float* ybase;  // FP32 path: per-row partial sums from another pass, added before the epilogue
@@ -552,8 +550,7 @@ static int fin_grid(fvg_ctx* c, const Sched& s) {
 }
 
 template <class VT, class XT, class AT, class YT, int EPI>
-static int crs_grid(fvg_ctx* c, int tile) {
-  (void)tile;
+static int crs_grid(fvg_ctx* c) {
   return occupancy_blocks((const void*)k_crs<VT, XT, AT, YT, EPI>, kThreads) * c->num_sms;
 }
 
@@ -567,7 +564,6 @@ static void launch_crs(fvg_ctx* c, DevCRS& a, const Sched& s, int storage, const
   p.x = x;
   p.items = s.items.as<Item>();
   p.nitems = s.nitems;
-  p.tile = s.tile;
   p.y = y;
   p.partials = ps.partials;
   p.label = lr ? lr->label : nullptr;
@@ -579,10 +575,9 @@ static void launch_crs(fvg_ctx* c, DevCRS& a, const Sched& s, int storage, const
   p.r = lr ? lr->r : nullptr;
   p.ybase = lr ? lr->ybase : nullptr;
   p.cta_part = ps.cta_part;
-  p.err = c->dev_err;
   p.loss = lr ? lr->loss : 0;
   p.eps = lr ? lr->eps : 0.0;
-  int grid = (int)std::max<i64>(1, std::min<i64>(crs_grid<VT, XT, AT, YT, EPI>(c, s.tile), s.nitems));
+  int grid = (int)std::max<i64>(1, std::min<i64>(crs_grid<VT, XT, AT, YT, EPI>(c), s.nitems));
   grid = std::min(grid, c->grid_spmv);
   if (s.nitems > 0) {
     k_crs<VT, XT, AT, YT, EPI><<<grid, kThreads, 0, c->stream>>>(p);
