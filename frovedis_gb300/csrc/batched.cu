@@ -156,8 +156,8 @@ __device__ __forceinline__ void col_fold(const double (&v)[NV], const BArgs& a, 
   }
 }
 
-// `cnt` partials from `part`, in order; eight loads issued before they are
-// combined
+// `cnt` partials from `part`, in order; four or eight loads issued before they
+// are added
 template <int NV>
 __device__ __forceinline__ void col_gather(double (&t)[NV], const BArgs& a, int rr, int j,
                                            const double* part, int cnt) {

@@ -208,8 +208,8 @@ void crs_build_transpose(fvg_ctx* c, const DevCRS& a, DevCRS& t, int master) {
 // rows share a row tile while the tile stays within `tile` nonzeros,
 // kTileRows rows and kLaneWork products per lane; a long row becomes its own
 // pieces of at most `tile` nonzeros, cut at 8-element boundaries.  Built on
-// the device once per matrix, in chunks of kSchedChunk rows packed by one
-// thread each (a tile never spans two chunks).
+// the device once per matrix, in chunks of kSchedChunk rows packed by one CTA
+// each (a tile never spans two chunks).
 constexpr i64 kSchedChunk = kPackRows;
 
 static const Sched& build_sched(fvg_ctx* c, DevCRS& a, int slot, int tile, int lane_work) {

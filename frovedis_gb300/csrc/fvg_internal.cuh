@@ -72,7 +72,7 @@ constexpr i64 kPad = 32;
 constexpr int kThreads = 256;
 constexpr int kTileRows = 248;  // rows per tile (their offsets are staged in shared memory)
 constexpr int kLaneWork = 32;   // products one lane may sum for one row in a tile
-// Rows one warp of the work-item packer takes (a tile never spans two such
+// Rows one CTA of the work-item packer takes (a tile never spans two such
 // chunks): short enough that the packers' tile after tile walks take a few
 // microseconds, long enough to fill kTileRows-row tiles.
 constexpr i64 kPackRows = 256;

@@ -119,7 +119,7 @@ __device__ __forceinline__ void grid_reduce(double (&v)[NV], double* part, unsig
 // thread reads back only what it wrote itself, its first element never
 // leaves its registers, and its next history entries are loaded before the
 // wait.  Bound by the chain of a step: FP64 adds of the reduction (64 clocks
-// each) and one trip to L2 and back.  Averaged over 20 iterations at n =
+// of a scheduler each) and one trip to L2 and back.  Averaged over 20 iterations at n =
 // 20,000: 87 us with a counter barrier and shared-memory trees, 71 us now;
 // n = 1,000,000, 10 iterations: 180 and 167 us.
 struct DirArgs {

@@ -1,5 +1,5 @@
 // FP64 loss and derivative of a logistic row without the general exp, log and
-// division: the FP64 unit runs one warp instruction in 64 clocks, and the
+// division: a warp's FP64 instruction takes its scheduler 64 clocks, and the
 // three calls took over 100 of them a row.
 //
 // exp and log are table driven, after P. T. P. Tang ("Table-driven

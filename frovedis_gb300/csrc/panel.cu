@@ -355,14 +355,15 @@ __global__ void k_tail_fill(const i32* __restrict__ off, const i32* __restrict__
 // among the lanes by position and joining the rows with marks, selects and a
 // segmented scan: that took 69 warp instructions per 32 entries of split
 // values, this 30.  10M x 1M split values, 4.7e8 head and 4.9e8 panel entries:
-// 1.12 + 1.29 ms before with 11,000-entry slices, 0.81 + 0.82 ms now with
-// 16,400 to 18,800, 5.4 TB/s of records, rows and sums; 2M x 200,000 BF16
-// values: 135 -> 124 us.  More copies in flight, larger copies, and records
-// asked into L2 ahead of the copies change nothing or cost time, as does
-// leaving out the gathers or the sums: the split stream is bound by HBM.  The
-// BF16 one, half the bytes a chunk, is bound by the chain of a warp's copies:
-// 8 / 16 / 24 warps take 188 / 124 / 113 us, but the split rings of 24 warps
-// leave too small a slice, and one layout serves every storage.)
+// 1.12 + 1.29 ms before with 11,000-entry slices, 0.81 each now with 17,484
+// head columns and panels of 16,448 rows, 5.4 TB/s of records, rows and sums;
+// 2M x 200,000 BF16 values: 135 -> 124 us.  More copies in flight, larger
+// copies, and records asked into L2 ahead of the copies change nothing or cost
+// time, as does leaving out the gathers or the sums: the split stream is bound
+// by HBM.  The BF16 one, half the bytes a chunk, is bound by the chain of a
+// warp's copies: 8 / 16 / 24 warps took 188 / 124 / 113 us, 20 take 124, but
+// the split rings of 24 warps leave too small a slice, and one layout serves
+// every storage.)
 constexpr int kStreamWarps = FVG_STREAM_WARPS;    // one CTA per SM
 constexpr int kStreamStages = FVG_STREAM_STAGES;  // copies in flight per warp
 constexpr int kStreamChunks = FVG_STREAM_CHUNKS;  // chunks of one copy
@@ -1161,6 +1162,7 @@ bool stream_layout(fvg_ctx* c, DevPanels& pn) {
 
 // The records of a value storage, from the matrix's own values.
 template <int ST> void fill_records(fvg_ctx* c, fvg_matrix* M, DevPanels& pn) {
+  ProfScope ps(c, pn.shared ? P_HEAD_BUILD : P_PANEL_BUILD);
   DBuf rec, slot;
   const i64 nrec = pn.nchunks + kStreamChunks;  // a copy may read past the last
   rec.alloc((size_t)nrec * StreamRec<ST>::kB, c->stream);

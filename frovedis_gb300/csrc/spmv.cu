@@ -172,10 +172,11 @@ __global__ void __launch_bounds__(kThreads, FVG_CRS_MIN_BLOCKS) k_crs(const CrsK
 }
 
 // ---------------------------------------------------------- FP64 products
-// The FP64 product.  GB300 runs about two FP64 operations a clock per SM, so
-// a warp-wide FP64 instruction costs 16 clocks whether 2 or 32 of its lanes
-// are used, while some 60 other instructions issue beside it: the row sums
-// must keep every lane's FP64 slot busy and may spend integer work freely.
+// The FP64 product.  A warp-wide FP64 instruction holds its scheduler's FP64
+// unit for 64 clocks whether 2 or 32 of its lanes are used (an SM of four
+// schedulers runs about two FP64 operations a clock), while some 60 other
+// instructions issue beside it: the row sums must keep every lane's FP64 slot
+// busy and may spend integer work freely.
 // Phase 1 (as k_crs): lane L streams nonzeros L, L+32, ... with coalesced
 // loads (one gather instruction covers 32 consecutive nonzeros) and puts the
 // gathered x and the value into the warp's shared slices.  Phase 2: lane L
@@ -480,7 +481,7 @@ __global__ void __launch_bounds__(kThreads) k_finalize(const FinK f) {
 // held a row total (12 of 32 at 40 entries a row) would.  The last CTA
 // reduces the CTAs' loss / bias partials in a fixed order.
 //
-// FP64: bound by the FP64 unit (64 clocks a warp instruction) and, on small
+// FP64: bound by the FP64 unit (64 clocks of its scheduler a warp instruction) and, on small
 // matrices, by the launch and the reduction.  With the loss of logistic64.cuh
 // and a thread's first row stored as its sum (the compensated add costs 4
 // FP64 instructions, and up to 311,000 rows a thread has one): 100,000

@@ -29,7 +29,7 @@ void check_device_error(fvg_ctx* c) {
     *word = 0u;
     std::string what;
     if (h & 2u) what += " a bulk copy did not complete in its poll budget;";
-    if (h & 4u) what += " a grid barrier was not reached in its poll budget;";
+    if (h & 4u) what += " a grid barrier (all CTAs' sums) was not reached in its poll budget;";
     fail(FVG_ERR_INTERNAL, "a device-side bounded wait gave up:" + what + " results are invalid");
   }
 }
