@@ -12,6 +12,7 @@
 namespace fvg {
 
 void throw_cuda(cudaError_t e, const char* what, const char* file, int line) {
+  cudaGetLastError();  // reported here: the next call's launch checks start clean
   char buf[512];
   snprintf(buf, sizeof(buf), "CUDA error %d (%s) in %s at %s:%d", (int)e, cudaGetErrorString(e), what, file, line);
   fail(e == cudaErrorMemoryAllocation ? FVG_ERR_OUT_OF_MEMORY : FVG_ERR_CUDA, buf);

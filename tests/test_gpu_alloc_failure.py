@@ -103,3 +103,22 @@ def test_first_use_by_a_trainer(what):
 
     with fv.Context(0) as ctx:
         assert _every_failure(lambda: ctx.matrix(a.m, a.n, a.off, a.idx, a.val), call) > 2
+
+
+def test_next_call_after_a_real_failure():
+    """More memory than any device has: refused by the driver itself, which keeps the error until it is read."""
+    a, _ = _matrix(m=50, n=40, lam=5.0)
+    x = np.random.default_rng(6).standard_normal(a.n)
+    n, k = 2_000_000_000, 128
+    with fv.Context(0) as ctx:
+        A = ctx.matrix(a.m, a.n, a.off, a.idx, a.val)
+        good = A.spmv(x)
+        W = ctx.matrix(1, n, np.array([0, 1], dtype=np.int32), np.array([7], dtype=np.int32), np.ones(1))
+        for _ in range(2):
+            with pytest.raises(fv.FvgError) as e:
+                # the FP32 copy of X (1 TB) is allocated before X is looked at; Y is never written
+                W.spmm_device(16, k, 16, storage="f32", vec="f64")
+            assert e.value.code == FVG_ERR_OUT_OF_MEMORY
+            assert np.array_equal(A.spmv(x), good)
+        W.close()
+        A.close()
