@@ -42,13 +42,13 @@ PEAKS = os.path.join(ROOT, "MEASURED_PEAKS.json")
 # the same pass (the CRS formulas of eval_bytes), per value storage, from ncu
 # captures of the benchmark matrix's kernels, the 1,000,000-row version
 # (profiles/ holds the summaries).  BF16 values: pass 1 with the forward head
-# (k_panel_stream + tail k_crs + k_finalize) 299.6 MB / 380.01 MB; pass 2 with
-# the row panels (rare-column k_crs + k_panel_stream + k_panel_colsum) 318.5
-# MB / 376.01 MB.  FP32 values: pass 1 425.0 MB / 500.0 MB, pass 2 446.8 MB /
+# (k_panel_stream + tail k_crs + k_finalize) 300.0 MB / 380.01 MB; pass 2 with
+# the row panels (rare-column k_crs + k_panel_stream + k_panel_colsum) 318.9
+# MB / 376.01 MB.  FP32 values: pass 1 425.7 MB / 500.0 MB, pass 2 448.7 MB /
 # 496.0 MB.
 NCU_TRAFFIC_RATIO = {"split": {"pass1": 574.1 / 620.81, "pass2": 594.1 / 609.21},
-                     "bf16": {"pass1": 299.6 / 380.01, "pass2": 318.5 / 376.01},
-                     "f32": {"pass1": 425.0 / 500.0, "pass2": 446.8 / 496.0}}
+                     "bf16": {"pass1": 300.0 / 380.01, "pass2": 318.9 / 376.01},
+                     "f32": {"pass1": 425.7 / 500.0, "pass2": 448.7 / 496.0}}
 TRAFFIC_SOURCE = {"split": "ncu dram bytes of every kernel of a pass / algorithmic bytes per pass (1/10-row "
                            "capture, all columns), x this run's algorithmic bytes per launch",
                   "bf16": "ncu dram bytes / algorithmic bytes per pass (1/10-row capture), x this run's "
