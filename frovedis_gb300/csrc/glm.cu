@@ -1167,10 +1167,13 @@ void sgd_train(fvg_ctx* c, fvg_matrix* M, const double* label_h, const double* s
     // used columns over all ranks, and rank 0's own count (each rank's
     // shrink table covers all of its minibatches)
     used.alloc(sizeof(int) * std::max<i64>(n, 1), s);
-    used0.alloc(sizeof(int) * std::max<i64>(n, 1) + 256, s);
+    used0.alloc(sizeof(int) * std::max<i64>(n, 1), s);
+    DBuf count0;  // rank 0's
+    count0.alloc(sizeof(unsigned long long), s);
     FVG_CUDA(cudaMemsetAsync(used.p, 0, sizeof(int) * std::max<i64>(n, 1), s));
-    FVG_CUDA(cudaMemsetAsync(used0.p, 0, sizeof(int) * std::max<i64>(n, 1) + 256, s));
-    unsigned long long* cnt0 = (unsigned long long*)((char*)used0.p + sizeof(int) * std::max<i64>(n, 1));
+    FVG_CUDA(cudaMemsetAsync(used0.p, 0, sizeof(int) * std::max<i64>(n, 1), s));
+    FVG_CUDA(cudaMemsetAsync(count0.p, 0, sizeof(unsigned long long), s));
+    unsigned long long* cnt0 = count0.as<unsigned long long>();
     for (int r = 0; r < P; r++)
       for (auto& b : ranks[r]) {
         const DevCRS& A = *b->op.oA;
