@@ -50,9 +50,11 @@ void crs_ensure_plane(fvg_ctx* c, DevCRS& a, int dt, int master) {
 // ------------------------------------------------------------------ upload
 // Counts and the longest row are combined per warp first: one atomic per
 // warp instead of one per row on a single address.
-__global__ void k_check_crs(const i32* __restrict__ off, const i32* __restrict__ idx, i64 m, i64 n, i64 nnz,
-                            unsigned long long* __restrict__ flags /* [0]=bad off, [1]=bad idx, [2]=max len */) {
-  unsigned bad_off = 0, bad_idx = 0, mx = 0;
+// flags: [0] bad offsets, [1] bad ids, [2] longest row, [3] of the first `pairs`
+// entries those with the column of the entry nnz / 2 further on
+__global__ void k_check_crs(const i32* __restrict__ off, const i32* __restrict__ idx, i64 m, i64 n, i64 nnz, i64 pairs,
+                            unsigned long long* __restrict__ flags) {
+  unsigned bad_off = 0, bad_idx = 0, mx = 0, same = 0;
   GRID_STRIDE(r, m) {
     i32 s = off[r], e = off[r + 1];
     if (e < s || s < 0 || e > nnz) bad_off++;
@@ -61,14 +63,17 @@ __global__ void k_check_crs(const i32* __restrict__ off, const i32* __restrict__
   GRID_STRIDE(p, nnz) {
     i32 c = idx[p];
     if (c < 0 || c >= n) bad_idx++;
+    if (p < pairs) same += c == idx[p + nnz / 2];
   }
   bad_off = __reduce_add_sync(0xffffffffu, bad_off);
   bad_idx = __reduce_add_sync(0xffffffffu, bad_idx);
   mx = __reduce_max_sync(0xffffffffu, mx);
+  same = __reduce_add_sync(0xffffffffu, same);
   if ((threadIdx.x & 31) == 0) {
     if (bad_off) atomicAdd(&flags[0], (unsigned long long)bad_off);
     if (bad_idx) atomicAdd(&flags[1], (unsigned long long)bad_idx);
     if (mx) atomicMax(&flags[2], (unsigned long long)mx);
+    if (same) atomicAdd(&flags[3], (unsigned long long)same);
   }
 }
 
@@ -101,18 +106,20 @@ void crs_upload(fvg_ctx* c, DevCRS& a, i64 m, i64 n, const i32* off, const i32* 
   alloc_plane(c, a.val[dt], nnz, dt);
   if (nnz) FVG_CUDA(cudaMemcpyAsync(a.val[dt].p, val, (size_t)dtype_size(dt) * nnz, kind, c->stream));
   DBuf flags;
-  flags.alloc(sizeof(unsigned long long) * 3, c->stream);
-  FVG_CUDA(cudaMemsetAsync(flags.p, 0, sizeof(unsigned long long) * 3, c->stream));
-  k_check_crs<<<grid_n(std::max(m, nnz)), 256, 0, c->stream>>>(a.off.as<i32>(), a.idx.as<i32>(), m, n, nnz,
+  flags.alloc(sizeof(unsigned long long) * 4, c->stream);
+  FVG_CUDA(cudaMemsetAsync(flags.p, 0, sizeof(unsigned long long) * 4, c->stream));
+  const i64 pairs = std::min<i64>(nnz / 2, 65536);
+  k_check_crs<<<grid_n(std::max(m, nnz)), 256, 0, c->stream>>>(a.off.as<i32>(), a.idx.as<i32>(), m, n, nnz, pairs,
                                                                 flags.as<unsigned long long>());
   check_launch("check_crs");
   count_launch(c);
-  unsigned long long h[3];
+  unsigned long long h[4];
   FVG_CUDA(cudaMemcpyAsync(h, flags.p, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
   FVG_CUDA(cudaStreamSynchronize(c->stream));
   if (h[0]) fail(FVG_ERR_INVALID_ARG, "row offsets are not non-decreasing within [0, nnz]");
   if (h[1]) fail(FVG_ERR_INVALID_ARG, "column index out of range [0, num_col)");
   a.max_row = (i64)h[2];
+  a.spread = (i64)h[3] * 1000 < pairs;
 }
 
 __global__ void k_max_row(const i32* __restrict__ off, i64 m, unsigned long long* __restrict__ mx) {

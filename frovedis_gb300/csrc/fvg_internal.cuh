@@ -125,6 +125,7 @@ struct DevCRS {
   i64 slab_rows = 0;
   const Sched* slab_of = nullptr;  // of which of sched[] its tiles are
   i64 max_row = 0;
+  bool spread = false;  // uploaded entries half the matrix apart hardly ever share a column (k_check_crs)
 };
 
 struct DevELL {  // column-major m x width, zero padded (ell_matrix.hpp:63-95)

@@ -695,22 +695,28 @@ __device__ __forceinline__ void pre_fetch(const SpmmK& p, EntryPre<AT>& pre, i32
 // padding included.  1M rows x 100 entries, 32 columns, BF16 values (with the
 // 8-byte stage): softmax pass 908 -> 780 us, transposed pass 722 -> 702 us.
 //
-// PRE (entries fetched a chunk ahead): plain products with FP32 values up to
-// 64 columns (300 000 rows x 50 entries, 64 columns: 217 us without, 192 with;
-// 128 columns of 100 000 rows: 151 without, 176 with) and FP64 ones up to 32
-// (150 000 rows x 60 entries, 32 columns: 545 without, 540 with; 64 columns:
-// 955 without, 1,011 with).  BF16 values are
-// faster without (60 000 rows x 20 entries, 64 columns: 55 without, 58 with),
-// and the epilogues' registers and the FP64 results of the transposed pass
-// leave no room for it (64 a thread): 796 -> 832, 702 -> 797 us.
-template <class VT, class XT, class AT, int G, bool PRE>
+// HOW:
+//   kBatch4  four steps' gathers together;
+//   kAhead   two, and the entries fetched a chunk ahead: plain products with
+//            FP32 values up to 64 columns (300 000 rows x 50 entries, 64
+//            columns: 217 us without, 192 with; 128 columns of 100 000 rows:
+//            151 without, 176 with) and FP64 ones up to 32 (150 000 rows x 60
+//            entries, 32 columns: 545 without, 540 with; 64 columns: 955
+//            without, 1,011 with).  BF16 values are faster without (60 000 rows
+//            x 20 entries, 64 columns: 55 without, 58 with), and the epilogues'
+//            registers and the FP64 results of the transposed pass leave no
+//            room for it (64 a thread): 796 -> 832, 702 -> 797 us;
+//   kBatch2  two: rows of a few entries, whose batch of four is half empty.
+// The rule for plain FP32 sums is in launch_grouped_l.
+enum { kBatch4, kAhead, kBatch2 };
+template <class VT, class XT, class AT, int G, int HOW>
 __device__ __forceinline__ void row_dot_g(const SpmmK& p, i32 e0, i32 e1, int lane, AT (&a)[GLay<XT, G>::CPL],
                                           StageE<AT>* st, bool lane_on, EntryPre<AT>& pre, const Item& item,
                                           const Item& next) {
   using L = GLay<XT, G>;
   constexpr int CPL = L::CPL;
-  constexpr bool PACK = sizeof(XT) == 4 && sizeof(AT) == 4;
-  constexpr int kStep = PRE ? 2 : 4;
+  constexpr bool PACK = sizeof(XT) == 4 && sizeof(AT) == 4, PRE = HOW == kAhead;
+  constexpr int kStep = HOW == kBatch4 ? 4 : 2;
   static_assert(32 / G >= kStep, "whole batches of steps in a chunk");
   const int sub = lane % L::LPR, grp = lane / L::LPR;
   const char* X = (const char*)((const XT*)p.X + sub * CPL);
@@ -828,7 +834,7 @@ __device__ __forceinline__ void row_dot_g(const SpmmK& p, i32 e0, i32 e1, int la
 template <class XT, class YT, int EPI, int G>
 constexpr int kGroupedCtas = EPI == EPI_STORE && sizeof(XT) == 4 && sizeof(YT) == 8 && G <= 4 ? 3 : 4;
 
-template <class VT, class XT, class AT, class YT, int EPI, int G>
+template <class VT, class XT, class AT, class YT, int EPI, int G, int HOW>
 __global__ void __launch_bounds__(kThreads, kGroupedCtas<XT, YT, EPI, G>) k_spmm_g(const SpmmK p) {
   using L = GLay<XT, G>;
   using Sum = typename SumOf<AT>::type;
@@ -856,8 +862,7 @@ __global__ void __launch_bounds__(kThreads, kGroupedCtas<XT, YT, EPI, G>) k_spmm
   __shared__ StageE<AT> stage[kThreads / 32][32];
   unsigned long long mw = mask_of(p, 0);
   AT lab = 0, w = 1;
-  // entries fetched ahead: see row_dot_g
-  constexpr bool PRE = EPI == EPI_STORE && sizeof(YT) == sizeof(AT) && sizeof(VT) == sizeof(AT) && G >= (sizeof(AT) == 8 ? 2 : 4);
+  constexpr bool PRE = HOW == kAhead;  // entries fetched ahead: see row_dot_g
   EntryPre<AT> pre;
   Item next{0, 0, 0, 0};
   if (PRE && gw < p.nitems) next = p.items[gw];
@@ -877,7 +882,7 @@ __global__ void __launch_bounds__(kThreads, kGroupedCtas<XT, YT, EPI, G>) k_spmm
         mw = mask_of(p, walk.d);
       }
       if (mw == 0) continue;  // the finalize skips the row too
-      row_dot_g<VT, XT, AT, G, PRE>(p, item.e0, item.e1, lane, a, stage[wib], cols_on(mw, lsh, CPL), pre, item,
+      row_dot_g<VT, XT, AT, G, HOW>(p, item.e0, item.e1, lane, a, stage[wib], cols_on(mw, lsh, CPL), pre, item,
                                     next);
       AT* part = (AT*)p.partials + (i64)(-1 - item.r1) * NC;
 #pragma unroll
@@ -890,7 +895,7 @@ __global__ void __launch_bounds__(kThreads, kGroupedCtas<XT, YT, EPI, G>) k_spmm
         mw = mask_of(p, walk.d);
       }
       if (mw == 0) continue;  // no column of this dataset is computed
-      row_dot_g<VT, XT, AT, G, PRE>(p, __ldg(p.off + r), __ldg(p.off + r + 1), lane, a, stage[wib], cols_on(mw, lsh, CPL), pre, item,
+      row_dot_g<VT, XT, AT, G, HOW>(p, __ldg(p.off + r), __ldg(p.off + r + 1), lane, a, stage[wib], cols_on(mw, lsh, CPL), pre, item,
                                     next);
       if constexpr (EPI == EPI_STORE) {
         YT* y = (YT*)p.Y + (i64)r * p.ldy;
@@ -1132,13 +1137,13 @@ static double* seg_slots(const SpmmSeg& sg) {
 // Grouped layout launch: k_spmm_g and its finalize kernel (NC / 32
 // columns a lane); for stacked datasets the slot reduction is left to
 // crs_spmm_seg_finish.
-template <class VT, class XT, class AT, class YT, int EPI, int G>
-static void launch_grouped_l(fvg_ctx* c, DevCRS& a, const Sched& s, int storage, SpmmK p, double* out,
+template <class VT, class XT, class AT, class YT, int EPI, int G, int HOW>
+static void launch_grouped_how(fvg_ctx* c, DevCRS& a, const Sched& s, int storage, SpmmK p, double* out,
                              double* gbias, char* scratch, SpmmSeg* sg) {
   using L = GLay<XT, G>;
   constexpr int NC = L::NC, CF = NC / 32;
   const int grid = (int)std::max<i64>(
-      1, std::min<i64>(occupancy_blocks((const void*)k_spmm_g<VT, XT, AT, YT, EPI, G>, kThreads) * c->num_sms,
+      1, std::min<i64>(occupancy_blocks((const void*)k_spmm_g<VT, XT, AT, YT, EPI, G, HOW>, kThreads) * c->num_sms,
                        (s.nitems + 7) / 8));
   const int fg = spmm_fin_grid(c, s.nlong);
   unsigned* ticket = (unsigned*)scratch;
@@ -1173,7 +1178,7 @@ static void launch_grouped_l(fvg_ctx* c, DevCRS& a, const Sched& s, int storage,
     p.mword = sg->mword;
   }
   if (s.nitems > 0 || seg) {
-    k_spmm_g<VT, XT, AT, YT, EPI, G><<<grid, kThreads, 0, c->stream>>>(p);
+    k_spmm_g<VT, XT, AT, YT, EPI, G, HOW><<<grid, kThreads, 0, c->stream>>>(p);
     check_launch("k_spmm_g");
     count_launch(c);
   }
@@ -1198,6 +1203,37 @@ static void launch_grouped_l(fvg_ctx* c, DevCRS& a, const Sched& s, int storage,
     sg->nw2 = nw2;
     sg->nc = NC;
     sg->icpt = p.icpt;
+  }
+}
+
+// How the gathers of plain sums (up to 64 FP32 or 32 FP64 columns) are issued.
+// Two steps at a time where rows are short: a batch of four is then mostly
+// predicates (300,000 rows x 5 entries, two / four: BF16 values, 8 columns 103
+// / 117 us, 64 columns 112 / 127; FP32 values, 8 columns 104 / 113 with entries
+// ahead; 13 entries, BF16, 8 columns 99 / 108, 64 columns 136 / 136).
+// Entries ahead for FP32 values, except where the columns are scattered
+// (DevCRS::spread) over more of X than L2 keeps beside the entries: the rows of
+// X then come from HBM, and four gathers under way do more than early entries
+// (300,000 power-law rows x 40 entries, 64 columns, ahead / four: X of 77 MB
+// 341 / 315 us, 128 MB 428 / 389; 40 columns, 48 MB 246 / 246).
+constexpr i64 kShortRows = 7, kShortRows16 = 15;
+constexpr i64 kSpreadX = 64ll << 20;
+template <class VT, class XT, class AT, class YT, int EPI, int G>
+static void launch_grouped_l(fvg_ctx* c, DevCRS& a, const Sched& s, int storage, SpmmK p, double* out,
+                             double* gbias, char* scratch, SpmmSeg* sg) {
+  auto launch = [&](auto how) {
+    launch_grouped_how<VT, XT, AT, YT, EPI, G, decltype(how)::value>(c, a, s, storage, p, out, gbias, scratch, sg);
+  };
+  if constexpr (EPI == EPI_STORE && sizeof(YT) == sizeof(AT) && sizeof(AT) == 8 && G >= 2) {
+    launch(std::integral_constant<int, kAhead>());
+  } else if constexpr (EPI == EPI_STORE && sizeof(YT) == sizeof(AT) && sizeof(AT) == 4 && G >= 4) {
+    const bool scattered = a.spread && a.n * p.ldx * (i64)sizeof(XT) > kSpreadX;
+    constexpr i64 kShort = sizeof(VT) == 2 && G == 8 ? kShortRows16 : kShortRows;
+    if (a.nnz < kShort * a.m) launch(std::integral_constant<int, kBatch2>());
+    else if (sizeof(VT) == 4 && !scattered) launch(std::integral_constant<int, kAhead>());
+    else launch(std::integral_constant<int, kBatch4>());
+  } else {
+    launch(std::integral_constant<int, kBatch4>());
   }
 }
 
