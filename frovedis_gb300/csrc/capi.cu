@@ -307,7 +307,7 @@ FVG_API fvg_status fvg_matrix_prepare(fvg_ctx* c, fvg_matrix* M, fvg_format fmt,
   if (with_transpose && M->AT) {  // the transposed copy's planes beside A's
     if (M->A.lo.p) crs_ensure_split(c, *M->AT, M->master);
     for (int dt : {FVG_F32, FVG_BF16})
-      if (M->A.val[dt].p) crs_ensure_plane(c, *M->AT, dt, M->master);
+      if ((fmt == FVG_CRS || fmt == FVG_ELL) && M->A.val[dt].p) crs_ensure_plane(c, *M->AT, dt, M->master);
   }
   // a matrix that already holds FP32 / BF16 values gets its row-panel
   // backward layout and its forward head now rather than at the first product
